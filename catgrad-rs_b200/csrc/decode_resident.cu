@@ -153,14 +153,6 @@ __device__ __forceinline__ void umma_bf16_first(uint32_t tmem_d, uint64_t da, ui
       ::"r"(tmem_d), "l"(da), "l"(db), "r"(idesc)
       : "memory");
 }
-__device__ __forceinline__ void umma_bf16_acc(uint32_t tmem_d, uint64_t da, uint64_t db, uint32_t idesc) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.eq.b32 p, 0, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-      ::"r"(tmem_d), "l"(da), "l"(db), "r"(idesc)
-      : "memory");
-}
 // Position in the shared-memory ring: slot index and the parity of the slot's current use.  The
 // roles advance it once per stage (no division by the runtime ring depth on the issue path).
 struct RingPos {

@@ -6,6 +6,9 @@
 //   * warp 0 streams 128-row weight tiles by TMA into a shared-memory ring and starts doing
 //     so BEFORE the preceding kernel has finished (programmatic dependent launch): weights
 //     do not depend on it.  Only the small bf16 activation tiles wait for the predecessor.
+//     Most CTAs find room only as their predecessors leave (median start of a CTA = end of the
+//     preceding kernel, per-CTA timeline of a Llama-3.2-1B step), so the first requests go out as soon
+//     as their barriers exist, ahead of the TMEM allocation and the CTA's first barrier.
 //   * a CTA keeps its shared-memory ring small (about a third of an SM) so that the CTAs of
 //     the NEXT GEMM in the stream can already be resident and prefetching their weights while
 //     this one computes: the HBM stream does not stop at kernel boundaries.
@@ -13,12 +16,19 @@
 //     pair of the FFN both 128-row tiles share the CTA and the epilogue writes
 //     act(gate) * up directly (llama.rs:27), so the [M, 2F] intermediate never exists.
 //   * split-K partials are PUSHED over distributed shared memory inside a thread-block cluster:
-//     every CTA stores its partial rows into the exchange area of the CTA that finishes them,
-//     one cluster barrier makes the stores visible, and the owner adds the partials in rank
+//     every CTA stores its partial rows (st.async) into the exchange area of the CTA that finishes
+//     them, whose own mbarrier counts the bytes, and the owner adds the partials in rank
 //     order (deterministic) out of its own shared memory and applies the epilogue (residual add /
-//     bf16 / act) once.  No CTA reads another's memory, so none has to wait for the others
-//     before it leaves; the residual of the element a thread will finish is fetched while the
-//     MMAs still run.
+//     bf16 / act) once.  No CTA reads another's memory; the residual of the element a thread will
+//     finish is fetched while the MMAs still run.
+//   * every kernel of a step waits for the one before it, so what a single thread issues between two
+//     arrivals is felt: slots and descriptors are counted along instead of divided and rebuilt (a
+//     division by the runtime ring depth and four descriptors per stage had cost 4 % of a step), the
+//     activations that follow the dependency are fetched by the idle epilogue warps, and TMEM is given
+//     back beside the epilogue.
+//     A step of the Llama-3.2-1B shape, batch 1 / batch 8: 733 / 835 us -> 645 / 754 us; four layers of
+//     the Gemma-2-2B shape 514 -> 491 us, the Ralapel design 792 -> 740 us.  Of that the early requests and
+//     the cheaper epilogue indices give 7 %.
 //
 //   * two optional hand-overs ride on the epilogue.  Norm hand-over: a residual GEMM also
 //     leaves bf16(out * gain) and per-CTA sums of out^2, and the GEMM behind the norm applies
@@ -50,12 +60,15 @@ struct DecArgs {
   int dual, act, up_off;
   int M, N, K;
   int kb_total, kb_per_split, splits, stages;
+  int lg_rows_per;  // log2 of the rows of a tile that a split finishes (128 / splits)
   int x_rows;       // activation rows per k block in the ring (8 or TN)
   int xstage_cols;  // split-K: token columns of the exchange area (>= min(TN, M)); 0 without split-K
   int xstage_in_ring;  // the exchange area lies over the ring (more than 16 tokens: it would cost the ring a
                        // stage): then a first cluster barrier says every CTA's ring is idle before anyone pushes
   int32_t* err;
   int trace;  // slot in the timeline buffer, or -1
+  const __nv_bfloat16* x;  // [M, K], leading dimension ldx
+  int64_t ldx;
   PeerPush push;  // out_mode 3
   int total_ctas;
   // norm hand-over (see DecGemm): producer side ...
@@ -119,6 +132,39 @@ __device__ __forceinline__ float finish(const DecArgs& p, int m, int n, float g,
   return 0.f;
 }
 
+__device__ __forceinline__ void st_async(uint32_t addr, uint32_t v, uint32_t bar) {
+  asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.b32 [%0], %1, [%2];" ::"r"(addr), "r"(v), "r"(bar)
+               : "memory");
+}
+
+// Activation chunks (16 bytes) of the first k blocks: chunk id = ((k block * x_rows) + row) * 8 + place.
+// Rows past M are not read (they feed unused columns); places past K are zero.
+constexpr int XCH = 4;
+__device__ __forceinline__ void load_x_chunks(const DecArgs& p, int kb0, int id0, int chunks, int lg_rows, uint4* v) {
+#pragma unroll
+  for (int j = 0; j < XCH; ++j) {
+    const int id = id0 + j * 128;
+    const int t = id >> 3, r = t & ((1 << lg_rows) - 1);
+    const int k = (kb0 + (t >> lg_rows)) * BK + (id & 7) * 8;
+    v[j] = make_uint4(0u, 0u, 0u, 0u);
+    if (id < chunks && r < p.M && k < p.K)
+      asm volatile("ld.global.cg.v4.u32 {%0, %1, %2, %3}, [%4];"
+                   : "=r"(v[j].x), "=r"(v[j].y), "=r"(v[j].z), "=r"(v[j].w)
+                   : "l"(p.x + (int64_t)r * p.ldx + k)
+                   : "memory");
+  }
+}
+__device__ __forceinline__ void store_x_chunks(uint32_t xbase, uint32_t stage_bytes, int id0, int chunks, int lg_rows, const uint4* v) {
+#pragma unroll
+  for (int j = 0; j < XCH; ++j) {
+    const int id = id0 + j * 128;
+    if (id >= chunks) break;
+    const int t = id >> 3, r = t & ((1 << lg_rows) - 1);
+    const uint32_t a = xbase + (uint32_t)(t >> lg_rows) * stage_bytes + (uint32_t)r * 128u + (uint32_t)(((id & 7) ^ (r & 7)) << 4);
+    asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(a), "r"(v[j].x), "r"(v[j].y), "r"(v[j].z), "r"(v[j].w) : "memory");
+  }
+}
+
 // OCC: CTAs per SM the register allocation must allow (the fewer registers a CTA holds, the
 // sooner the CTAs of the NEXT kernels in the stream fit beside it and start fetching their weights)
 template <int TN, int OCC>
@@ -144,9 +190,10 @@ k_gemm_dec(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CU
   const uint32_t boff = STAGES * stage_bytes + (p.xstage_in_ring ? 0u : xbytes);
   const uint32_t bars = base + boff;  // full[STAGES], empty[STAGES], accum
   const uint32_t bar_accum = bars + 16 * STAGES;
+  const uint32_t bar_x = bar_accum + 16;  // split-K: every addend of this CTA's rows has arrived
   volatile uint32_t* tmem_slot = (volatile uint32_t*)(gen + boff + 16 * STAGES + 8);
   volatile int* cta_abort = (volatile int*)(gen + boff + 16 * STAGES + 12);
-  float* sc = (float*)(gen + boff + 16 * 8 + 64);  // [32] per-token 1 / rms (consumer side)
+  float* sc = (float*)(gen + boff + 16 * 8 + 64);  // [32] per-token 1 / rms (consumer side), [4][32] the warps' sums
   // [SQ_FLOATS] squared outputs (producer side): in the ring, which is idle by then (only this
   // CTA touches its ring)
   float* sq = (float*)(gen + (p.xstage_in_ring ? xbytes : 0u));
@@ -156,17 +203,34 @@ k_gemm_dec(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CU
   const int kb0 = split * p.kb_per_split;
   const int nkb = min(p.kb_total, kb0 + p.kb_per_split) - kb0;
   const uint32_t ncols = p.dual ? 2 * TN : (TN < 32 ? 32 : TN);
+  const bool cluster = p.splits > 1;
   if (tid == 0) trace_min(p.trace, 0);
 
   if (tid == 0) {
+    asm volatile("prefetch.tensormap [%0];" ::"l"(&map_w) : "memory");
     for (int s = 0; s < STAGES; ++s) {
       mbar_init(bars + 8 * s, 2);             // full[s]: weight arrival + activation arrival
       mbar_init(bars + 8 * (STAGES + s), 1);  // empty[s]: one tcgen05.commit
     }
     mbar_init(bar_accum, 1);
+    if (cluster) {
+      // all 128 rows / splits rows of every split, M tokens of one or two accumulators
+      mbar_init(bar_x, 1);
+      mbar_expect_tx(bar_x, (uint32_t)((p.dual ? 2 : 1) * p.M) * BM * 4u);
+    }
     *cta_abort = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    // weights first, before this CTA is even set up: they depend neither on the preceding kernel nor on
+    // TMEM, and a CTA that starts when its predecessors leave is waited for from here on
+    for (int i = 0; i < min(nkb, STAGES); ++i) {
+      const uint32_t full = bars + 8 * i;
+      const uint32_t a = base + i * stage_bytes;
+      const int k = (kb0 + i) * BK;
+      mbar_expect_tx(full, wbytes);
+      tma_load_2d(a, &map_w, k, n0, full);
+      if (p.dual) tma_load_2d(a + A_BYTES, &map_w, k, p.up_off + n0, full);
+    }
   }
   if (warp == 1) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32((const void*)tmem_slot)),
@@ -178,72 +242,83 @@ k_gemm_dec(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CU
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem_acc = *tmem_slot;
+  // the peers' barriers exist once they have arrived here; waited for just before the pushes
+  if (cluster && !p.xstage_in_ring) asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
 
   bool acc_ok = false;
   Prefetched pre{false, 0.f, 0.f};
   if (warp == 0) {
-    if (lane == 0 && nkb > 0) {
-      // weights first: they do not depend on the preceding kernel
-      asm volatile("prefetch.tensormap [%0];" ::"l"(&map_x) : "memory");
+    if (lane == 0) {
       const int pre = min(nkb, STAGES);
-      for (int i = 0; i < pre; ++i) {
-        const uint32_t full = bars + 8 * i;
-        const uint32_t a = base + i * stage_bytes;
+      if (nkb > pre) asm volatile("prefetch.tensormap [%0];" ::"l"(&map_x) : "memory");
+      asm volatile("griddepcontrol.wait;" ::: "memory");
+      trace_min(p.trace, 1);
+      // (slot and parity are counted along: a division by the runtime ring depth per stage is felt)
+      int sl = 0;
+      uint32_t par = 0;
+      for (int i = pre; i < nkb; ++i) {
+        const uint32_t full = bars + 8 * sl;
+        const uint32_t a = base + sl * stage_bytes;
         const int k = (kb0 + i) * BK;
+        // (the epilogue warps fetch the activations of the first `pre` blocks)
+        if (!mbar_wait(bars + 8 * (STAGES + sl), par, cta_abort, p.err)) break;
         mbar_expect_tx(full, wbytes);
         tma_load_2d(a, &map_w, k, n0, full);
         if (p.dual) tma_load_2d(a + A_BYTES, &map_w, k, p.up_off + n0, full);
-      }
-      asm volatile("griddepcontrol.wait;" ::: "memory");
-      trace_min(p.trace, 1);
-      for (int i = 0; i < nkb; ++i) {
-        const int s = i % STAGES;
-        const uint32_t full = bars + 8 * s;
-        const uint32_t a = base + s * stage_bytes;
-        const int k = (kb0 + i) * BK;
-        if (i >= pre) {
-          const uint32_t ph = (uint32_t)(i / STAGES) & 1u;
-          if (!mbar_wait(bars + 8 * (STAGES + s), ph ^ 1u, cta_abort, p.err)) break;
-          mbar_expect_tx(full, wbytes);
-          tma_load_2d(a, &map_w, k, n0, full);
-          if (p.dual) tma_load_2d(a + A_BYTES, &map_w, k, p.up_off + n0, full);
-        }
         mbar_expect_tx(full, X_TILE);
         tma_load_2d(a + wbytes, &map_x, k, 0, full);
+        if (++sl == STAGES) { sl = 0; par ^= 1u; }
       }
     }
   } else if (warp == 1) {
     if (lane == 0 && nkb > 0) {
       const uint32_t idesc = umma_idesc(TN);
+      // descriptors of slot 0: a slot or 16 k further on only the address field moves
+      const uint64_t da0 = umma_desc(base), db0 = umma_desc(base + wbytes);
+      const uint64_t dslot = stage_bytes >> 4;
+      constexpr uint64_t DK = UMMA_K * 2 >> 4, DUP = A_BYTES >> 4;
+      uint64_t off = 0;
+      int sl = 0;
+      uint32_t par = 0;
       bool ok = true;
-      for (int i = 0; i < nkb && ok; ++i) {
-        const int s = i % STAGES;
-        const uint32_t ph = (uint32_t)(i / STAGES) & 1u;
-        ok = mbar_wait(bars + 8 * s, ph, cta_abort, p.err);
+      for (int i = 0; i < nkb; ++i) {
+        ok = mbar_wait(bars + 8 * sl, par, cta_abort, p.err);
         if (!ok) break;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        const uint32_t a = base + s * stage_bytes;
+        const uint64_t da = da0 + off, db = db0 + off;
+        umma_bf16(tmem_acc, da, db, idesc, i > 0 ? 1u : 0u);
 #pragma unroll
-        for (int kk = 0; kk < BK / UMMA_K; ++kk) {
-          const uint64_t db = umma_desc(a + wbytes + kk * UMMA_K * 2);
-          umma_bf16(tmem_acc, umma_desc(a + kk * UMMA_K * 2), db, idesc, (i > 0 || kk > 0) ? 1u : 0u);
-          if (p.dual) umma_bf16(tmem_acc + TN, umma_desc(a + A_BYTES + kk * UMMA_K * 2), db, idesc, (i > 0 || kk > 0) ? 1u : 0u);
+        for (int kk = 1; kk < BK / UMMA_K; ++kk) umma_bf16_acc(tmem_acc, da + kk * DK, db + kk * DK, idesc);
+        if (p.dual) {
+          umma_bf16(tmem_acc + TN, da + DUP, db, idesc, i > 0 ? 1u : 0u);
+#pragma unroll
+          for (int kk = 1; kk < BK / UMMA_K; ++kk) umma_bf16_acc(tmem_acc + TN, da + DUP + kk * DK, db + kk * DK, idesc);
         }
-        umma_commit(bars + 8 * (STAGES + s));
+        if (i + STAGES < nkb) umma_commit(bars + 8 * (STAGES + sl));  // (nobody waits for a slot's last use)
+        off += dslot;
+        if (++sl == STAGES) { sl = 0; par ^= 1u; off = 0; }
       }
       if (ok) umma_commit(bar_accum);
     }
   } else {
     // outputs (and the residual) belong to the stream order: wait for the preceding kernel
     asm volatile("griddepcontrol.wait;" ::: "memory");
+    const int et = tid - 64;
+    // The activations of the k blocks whose weights are already on their way: plain 16-byte loads by
+    // these idle warps, stored in the 128-byte swizzle the MMA reads.  They are all there is between
+    // the predecessor's end and the MMAs, and a TMA load takes about 0.4 us longer to come back.
+    const int npre = min(nkb, STAGES);
+    const int lg_rows = p.x_rows == 8 ? 3 : p.x_rows == 16 ? 4 : 5;
+    const int chunks = npre << (lg_rows + 3);
+    uint4 xv[XCH];
+    load_x_chunks(p, kb0, et, chunks, lg_rows, xv);
     if (p.splits > 1 && (p.out_mode == 2 || p.xb_out)) {
       // split-K: the element this thread will finish first is known now; fetch its residual (and
       // the next norm's gain) while the MMAs run instead of after the reduction
-      const int rows_per = BM / p.splits;
-      const int e = tid - 64;
-      if (e < rows_per * min(TN, p.M)) {
-        const int col = e / rows_per;
-        const int n = n0 + split * rows_per + (e - col * rows_per);
+      const int lg = p.lg_rows_per;
+      if (et < min(TN, p.M) << lg) {
+        const int col = et >> lg;
+        const int n = n0 + (split << lg) + (et & ((1 << lg) - 1));
         if (n < p.N) {
           asm volatile("ld.global.f32 %0, [%1];" : "=f"(pre.res) : "l"(p.residual + (int64_t)col * p.ldo + n) : "memory");
           if (p.xb_out) asm volatile("ld.global.f32 %0, [%1];" : "=f"(pre.gain) : "l"(p.g_next + n) : "memory");
@@ -251,16 +326,35 @@ k_gemm_dec(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CU
         }
       }
     }
+    store_x_chunks(base + wbytes, stage_bytes, et, chunks, lg_rows, xv);
+    for (int c0 = et + 128 * XCH; c0 < chunks + et; c0 += 128 * XCH) {
+      load_x_chunks(p, kb0, c0, chunks, lg_rows, xv);
+      store_x_chunks(base + wbytes, stage_bytes, c0, chunks, lg_rows, xv);
+    }
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    asm volatile("bar.sync 1, 128;" ::: "memory");
+    if (et < npre) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bars + 8 * et) : "memory");
     if (p.ss_in) {
-      // per-token sum of squares = the producer's per-CTA partials added in a fixed order
-      // (four interleaved quarters per token, then the quarters): loads fly while the MMAs run
-      const int et = tid - 64, m = et >> 2, j = et & 3;
-      float a = 0.f;
-      if (m < p.M)
-        for (int i = j; i < p.ss_parts; i += 4) a += __ldcg(p.ss_in + (int64_t)i * 32 + m);
-      const float a1 = __shfl_down_sync(0xffffffffu, a, 1), a2 = __shfl_down_sync(0xffffffffu, a, 2),
-                  a3 = __shfl_down_sync(0xffffffffu, a, 3);
-      if (j == 0 && m < p.M) sc[m] = 1.0f / sqrtf((((a + a1) + a2) + a3) * p.ss_inv_h + p.ss_eps);
+      // per-token sum of squares = the producer's per-CTA partials, in a fixed order: 128 / G threads
+      // over the parts for each group of four tokens, then a shuffle tree, then the four warps in order
+      const int lg = p.M <= 4 ? 0 : p.M <= 8 ? 1 : p.M <= 16 ? 2 : 3;
+      const float* src = p.ss_in + ((et & ((1 << lg) - 1)) << 2);
+      float4 a = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 4
+      for (int i = et >> lg; i < p.ss_parts; i += 128 >> lg) {
+        const float4 v = __ldcg((const float4*)(src + (int64_t)i * 32));
+        a.x += v.x; a.y += v.y; a.z += v.z; a.w += v.w;
+      }
+      for (int o = 16; o >= (1 << lg); o >>= 1) {
+        a.x += __shfl_xor_sync(0xffffffffu, a.x, o);
+        a.y += __shfl_xor_sync(0xffffffffu, a.y, o);
+        a.z += __shfl_xor_sync(0xffffffffu, a.z, o);
+        a.w += __shfl_xor_sync(0xffffffffu, a.w, o);
+      }
+      if (lane < (1 << lg)) *(float4*)(sc + 32 + (warp - 2) * 32 + lane * 4) = a;
+      asm volatile("bar.sync 1, 128;" ::: "memory");
+      if (et < p.M)
+        sc[et] = 1.0f / sqrtf((((sc[32 + et] + sc[64 + et]) + sc[96 + et]) + sc[128 + et]) * p.ss_inv_h + p.ss_eps);
       asm volatile("bar.sync 1, 128;" ::: "memory");
     }
     if (nkb > 0) {
@@ -270,29 +364,33 @@ k_gemm_dec(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CU
     }
   }
 
-  const bool cluster = p.splits > 1;
   // the reduction this kernel contributes to: one more than the last one this rank pushed
   // (stable until this kernel's last CTA has seen every other CTA finish)
   uint32_t parity = 0;
   if (p.out_mode == 3 && warp >= 2) parity = peer_push_parity(p.push);
-  if (cluster && p.xstage_in_ring) {
-    // every thread of every CTA of the cluster is here only after its CTA's loads have landed
-    // and its MMAs have read them: from here on the rings may be written by the peers
+  if (cluster) {
+    // (exchange area in the ring: every thread of every CTA of the cluster arrives only after its CTA's
+    // loads have landed and its MMAs have read them; after this the rings may be written by the peers)
     __syncwarp();
-    cluster_sync_all();
+    if (p.xstage_in_ring) asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
   }
-  if (warp >= 2 && acc_ok) {
+  // with split-K a CTA whose accumulator never came pushes all the same: its peers count on the bytes
+  // (the error word is set, and nothing is written from them)
+  if (warp >= 2 && (acc_ok || cluster)) {
     const int q = warp & 3;
     const int row = q * 32 + lane;
     const int n = n0 + row;
     // split-K: every value goes straight into the exchange area of the CTA that finishes its row
     // (rows [r * 128 / S, (r + 1) * 128 / S) belong to cluster rank r), slot [this split][col][row]
-    const int rows_per = BM / p.splits;
+    const int lg = p.lg_rows_per;
     const int xcols = (p.dual ? 2 : 1) * p.xstage_cols;
-    uint32_t xdst = 0;
+    uint32_t xdst = 0, xbar = 0;
     if (cluster) {
-      asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(xdst) : "r"(base + xoff), "r"((uint32_t)(row / rows_per)));
-      xdst += (uint32_t)(split * xcols * rows_per + row % rows_per) * 4u;
+      const uint32_t owner = (uint32_t)(row >> lg);
+      asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(xdst) : "r"(base + xoff), "r"(owner));
+      asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(xbar) : "r"(bar_x), "r"(owner));
+      xdst += (uint32_t)(((split * xcols) << lg) + (row & ((1 << lg) - 1))) * 4u;
     }
 #pragma unroll 1
     for (int c0 = 0; c0 < TN; c0 += 16) {
@@ -305,10 +403,8 @@ k_gemm_dec(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CU
 #pragma unroll
         for (int j = 0; j < 16; ++j) {
           if (c0 + j >= p.M) break;
-          asm volatile("st.shared::cluster.b32 [%0], %1;" ::"r"(xdst + (uint32_t)((c0 + j) * rows_per) * 4u), "r"(g[j]) : "memory");
-          if (p.dual)
-            asm volatile("st.shared::cluster.b32 [%0], %1;" ::"r"(xdst + (uint32_t)((p.xstage_cols + c0 + j) * rows_per) * 4u), "r"(u[j])
-                         : "memory");
+          st_async(xdst + ((uint32_t)(c0 + j) << (lg + 2)), g[j], xbar);
+          if (p.dual) st_async(xdst + ((uint32_t)(p.xstage_cols + c0 + j) << (lg + 2)), u[j], xbar);
         }
       } else {
 #pragma unroll
@@ -332,56 +428,79 @@ k_gemm_dec(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CU
     if (acc_ok && et < p.M) p.ss_out[(int64_t)blockIdx.x * 32 + et] = ((sq[et] + sq[32 + et]) + sq[64 + et]) + sq[96 + et];
   }
 
+  if (warp >= 2 && p.out_mode != 3) {
+    // the accumulators have been read: warp 1 gives the TMEM back beside the rest of the epilogue
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    asm volatile("bar.arrive 3, 160;" ::: "memory");
+  }
   if (cluster) {
-    // One cluster barrier: every CTA's pushes are visible after it, and nobody touches another
-    // CTA's shared memory again, so a CTA may leave as soon as its own rows are finished.
+    // Arrived when every CTA of the cluster has issued its pushes; waited for before this CTA leaves,
+    // so that no push can find its target gone even where a wait has given up.
     __syncwarp();
-    cluster_sync_all();
-    if (warp >= 2 && !*cta_abort) {
-      const int S = p.splits;
-      const int rows_per = BM / S;
-      const int cols = min(TN, p.M);
+    asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
+    // the bytes themselves are counted on this CTA's own barrier, which costs one way across the
+    // cluster where a barrier over all threads costs a return trip
+    if (warp >= 2) {
+      const bool got = mbar_wait_cluster(bar_x, 0, cta_abort, p.err) && !*cta_abort;
+      const int S = p.splits, lg = p.lg_rows_per, et = tid - 64;
+      const int todo = min(TN, p.M) << lg;  // columns x rows this CTA finishes
       const int xcols = (p.dual ? 2 : 1) * p.xstage_cols;
       const float* xs = (const float*)(gen + xoff);
-      for (int e = tid - 64; e < rows_per * cols; e += 128) {
-        const int col = e / rows_per, rl = e - col * rows_per;
-        const int row = split * rows_per + rl;
-        // the splits' partial sums in rank order (all loads first)
-        float pg[16], pu[16];
-#pragma unroll
-        for (int s = 0; s < 16; ++s) {
-          pg[s] = s < S ? xs[(s * xcols + col) * rows_per + rl] : 0.f;
-          pu[s] = (p.dual && s < S) ? xs[(s * xcols + p.xstage_cols + col) * rows_per + rl] : 0.f;
-        }
-        float g = 0.f, u = 0.f;
-#pragma unroll
-        for (int s = 0; s < 16; ++s) { g += pg[s]; u += pu[s]; }  // the zeros of absent ranks change nothing
-        const int n = n0 + row;
+      for (int e = et; e < todo + et; e += 128) {  // (the same number of turns for every thread)
+        const int col = e >> lg, rl = e & ((1 << lg) - 1);
+        const bool in = got && e < todo;
         float r2 = 0.f;
-        if (n < p.N) r2 = finish(p, col, n, g, u, parity, sc, e == tid - 64 ? pre : Prefetched{false, 0.f, 0.f});
-        if (p.ss_out) sq[e] = r2;  // e = col * rows_per + local row
+        if (in) {
+          // the splits' partial sums in rank order (all loads first)
+          const float* x0 = xs + (col << lg) + rl;
+          const int step = xcols << lg, up = p.xstage_cols << lg;
+          float pg[16], pu[16];
+#pragma unroll
+          for (int s = 0; s < 16; ++s) {
+            pg[s] = s < S ? x0[s * step] : 0.f;
+            pu[s] = (p.dual && s < S) ? x0[s * step + up] : 0.f;
+          }
+          float g = 0.f, u = 0.f;
+#pragma unroll
+          for (int s = 0; s < 16; ++s) { g += pg[s]; u += pu[s]; }  // the zeros of absent ranks change nothing
+          const int n = n0 + (split << lg) + rl;
+          if (n < p.N) r2 = finish(p, col, n, g, u, parity, sc, e == et ? pre : Prefetched{false, 0.f, 0.f});
+        }
+        if (p.ss_out && lg <= 5) {
+          // a token's rows are neighbouring lanes
+          for (int o = 1 << lg >> 1; o; o >>= 1) r2 += __shfl_xor_sync(0xffffffffu, r2, o);
+          if (in && rl == 0) p.ss_out[((int64_t)blockIdx.x * S + split) * 32 + col] = r2;
+        } else if (p.ss_out && in) {
+          sq[e] = r2;
+        }
       }
-      if (p.ss_out) {
+      if (p.ss_out && lg > 5) {
         asm volatile("bar.sync 2, 128;" ::: "memory");
-        const int et = tid - 64;
-        if (et < cols) {
+        if (got && et < min(TN, p.M)) {
           float a = 0.f;
-          for (int i = 0; i < rows_per; ++i) a += sq[et * rows_per + i];
+          for (int i = 0; i < 1 << lg; ++i) a += sq[(et << lg) + i];
           p.ss_out[((int64_t)blockIdx.x * S + split) * 32 + et] = a;
         }
       }
     }
+    __syncwarp();
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+    if (*cta_abort) mbar_wait_cluster(bar_x, 0, cta_abort, p.err);  // (what is still on its way, after a wait gave up)
   }
 
-  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-  __syncthreads();
+  if (p.out_mode == 3) {
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+  }
   if (warp == 1) {
     __syncwarp();
+    if (p.out_mode != 3) asm volatile("bar.sync 3, 160;" ::: "memory");
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_acc), "r"(ncols) : "memory");
   }
   // every thread's pushes precede the barrier above
   if (p.out_mode == 3 && tid == 0) peer_push_done(p.push, (unsigned)p.total_ctas);
-  if (tid == 0) trace_max(p.trace, 3);
+  if (tid == 64) trace_max(p.trace, 3);
 }
 
 template <int TN, int OCC>
@@ -445,7 +564,7 @@ int gemm_dec(cg_ctx* c, const DecGemm& g) {
   const size_t xarea = (size_t)(g.dual ? 2 : 1) * xstage_cols * BM * 4;
   const size_t xbytes = x_in_ring ? 0 : xarea;
   // (with the 8-row box the MMA of the last stage reads 1 KB past its activation slot: keep that inside the allocation)
-  const size_t fixed = 1024 + 16 * 8 + 64 + 128 + (x_rows < tn ? 1024 : 0);
+  const size_t fixed = 1024 + 16 * 8 + 64 + 5 * 128 + (x_rows < tn ? 1024 : 0);
   // (smaller budgets -- 57 or 43 KB, 78 KB for the pair -- were measured 2-5 % slower per step)
   const size_t budget = (g.dual ? 113 * 1024 : 75 * 1024) - fixed;
   int stages = (int)std::max<size_t>(2, (budget > xbytes ? budget - xbytes : 0) / stage);
@@ -468,7 +587,10 @@ int gemm_dec(cg_ctx* c, const DecGemm& g) {
   a.dual = g.dual; a.act = g.act; a.up_off = (int)g.N;
   a.M = (int)g.M; a.N = (int)g.N; a.K = (int)g.K;
   a.kb_total = kb_total; a.kb_per_split = kb_per; a.splits = splits; a.stages = stages;
+  a.lg_rows_per = 0;
+  while (BM >> (a.lg_rows_per + 1) >= splits) ++a.lg_rows_per;
   a.x_rows = x_rows;
+  a.x = (const __nv_bfloat16*)g.x; a.ldx = g.ldx;
   a.xstage_cols = xstage_cols;
   a.xstage_in_ring = x_in_ring && splits > 1 ? 1 : 0;
   a.err = c->core->dev_err;

@@ -234,3 +234,24 @@ def test_resident_decode_kernel_agrees_with_per_operation_path(cuda_bf16, cfg, b
     first_diff = np.argmax(np.concatenate([t_free != toks, np.ones((batch, 1), bool)], axis=1), axis=1)
     assert (first_diff >= 1).all()   # the prefill's token is common to both
     dec.close()
+
+
+@pytest.mark.parametrize("hidden,ffn,vocab", [(328, 1096, 1000), (2048, 8192, 60008), (336, 1096, 2056)], ids=["ragged", "ring", "blocks"])
+@pytest.mark.parametrize("batch", [1, 8, 9, 16, 17, 32])
+def test_decode_step_equals_prompt_at_the_edges_of_its_token_tiles(cuda_bf16, batch, hidden, ffn, vocab):
+    """One cached step (weight-streaming GEMMs: 8, 16 or 32 token columns, k slices over a cluster, one or several
+    passes over the ring, sizes that end inside a 64-wide k block) against the same position of a longer prompt
+    (tiled GEMMs).  Both round the same activations to bf16 and differ by the order of sums, which moves a few of
+    those roundings: 1e-2 of the logits' norm is five roundings of 2^-9; a lost tile, column or slice is of order 1."""
+    C = cuda_bf16
+    cfg = synth.ModelConfig("edges", hidden, ffn, 2, 8, 1, vocab, head_dim=64, rope_theta=500000.0, dtype="bf16")
+    dec = cg.Decoder(C, cfg, max_seq=48, max_batch=batch)
+    dec.load_random(cfg, 3)
+    ids = synth.make_tokens(cfg, batch, 40, seed=batch)
+    dec.prefill(C.from_numpy(np.ascontiguousarray(ids[:, :39])))
+    got = C.to_numpy(dec.step_with(C.from_numpy(np.ascontiguousarray(ids[:, 39])), want_logits=True))
+    picked = dec.tokens()[:, -1]
+    want = C.to_numpy(dec.prefill(C.from_numpy(ids), want_logits=True))
+    dec.close()
+    assert np.linalg.norm(got - want) <= 1e-2 * np.linalg.norm(want)
+    assert (picked == got.argmax(-1)).all()   # (exact: the pick is taken from these logits)
