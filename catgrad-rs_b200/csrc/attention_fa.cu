@@ -1,9 +1,10 @@
-// attention_fa.cu — causal prefill attention on the Blackwell tensor cores (tcgen05 + TMEM),
-// for head sizes 64 and 128 without soft-cap.
+// attention_fa.cu — causal prefill attention on the Blackwell tensor cores (tcgen05 + TMEM): k_attn_fq for head
+// sizes 64, 128 and 256 with or without soft-cap, k_attn_fa for distance biases and gates per value (head
+// sizes 64 and 128) and as the 64-key variant.
 //
 // Same mathematics as attention.cu (catgrad-llm/src/models/llama.rs:97-108 after repeat_kv,
 // catgrad-llm/src/helpers.rs:147-161, as an online-softmax pass over key tiles); what changes
-// is where the two matrix products run:
+// is where the two matrix products run.  k_attn_fa (k_attn_fq's own comment says what it does differently):
 //
 //   warp 0      TMA: the 128-query tile once, then 128-key K and V tiles through two
 //               shared-memory buffers each
@@ -21,6 +22,7 @@
 // Every mbarrier wait is bounded; on expiry the kernel raises the context's error word, all
 // roles leave their loops, TMEM is freed and the kernel returns.
 #include <algorithm>
+#include <type_traits>
 
 #include "act.cuh"
 #include "kernels.h"
@@ -50,6 +52,7 @@ struct FaArgs {
   const float* bias;   // EXTRA: bias[h * ld_bias + distance] is taken off the scores
   int64_t ld_bias;
   float out_scale;
+  float cap_log2e, cap_unit;  // soft-cap c: c log2(e), -2 log2(e) score factor / c
   RowsDev rows;        // rows of unequal length (rows.rows > 0)
   int32_t* err;
 };
@@ -452,24 +455,401 @@ k_attn_fa(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUt
   }
 }
 
-template <int D, int FA_BK, bool EXTRA>
-int launch_fa(cg_ctx* c, const AttnArgs& a) {
-  constexpr size_t smem =
-      (size_t)(D / 64) * (128 + 4 * FA_BK) * 128 + (size_t)(FA_BK / 64) * 128 * 128 + (FA_BK == 64 ? 0 : 1024) + 160 +
-      (EXTRA ? (size_t)2 * 4 * (127 + FA_BK + 9) * 4 : 0);
-  static PerDeviceFlag configured_on;
-  bool& configured = configured_on.at(c->core->device);
-  if (!configured) {
-    CG_CUDA(c, cudaFuncSetAttribute(k_attn_fa<D, FA_BK, EXTRA>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    configured = true;
+// ---- two query tiles per CTA, probabilities and outputs in TMEM -----------------------------------
+//
+// k_attn_fa above is one softmax warpgroup deep: its chain (scores -> maximum -> exponentials -> P V -> fold into
+// registers) leaves the tensor cores idle four fifths of the time.  Here
+//   * NQ = 2 groups of four softmax warps, each with its own 128 queries, take turns on the tensor cores over
+//     the same key tiles: while one group exponentiates, the other's products run;
+//   * P is written back over its scores in TMEM (bf16, two to a column) and is the A operand of P V from there:
+//     no shared memory, no proxy fence, and room for two query tiles beside the key and value ring;
+//   * O stays in TMEM and is accumulated there.  It is rescaled only where a row's maximum has grown by more than
+//     2^8 since the last time: until then the exponentials are taken against the old maximum, which at
+//     most makes them 2^8 times larger (bf16 and f32 keep their relative precision).
+// Head size 256 (with or without soft-cap) has one query tile (its outputs fill half of the TMEM) and two score
+// buffers instead, so that the next scores are computed while this tile's softmax runs.
+// Columns: scores of slot s at s BK (two slots), then O of group w.
+// One layer, before (k_attn_fa; head size 256 k_attn_prefill on mma.sync) -> now: 1 x 8191 tokens, 32 heads of 128: 1196 ->
+// 636 us (864 TFLOP/s); 32 x 509: 321 -> 194; 8 x 512, 32 heads of 64: 56 -> 48; 13 x 389: 79 -> 73; 4 x 2048, 8 heads of
+// 256, soft-cap: 780 -> 145 us (473 TFLOP/s).
+constexpr float FQ_SLACK = 8.f;  // log2 of how far a maximum may grow before the outputs are rescaled
+
+__device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t* v) {
+  asm volatile(
+      "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};" ::"r"(taddr),
+      "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]), "r"(v[8]), "r"(v[9]), "r"(v[10]),
+      "r"(v[11]), "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15])
+      : "memory");
+}
+// A from TMEM (bf16, two consecutive k per column), B from shared memory
+__device__ __forceinline__ void umma_bf16_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t db, uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
+      ::"r"(tmem_d), "r"(tmem_a), "l"(db), "r"(idesc), "r"(accumulate)
+      : "memory");
+}
+__device__ __forceinline__ float fast_rcp(float x) {
+  float y;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+
+template <int D, int BK, int NQ, bool CAP>
+__global__ void __launch_bounds__(128 + NQ * 128, 1)
+k_attn_fq(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
+          const __grid_constant__ CUtensorMap map_v, FaArgs p) {
+  constexpr int SUB = D / 64;
+  constexpr uint32_t BOX = 128 * 128, KBOX = BK * 128;
+  constexpr uint32_t Q_BYTES = SUB * BOX, KV_BYTES = SUB * KBOX;
+  constexpr uint32_t O_COL = 2 * BK, NCOLS = 512;
+  static_assert(O_COL + NQ * D <= NCOLS, "TMEM");
+
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  extern __shared__ __align__(1024) uint8_t smem_raw[];
+  const uint32_t raw = smem_u32(smem_raw);
+  const uint32_t base = (raw + 1023u) & ~1023u;
+  uint8_t* gen = smem_raw + (base - raw);
+  const uint32_t sq = base, sk = sq + NQ * Q_BYTES, sv = sk + 2 * KV_BYTES, bars = sv + 2 * KV_BYTES;
+  const uint32_t b_q_full = bars, b_k_full = bars + 8, b_v_full = bars + 24, b_k_empty = bars + 40, b_v_empty = bars + 56,
+                 b_s_full = bars + 72, b_p_full = bars + 88, b_o_full = bars + 104, b_v_last = bars + 120, b_v_ready = bars + 128;
+  volatile uint32_t* tmem_slot = (volatile uint32_t*)(gen + (bars - base) + 136);
+  volatile int* cta_abort = (volatile int*)(gen + (bars - base) + 140);
+
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int qt = (int)gridDim.x - 1 - (int)blockIdx.x, h = blockIdx.y;  // longest tiles first
+  int64_t b = blockIdx.z, tok0 = b * p.S, len = p.S, start_pos = p.pos0;
+  if (p.rows.rows > 0) {
+    const int row = (int)b;  // (the row tables are written in plain stream order before a prompt's kernels)
+    tok0 = p.rows.start[row];
+    len = p.rows.start[row + 1] - tok0;
+    start_pos = row_pos0(p.rows, row);
+    b = p.rows.slot[row];
   }
-  CUtensorMap mq, mk, mv;
-  CG_TRY(make_map(c, &mq, a.q, a.rows.rows ? a.rows.M : a.B * a.S, (int64_t)a.nh * D, (int64_t)a.nh * D, 128));
+  const int kvh = h / (p.nh / p.nkv);
+  const int64_t q0 = (int64_t)qt * (128 * NQ);
+  if (q0 >= len) return;  // uniform over the CTA, before anything is allocated
+  // key tiles: nk of kept first tokens, then from tile j0 on; group w needs the first nt[w] of them
+  const int j0 = p.window > 0 ? (int)(std::max<int64_t>(0, start_pos + q0 - p.window + 1) / BK) : 0;
+  const int nk = (int)std::min<int64_t>(j0, (p.keep + BK - 1) / BK);
+  auto tiles_to = [&](int64_t q_end) { return nk + (int)((start_pos + std::min<int64_t>(len, q_end) - 1) / BK) + 1 - j0; };
+  const int nt0 = tiles_to(q0 + 128);
+  const int nt1 = NQ == 2 && q0 + 128 < len ? tiles_to(q0 + 256) : 0;
+  const int nt = nt1 > nt0 ? nt1 : nt0;
+  // keys of the last tile that some query of this CTA sees.  What lies behind them (rows of the cache that
+  // nothing or another sequence wrote) is cleared in shared memory: a probability of 0 times an infinity
+  // would not be 0
+  const int seen = (int)(start_pos + std::min<int64_t>(len, q0 + 128 * NQ) - (int64_t)(j0 + nt - 1 - nk) * BK);
+  auto tile_of = [&](int j) { return j < nk ? j : j0 + j - nk; };
+
+  if (tid == 0) {
+    mbar_init(b_q_full, 1);
+    for (int i = 0; i < 2; ++i) {
+      mbar_init(b_k_full + 8 * i, 1);
+      mbar_init(b_v_full + 8 * i, 1);
+      mbar_init(b_k_empty + 8 * i, 1);
+      mbar_init(b_v_empty + 8 * i, 1);
+      mbar_init(b_s_full + 8 * i, 1);
+      mbar_init(b_p_full + 8 * i, 4);  // (a warp each: 128 arrivals on one address take turns)
+      mbar_init(b_o_full + 8 * i, 1);
+    }
+    mbar_init(b_v_last, 1);
+    mbar_init(b_v_ready, 1);
+    *cta_abort = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+  }
+  if (warp == 1) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32((const void*)tmem_slot)),
+                 "r"(NCOLS)
+                 : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  const uint32_t tmem_base = *tmem_slot;
+
+  // q and the cache are written by the preceding kernels
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+
+  if (warp == 0) {
+    if (lane == 0) {
+      const int groups = nt1 > 0 ? 2 : 1;
+      mbar_expect_tx(b_q_full, groups * Q_BYTES);
+      for (int w = 0; w < groups; ++w)
+        for (int s = 0; s < SUB; ++s) tma_load_2d(sq + w * Q_BYTES + s * BOX, &map_q, h * D + s * 64, (int)(tok0 + q0) + w * 128, b_q_full);
+      const int64_t kvrow0 = p.token_major ? b * p.Tmax : (b * p.nkv + kvh) * p.Tmax;
+      const int kx = p.token_major ? kvh * D : 0;
+      for (int j = 0; j < nt; ++j) {
+        const uint32_t buf = (uint32_t)j & 1u, ph = ((uint32_t)j >> 1) & 1u;
+        const int row = (int)(kvrow0 + (int64_t)tile_of(j) * BK);
+        if (j >= 2 && !mbar_wait(b_k_empty + 8 * buf, ph ^ 1u, cta_abort, p.err)) break;
+        mbar_expect_tx(b_k_full + 8 * buf, KV_BYTES);
+        for (int s = 0; s < SUB; ++s) tma_load_2d(sk + buf * KV_BYTES + s * KBOX, &map_k, kx + s * 64, row, b_k_full + 8 * buf);
+        if (j >= 2 && !mbar_wait(b_v_empty + 8 * buf, ph ^ 1u, cta_abort, p.err)) break;
+        mbar_expect_tx(b_v_full + 8 * buf, KV_BYTES);
+        for (int s = 0; s < SUB; ++s) tma_load_2d(sv + buf * KV_BYTES + s * KBOX, &map_v, kx + s * 64, row, b_v_full + 8 * buf);
+      }
+    }
+  } else if (warp == 1) {
+    if (lane == 0) {
+      constexpr uint32_t idesc_s = umma_idesc(BK), idesc_o = umma_idesc(D) | (1u << 16);  // (V: MN-major)
+      const uint64_t dq = umma_desc(sq), dk = umma_desc(sk), dv = umma_desc_mn(sv, KBOX);
+      // the last group that reads tile j frees its buffer (products complete in the order they are issued)
+      auto last = [&](int j) { return j < nt1 ? 1 : 0; };
+      auto slot_of = [&](int w, int j) { return NQ == 2 ? w : j & 1; };
+      auto slot_phase = [&](int j) { return (uint32_t)(NQ == 2 ? j : j >> 1) & 1u; };
+      auto qk = [&](int w, int j) {
+        const uint32_t buf = (uint32_t)j & 1u;
+        if (!mbar_wait(b_k_full + 8 * buf, ((uint32_t)j >> 1) & 1u, cta_abort, p.err)) return false;
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        const int slot = slot_of(w, j);
+#pragma unroll
+        for (int kk = 0; kk < D / UMMA_K; ++kk) {
+          const uint64_t oq = ((uint32_t)(kk / 4) * BOX + (uint32_t)(kk % 4) * 32u) >> 4, ok = ((uint32_t)(kk / 4) * KBOX + (uint32_t)(kk % 4) * 32u) >> 4;
+          umma_bf16(tmem_base + slot * BK, dq + ((w * Q_BYTES) >> 4) + oq, dk + ((buf * KV_BYTES) >> 4) + ok, idesc_s, kk > 0 ? 1u : 0u);
+        }
+        umma_commit(b_s_full + 8 * slot);
+        if (w == last(j)) umma_commit(b_k_empty + 8 * buf);
+        return true;
+      };
+      auto pv = [&](int w, int j) {
+        const uint32_t buf = (uint32_t)j & 1u;
+        const int slot = slot_of(w, j);
+        if (!mbar_wait(b_v_full + 8 * buf, ((uint32_t)j >> 1) & 1u, cta_abort, p.err)) return false;
+        if (j == nt - 1 && seen < BK) {
+          // (warp 2 clears what no query sees while the softmax runs)
+          if (w == 0 || nt0 < nt) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(b_v_last) : "memory");
+          if (!mbar_wait(b_v_ready, 0, cta_abort, p.err)) return false;
+        }
+        if (!mbar_wait(b_p_full + 8 * slot, slot_phase(j), cta_abort, p.err)) return false;
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+#pragma unroll
+        for (int kk = 0; kk < BK / UMMA_K; ++kk)
+          umma_bf16_ts(tmem_base + O_COL + w * D, tmem_base + slot * BK + kk * (UMMA_K / 2), dv + ((buf * KV_BYTES + (uint32_t)kk * (UMMA_K * 128u)) >> 4),
+                       idesc_o, j > 0 || kk > 0 ? 1u : 0u);
+        umma_commit(b_o_full + 8 * w);
+        if (w == last(j)) umma_commit(b_v_empty + 8 * buf);
+        return true;
+      };
+      // Scores overwrite the probabilities that lay in their columns, and products with different accumulators are not
+      // ordered among themselves: the product that reads them is waited for, phase by phase.
+      auto done = [&](int w, int j) { return mbar_wait(b_o_full + 8 * w, (uint32_t)j & 1u, cta_abort, p.err); };
+      bool ok = mbar_wait(b_q_full, 0, cta_abort, p.err) && qk(0, 0);
+      if (NQ == 2) {
+        if (ok && nt1 > 0) ok = qk(1, 0);
+        for (int j = 0; j < nt && ok; ++j) {
+          if (j < nt0) ok = pv(0, j) && (j + 1 >= nt0 || (done(0, j) && qk(0, j + 1)));
+          if (ok && j < nt1) ok = pv(1, j) && (j + 1 >= nt1 || (done(1, j) && qk(1, j + 1)));
+        }
+      } else {
+        for (int j = 0; j < nt && ok; ++j) ok = (j + 1 >= nt || ((j == 0 || done(0, j - 1)) && qk(0, j + 1))) && pv(0, j);
+      }
+    }
+  } else if (warp == 2) {
+    if (seen < BK) {
+      const uint32_t buf = (uint32_t)(nt - 1) & 1u;
+      if (mbar_wait(b_v_last, 0, cta_abort, p.err)) {  // the last values have arrived
+        for (int i = lane; i < SUB * (BK - seen) * 8; i += 32) {
+          const int sub = i / ((BK - seen) * 8), x = i - sub * ((BK - seen) * 8);
+          asm volatile("st.shared.v4.b32 [%0], {%1, %1, %1, %1};" ::"r"(sv + buf * KV_BYTES + sub * KBOX + (uint32_t)seen * 128u + (uint32_t)x * 16u), "r"(0)
+                       : "memory");
+        }
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        __syncwarp();
+        if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(b_v_ready) : "memory");
+      }
+    }
+  } else if (warp >= 4) {
+    const int w = (warp - 4) >> 2, q = warp & 3;
+    const int r = q * 32 + lane;  // query row of this thread = TMEM lane
+    const int mine = w ? nt1 : nt0;
+    const uint32_t lane_base = tmem_base + ((uint32_t)(q * 32) << 16);
+    const uint32_t o_addr = lane_base + O_COL + w * D;
+    const int64_t qw = q0 + w * 128, qi = qw + r, qpos = start_pos + qi;
+    const int64_t last_q = start_pos + std::min<int64_t>(len, qw + 128) - 1;
+    float m = -INFINITY, l = 0.f;  // (m in units of log2: what a score is in the exponent of 2)
+    bool ok = true;
+    for (int j = 0; j < mine && ok; ++j) {
+      const int slot = NQ == 2 ? w : j & 1;
+      ok = mbar_wait(b_s_full + 8 * slot, (uint32_t)(NQ == 2 ? j : j >> 1) & 1u, cta_abort, p.err);
+      if (!ok) break;
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      const int k0 = tile_of(j) * BK;
+      // a key column c of this tile is visible to this row iff low <= c <= lim (window and causal mask)
+      // or c <= lim and c < kept; a bit per column and group of 32
+      const int64_t lim64 = qpos - k0;
+      const int lim = lim64 > BK ? BK : (lim64 < -1 ? -1 : (int)lim64);
+      const int64_t low64 = p.window > 0 ? lim64 - p.window + 1 : 0;
+      const int low = low64 < 0 ? 0 : (low64 > BK ? BK : (int)low64);
+      const int64_t kept64 = p.keep - k0;
+      const int kept = kept64 < 0 ? 0 : (kept64 > BK ? BK : (int)kept64);
+      auto visible = [&](int c) {
+        return bits_below(lim + 1 - c * 32) & (~bits_below(low - c * 32) | bits_below(kept - c * 32));
+      };
+      // uniform: some key may be masked for some row
+      const bool diag = (int64_t)k0 + BK - 1 > start_pos + qw || (p.window > 0 && k0 <= last_q - p.window && kept < BK);
+      const uint32_t s_addr = lane_base + slot * BK;
+      constexpr int NCH = BK / 32;
+      uint32_t va[32], vb[32];
+      // pass 1: row maximum of the visible scores (four chains; chunk c + 1 is in flight while chunk c is reduced)
+      float mx4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
+      // (Both passes are rolled over pairs of chunks: unrolled, with a masked and a plain form each, the loop body left
+      // the instruction cache and prompts of 512 took 21 % longer.)
+      auto largest = [&](int c, const uint32_t* cur) {
+        if (!diag) {
+#pragma unroll
+          for (int i = 0; i < 32; ++i) mx4[i & 3] = fmaxf(mx4[i & 3], __uint_as_float(cur[i]));
+        } else {
+          const uint32_t vis = visible(c);
+#pragma unroll
+          for (int i = 0; i < 32; ++i) mx4[i & 3] = vis & (1u << i) ? fmaxf(mx4[i & 3], __uint_as_float(cur[i])) : mx4[i & 3];
+        }
+      };
+      tmem_ld32(s_addr, va);
+      asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll 1
+      for (int c = 0; c < NCH; c += 2) {
+        tmem_ld32(s_addr + (uint32_t)(c + 1) * 32u, vb);
+        largest(c, va);
+        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+        tmem_ld32(s_addr + (uint32_t)(c + 2 < NCH ? c + 2 : 0) * 32u, va);  // (pass 2 starts from the first chunk again)
+        largest(c + 1, vb);
+        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+      }
+      const float raw_max = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3]));
+      float mx;  // (the soft-cap is monotone)
+      if (CAP) mx = raw_max == -INFINITY ? -INFINITY : fmaf(2.f * p.cap_log2e, fast_rcp(1.f + fast_exp2(raw_max * p.cap_unit)), -p.cap_log2e);
+      else mx = raw_max * p.scale_log2e;
+      if (j == 0) {
+        m = mx;
+      } else {
+        const bool grown = mx > m + FQ_SLACK;
+        if (__any_sync(0xffffffffu, grown)) {
+          const float m_new = grown ? mx : m;
+          const float corr = grown ? fast_exp2(m - m_new) : 1.f;  // 0 while m is -inf
+          // (the product before the last was complete before this tile's scores could be issued, so the parity is that
+          // of the last)
+          ok = mbar_wait(b_o_full + 8 * w, (uint32_t)(j - 1) & 1u, cta_abort, p.err);
+          if (!__all_sync(0xffffffffu, ok)) { ok = false; break; }
+          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+#pragma unroll 1
+          for (int c = 0; c < D; c += 16) {
+            uint32_t t[16];
+            tmem_ld16(o_addr + c, t);
+            asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+            for (int i = 0; i < 16; ++i) t[i] = __float_as_uint(__uint_as_float(t[i]) * corr);
+            tmem_st16(o_addr + c, t);
+          }
+          l *= corr;
+          m = m_new;
+        }
+      }
+      const float mc = m == -INFINITY ? 0.f : m;
+      // pass 2: p = 2^(score - m), row sum, bf16 P over the scores (chunk c's 16 columns end before chunk c + 1's scores)
+      float ls[2] = {0.f, 0.f};
+      auto chunk = [&](int c, const uint32_t* cur, auto masked) {
+        const uint32_t vis = masked.value ? visible(c) : 0u;
+        uint32_t pk[16];
+#pragma unroll
+        for (int i = 0; i < 32; i += 2) {
+          float e[2];
+#pragma unroll
+          for (int t = 0; t < 2; ++t) {
+            const float x = __uint_as_float(cur[i + t]);
+            if (CAP) e[t] = fast_exp2(fmaf(2.f * p.cap_log2e, fast_rcp(1.f + fast_exp2(x * p.cap_unit)), -p.cap_log2e - mc));
+            else e[t] = fast_exp2(fmaf(x, p.scale_log2e, -mc));
+            if (masked.value) e[t] = vis & (1u << (i + t)) ? e[t] : 0.f;
+            ls[t] += e[t];
+          }
+          const __nv_bfloat162 pr = __floats2bfloat162_rn(e[0], e[1]);
+          pk[i / 2] = *(const uint32_t*)&pr;
+        }
+        tmem_st16(s_addr + (uint32_t)c * 16u, pk);
+      };
+      if (diag) {
+#pragma unroll 1
+        for (int c = 0; c < NCH; c += 2) {
+          tmem_ld32(s_addr + (uint32_t)(c + 1) * 32u, vb);
+          chunk(c, va, std::true_type{});
+          asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+          if (c + 2 < NCH) tmem_ld32(s_addr + (uint32_t)(c + 2) * 32u, va);
+          chunk(c + 1, vb, std::true_type{});
+          if (c + 2 < NCH) asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+        }
+      } else {
+#pragma unroll 1
+        for (int c = 0; c < NCH; c += 2) {
+          tmem_ld32(s_addr + (uint32_t)(c + 1) * 32u, vb);
+          chunk(c, va, std::false_type{});
+          asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+          if (c + 2 < NCH) tmem_ld32(s_addr + (uint32_t)(c + 2) * 32u, va);
+          chunk(c + 1, vb, std::false_type{});
+          if (c + 2 < NCH) asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+        }
+      }
+      // (With one group this warp may be a whole product ahead of the tensor core, and a parity tells only neighbouring
+      // phases apart: the last product but one is waited for here, where the last cannot have been issued.)
+      if (NQ == 1 && j > 0 && j + 1 == mine) ok = mbar_wait(b_o_full + 8 * w, (uint32_t)(j - 1) & 1u, cta_abort, p.err);
+      asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+      asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+      __syncwarp();
+      if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(b_p_full + 8 * slot) : "memory");
+      l += ls[0] + ls[1];
+    }
+    if (mine > 0) {
+      ok = ok && mbar_wait(b_o_full + 8 * w, (uint32_t)(mine - 1) & 1u, cta_abort, p.err);
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      float inv = l > 0.f ? 1.f / l : 0.f;
+      if (p.sink) {
+        // one more term of the denominator, without a value
+        const float sk2 = p.sink[h] * LOG2E, top = fmaxf(m, sk2);
+        const float f = fast_exp2(m - top);
+        inv = f / (l * f + fast_exp2(sk2 - top));
+      }
+      const bool out = ok && qi < len;
+      inv *= p.out_scale;
+      if (p.gate && out) inv *= 1.f / (1.f + expf(-p.gate[(tok0 + qi) * p.ld_gate + h]));
+      __nv_bfloat16* dst = p.out + (tok0 + qi) * p.ld_out + (int64_t)h * D;
+#pragma unroll 1
+      for (int c0 = 0; c0 < D; c0 += 32) {
+        uint32_t v[32];
+        tmem_ld32(o_addr + c0, v);
+        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+        if (out) {
+#pragma unroll
+          for (int t = 0; t < 4; ++t) {
+            uint32_t x[4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+              const __nv_bfloat162 pr = __floats2bfloat162_rn(__uint_as_float(v[8 * t + 2 * i]) * inv, __uint_as_float(v[8 * t + 2 * i + 1]) * inv);
+              x[i] = *(const uint32_t*)&pr;
+            }
+            *(uint4*)(dst + c0 + 8 * t) = make_uint4(x[0], x[1], x[2], x[3]);
+          }
+        }
+      }
+    }
+  }
+
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  if (warp == 1) {
+    __syncwarp();
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(NCOLS) : "memory");
+  }
+}
+
+int fa_args(cg_ctx* c, const AttnArgs& a, int D, int BK, CUtensorMap* mq, CUtensorMap* mk, CUtensorMap* mv, FaArgs* args) {
+  CG_TRY(make_map(c, mq, a.q, a.rows.rows ? a.rows.M : a.B * a.S, (int64_t)a.nh * D, (int64_t)a.nh * D, 128));
   const bool tm = a.kv_ld > 0;
   const int64_t kv_rows = tm ? a.B * a.Tmax : a.B * a.nkv * a.Tmax, kv_cols = tm ? (int64_t)a.nkv * D : D, kv_ld = tm ? a.kv_ld : D;
-  CG_TRY(make_map(c, &mk, a.k_cache, kv_rows, kv_cols, kv_ld, FA_BK));
-  CG_TRY(make_map(c, &mv, a.v_cache, kv_rows, kv_cols, kv_ld, FA_BK));
-  FaArgs p;
+  CG_TRY(make_map(c, mk, a.k_cache, kv_rows, kv_cols, kv_ld, BK));
+  CG_TRY(make_map(c, mv, a.v_cache, kv_rows, kv_cols, kv_ld, BK));
+  FaArgs& p = *args;
   p.out = a.out;
   p.S = a.S; p.pos0 = a.pos0; p.Tmax = a.Tmax;
   p.nh = a.nh; p.nkv = a.nkv;
@@ -483,6 +863,46 @@ int launch_fa(cg_ctx* c, const AttnArgs& a) {
   p.ld_out = a.ld_out > 0 ? a.ld_out : (int64_t)a.nh * D;
   p.rows = a.rows;
   p.err = c->core->dev_err;
+  p.cap_log2e = p.cap_unit = 0.f;
+  if (a.softcap > 0.f) {
+    p.cap_log2e = a.softcap * LOG2E;
+    p.cap_unit = -2.f * p.scale_log2e / a.softcap;
+  }
+  return CG_OK;
+}
+
+template <int D, int BK, int NQ, bool CAP>
+int launch_fq(cg_ctx* c, const AttnArgs& a) {
+  constexpr size_t smem = (size_t)(D / 64) * (NQ * 128 + 4 * BK) * 128 + 1024 + 144;
+  static PerDeviceFlag configured_on;
+  bool& configured = configured_on.at(c->core->device);
+  if (!configured) {
+    CG_CUDA(c, cudaFuncSetAttribute(k_attn_fq<D, BK, NQ, CAP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    configured = true;
+  }
+  CUtensorMap mq, mk, mv;
+  FaArgs p;
+  CG_TRY(fa_args(c, a, D, BK, &mq, &mk, &mv, &p));
+  dim3 grid((unsigned)((a.S + 128 * NQ - 1) / (128 * NQ)), (unsigned)a.nh, (unsigned)(a.rows.rows ? a.rows.rows : a.B));
+  CG_CUDA(c, launch_kernel(c, k_attn_fq<D, BK, NQ, CAP>, grid, dim3(128 + NQ * 128), smem, 1, mq, mk, mv, p));
+  CG_LAUNCHED(c);
+  return CG_OK;
+}
+
+template <int D, int FA_BK, bool EXTRA>
+int launch_fa(cg_ctx* c, const AttnArgs& a) {
+  constexpr size_t smem =
+      (size_t)(D / 64) * (128 + 4 * FA_BK) * 128 + (size_t)(FA_BK / 64) * 128 * 128 + (FA_BK == 64 ? 0 : 1024) + 160 +
+      (EXTRA ? (size_t)2 * 4 * (127 + FA_BK + 9) * 4 : 0);
+  static PerDeviceFlag configured_on;
+  bool& configured = configured_on.at(c->core->device);
+  if (!configured) {
+    CG_CUDA(c, cudaFuncSetAttribute(k_attn_fa<D, FA_BK, EXTRA>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    configured = true;
+  }
+  CUtensorMap mq, mk, mv;
+  FaArgs p;
+  CG_TRY(fa_args(c, a, D, FA_BK, &mq, &mk, &mv, &p));
   dim3 grid((unsigned)((a.S + FA_BQ - 1) / FA_BQ), (unsigned)a.nh, (unsigned)(a.rows.rows ? a.rows.rows : a.B));
   CG_CUDA(c, launch_kernel(c, k_attn_fa<D, FA_BK, EXTRA>, grid, dim3(192), smem, 1, mq, mk, mv, p));
   CG_LAUNCHED(c);
@@ -491,8 +911,11 @@ int launch_fa(cg_ctx* c, const AttnArgs& a) {
 
 }  // namespace
 
+// what only k_attn_fa<EXTRA> does
+static bool plain_only(const AttnArgs& a) { return a.bias || (a.gate && a.wide_gate); }
+
 bool attn_fa_supported(const AttnArgs& a) {
-  return (a.d == 64 || a.d == 128) && a.softcap <= 0.f && !a.pos_dev && a.S >= 64 &&
+  return (a.d == 64 || a.d == 128 || a.d == 256) && !(plain_only(a) && (a.softcap > 0.f || a.d == 256)) && !a.pos_dev && a.S >= (plain_only(a) ? 64 : 17) &&
          (a.rows.rows ? a.rows.M : a.B * a.S) < 2147483647ll && a.B * a.nkv * a.Tmax < 2147483647ll && ((uintptr_t)a.q % 16) == 0 &&
          ((uintptr_t)a.k_cache % 16) == 0 && ((uintptr_t)a.v_cache % 16) == 0 && a.kv_ld % 8 == 0 && ((uintptr_t)a.out % 16) == 0 && a.ld_out % 8 == 0 &&
          (!a.wide_gate || (((uintptr_t)a.gate % 16) == 0 && a.ld_gate % 4 == 0));
@@ -500,15 +923,20 @@ bool attn_fa_supported(const AttnArgs& a) {
 
 int k_launch_attn_fa(cg_ctx* c, const AttnArgs& a) {
   if (a.B == 0 || a.S == 0) return CG_OK;
-  // 64-key tiles: two CTAs per SM.  Head size 64 gains from it (8 x 1024 tokens, 64 heads: 380 -> 315 us,
-  // with a window of 128 225 -> 165 us), head size 128 does not (242 -> 264 us).
+  const bool cap = a.softcap > 0.f;
+  // 64-key tiles: two CTAs per SM (asked for by the option; with biases and wide gates head size 64 gains from it)
   const bool k64 = c->opt_fa == 2 || a.d == 64;
-  if (a.bias || (a.gate && a.wide_gate)) {
+  if (plain_only(a)) {
     if (a.d == 64) return launch_fa<64, 64, true>(c, a);
     return k64 ? launch_fa<128, 64, true>(c, a) : launch_fa<128, 128, true>(c, a);
   }
-  if (a.d == 64) return k64 ? launch_fa<64, 64, false>(c, a) : launch_fa<64, 128, false>(c, a);
-  return k64 ? launch_fa<128, 64, false>(c, a) : launch_fa<128, 128, false>(c, a);
+  // 256 queries that share three 128-key tiles see half of each with a short window: 64-key tiles and 128 queries
+  // waste less (8 x 1024 tokens, 64 heads of 64, window 128: 159 us against 175)
+  const bool narrow = a.d == 64 && !cap && a.window > 0 && a.window <= 256;
+  if (narrow || (c->opt_fa == 2 && a.d <= 128 && !cap)) return a.d == 64 ? launch_fa<64, 64, false>(c, a) : launch_fa<128, 64, false>(c, a);
+  if (a.d == 64) return cap ? launch_fq<64, 128, 2, true>(c, a) : launch_fq<64, 128, 2, false>(c, a);
+  if (a.d == 128) return cap ? launch_fq<128, 128, 2, true>(c, a) : launch_fq<128, 128, 2, false>(c, a);
+  return cap ? launch_fq<256, 64, 1, true>(c, a) : launch_fq<256, 64, 1, false>(c, a);
 }
 
 }  // namespace cg

@@ -296,3 +296,26 @@ def test_fused_attention_tcgen05(cuda, b, nh, nkv, s, d, variant):
     np.testing.assert_allclose(got, want, rtol=0, atol=2e-2)
     assert np.abs(got - want).mean() < 3e-3
     np.testing.assert_allclose(got, base, rtol=0, atol=2e-2)
+
+
+@pytest.mark.parametrize("d,window,cap", [(64, 0, 0.0), (128, 0, 0.0), (256, 0, 0.0), (64, 0, 30.0), (128, 100, 30.0), (256, 0, 50.0),
+                                          (256, 100, 50.0), (128, 100, 0.0)])
+@pytest.mark.parametrize("s", [17, 40, 64, 127, 128, 129, 256, 257, 600])
+def test_fused_attention_query_tiles(cuda, d, window, cap, s):
+    """The two-query-tile prefill attention where its tiles end: one tile and none beside it, one row of the second, whole
+    tiles, windows that end inside a tile, growing scores (the outputs' rescaling), against float64.  Each probability and
+    the result are rounded to bf16, 2^-9 of itself: an output, a mean of values, is off by at most 2^-8 of the largest value."""
+    b, nh, nkv = 2, 2, 1
+    q, k, v = (synth.bf16_round(rnd((b, n, s, d))) for n in (nh, nkv, nkv))
+    k = synth.bf16_round(k * np.linspace(0.2, 4.0, s, dtype=np.float32)[:, None])  # maxima that grow along the keys
+    v[:, :, -1] = 3.0
+    got = cuda.to_numpy(cuda.fused_attention(cuda.from_numpy(q), cuda.from_numpy(k), cuda.from_numpy(v), window, cap))
+    sc = np.einsum("bhqd,bhkd->bhqk", q.astype(np.float64), np.repeat(k, nh // nkv, axis=1)) / np.sqrt(d)
+    sc = cap * np.tanh(sc / cap) if cap else sc
+    i = np.arange(s)
+    seen = (i[None, :] <= i[:, None]) & ((i[None, :] > i[:, None] - window) if window else True)
+    sc = np.where(seen, sc, -np.inf)
+    pr = np.exp(sc - sc.max(-1, keepdims=True))
+    want = np.einsum("bhqk,bhkd->bhqd", pr / pr.sum(-1, keepdims=True), np.repeat(v, nh // nkv, axis=1).astype(np.float64))
+    np.testing.assert_allclose(got, want, rtol=0, atol=2.0 ** -8 * np.abs(v).max() + 1e-3)
+    assert np.abs(got - want).mean() < 3e-3
