@@ -973,7 +973,7 @@ static int to_vec(cg_ctx* c, int tag, const cg_tensor* x, void* dst, int64_t n) 
   if (n != x->numel()) return fail(c, CG_ERR_SHAPE, "to_vec: element count differs");
   Hold src;
   CG_TRY(as_contiguous_f32(c, x, &src.t));
-  if (n) CG_CUDA(c, cudaMemcpyAsync(dst, src.t->data(), (size_t)n * 4, cudaMemcpyDeviceToHost, c->core->stream));
+  if (n) CG_CUDA(c, c->core->copy_out(dst, src.t->data(), (size_t)n * 4));
   return cg_sync(c);
 }
 int32_t cg_to_vec_f32(cg_ctx* c, const cg_tensor* x, float* dst, int64_t n) { return to_vec(c, CG_F32, x, dst, n); }

@@ -53,7 +53,15 @@ struct Core {
   std::multimap<size_t, void*> free_blocks;  // size -> ptr, reusable at once: one stream
   int64_t reserved = 0;                      // bytes obtained from cudaMalloc and not returned
   int32_t* dev_err = nullptr;                // device error word (DevErr)
+  // pinned memory that large reads to pageable memory pass through (copy_out); made on first use
+  static constexpr size_t OUT_SEG = size_t(512) << 10;
+  static constexpr int OUT_SLOTS = 16;
+  std::mutex out_mu;
+  char* out_stage = nullptr;                 // [OUT_SLOTS][OUT_SEG]
+  cudaEvent_t out_done[OUT_SLOTS] = {};      // the copy into a slot has arrived
+  bool out_failed = false;                   // no pinned memory to be had: reads go the driver's way
   ~Core();
+  cudaError_t copy_out(void* dst, const void* src, size_t bytes);
   void* alloc(size_t bytes, size_t* got);
   void recycle(void* p, size_t bytes);
   void trim();
