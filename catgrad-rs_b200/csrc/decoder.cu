@@ -165,8 +165,9 @@ __global__ void k_add_rows(float* x, const float* t, int64_t n) {
 }
 
 // The expert block of layer L on M tokens; under tensor parallelism every rank owns whole
-// experts and the partial sums meet in the all-reduce of the residual stream.
-int moe_block(cg_decoder* D, Layer& L, int64_t M, bool push = false) {
+// experts and the partial sums meet in the all-reduce of the residual stream.  next_norm: of the block behind
+// (xn_ready says whether it has been applied).
+int moe_block(cg_decoder* D, Layer& L, int64_t M, bool push = false, const cg_tensor* next_norm = nullptr) {
   const cg_decoder_config& cfg = D->cfg;
   const int64_t P = M * cfg.top_k;
   MoeArgs a;
@@ -224,6 +225,10 @@ int moe_block(cg_decoder* D, Layer& L, int64_t M, bool push = false) {
     px = peer_push_of(D->c->xchg);
     a.push = &px;
     return moe_ffn(D->c, a);
+  }
+  if (next_norm && cfg.tp_world == 1 && ((uintptr_t)next_norm->data() & 15) == 0 && moe_norms_behind(a)) {
+    a.next_gamma = (const float*)next_norm->data();
+    D->xn_ready = true;
   }
   CG_TRY(moe_ffn(D->c, a));
   return all_reduce_f32(D, (float*)D->x->data(), M * D->H);
@@ -346,7 +351,8 @@ bool use_push(cg_decoder* D, int64_t M, int64_t S) {
          M * D->H <= D->c->xchg.max_elems;
 }
 
-// All layers for M = B * S new tokens at positions [pos0, pos0 + S); x holds the embeddings.
+// All layers for M = B * S new tokens at positions [pos0, pos0 + S); x holds the embeddings
+// (embed_rows).
 int run_layers(cg_decoder* D, int64_t B, int64_t S, int64_t pos0, bool from_dev_pos) {
   cg_ctx* c = D->c;
   const cg_decoder_config& cfg = D->cfg;
@@ -452,7 +458,7 @@ int run_layers(cg_decoder* D, int64_t B, int64_t S, int64_t pos0, bool from_dev_
       continue;
     }
     if (L.moe) {
-      CG_TRY(moe_block(D, L, M));
+      CG_TRY(moe_block(D, L, M, false, li + 1 < cfg.num_layers ? D->layers[li + 1].ln_in : nullptr));
       continue;
     }
     if (!D->xn_ready)
@@ -511,9 +517,8 @@ int run_head(cg_decoder* D, int64_t B, int64_t S, bool advance) {
 
 // One decode step for B rows reading position / count from device memory.
 int enqueue_step(cg_decoder* D, int64_t B) {
-  cg_ctx* c = D->c;
   if (D->mixed) return mixed_step(D);
-  CG_TRY(k_launch_embed(c, (const uint32_t*)D->cur->data(), 1, 0, 1, D->embed->data(), D->embed->storage, D->cfg.vocab, B,
+  CG_TRY(k_launch_embed(D->c, (const uint32_t*)D->cur->data(), 1, 0, 1, D->embed->data(), D->embed->storage, D->cfg.vocab, B,
                         D->H, D->cfg.embed_scale > 0.f ? D->cfg.embed_scale : 1.f, (float*)D->x->data()));
   CG_TRY(run_layers(D, B, 1, 0, true));
   return run_head(D, B, 1, true);

@@ -817,7 +817,7 @@ int experts_ff(cg_decoder* D, const MixedLayer& L, int64_t M) {
   a.w.h = (__nv_bfloat16*)X.m_h->data();
   a.w.y = (float*)X.m_y->data();
   CG_TRY(lin(D, X.xn->data(), X.Wp, M, L.router, 0, a.E, a.logits, a.E));
-  CG_TRY(moe_topk(c, a));
+  CG_TRY(moe_choose(c, a, X.f32));
   if (X.f32)
     return moe_experts_f32(c, a, (const float*)X.xn->data(), L.we_gate ? (const float*)L.we_gate->data() : nullptr, (const float*)L.we_up->data(),
                            (const float*)L.we_down->data(), (float*)X.m_h->data());

@@ -270,14 +270,17 @@ struct MoeArgs {
   int add_residual;           // 1: out = x + expert sum; 0: out = this rank's expert sum only
   const PeerPush* push = nullptr;  // tensor-parallel decode: x (= out) first receives the addends pushed by the
                               // preceding row-parallel GEMM, and the expert sum is pushed as the next addend
+  const float* next_gamma = nullptr;  // where moe_norms_behind: xn receives the norm of the result with these gains
   int64_t M;
   __nv_bfloat16* xn;          // [M, H] scratch: the normalised rows
   MoeWork w;
 };
+bool moe_norms_behind(const MoeArgs& a);
 int moe_ffn(cg_ctx* c, const MoeArgs& a);
-// The parts, for callers with normed rows (a.xn) and router logits (a.logits): ids and weights; then the
+// The parts, for callers with normed rows (a.xn) and router logits (a.logits): ids, weights and the plan (f32: of the
+// f32 form); then the
 // experts' results, a.w.y[a.w.pos[pair]] (the weighted sum is the caller's).
-int moe_topk(cg_ctx* c, const MoeArgs& a);
+int moe_choose(cg_ctx* c, const MoeArgs& a, bool f32);
 int moe_experts(cg_ctx* c, const MoeArgs& a);
 // The latter in f32 (h [pairs, Fe]; a.w.xg holds 2 [pairs] words; w_gate null: not gated)
 int moe_experts_f32(cg_ctx* c, const MoeArgs& a, const float* x, const float* w_gate, const float* w_up, const float* w_down, float* h);

@@ -186,21 +186,67 @@ __global__ void k_moe_norm_split(float* x, const float* gamma, float eps, int pl
   }
 }
 
+// The same (no REDUCE) with the row in registers: every load is issued at once, the gains (weights) before the dependency.
+// Eight rows of 2048 in a step: 8.3 -> 3.5 us (four layers of the Qwen3-30B-A3B shape, 688 -> 669 us a step).
+constexpr int NSP_THREADS = 256, NSP_VECS = 8;
+__global__ void __launch_bounds__(NSP_THREADS)
+k_moe_norm_split_vec(const float* x, const float* gamma, float eps, int plus_one, int H, __nv_bfloat16* xn, __nv_bfloat16* xs3) {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  __shared__ float red[32];
+  const int64_t m = blockIdx.x;
+  const int n4 = H / 4, tid = threadIdx.x;
+  const float one = plus_one ? 1.f : 0.f;
+  float4 g[NSP_VECS], v[NSP_VECS];
+#pragma unroll
+  for (int j = 0; j < NSP_VECS; ++j) {
+    const int i = tid + j * NSP_THREADS;
+    g[j] = gamma && i < n4 ? __ldg((const float4*)gamma + i) : make_float4(0.f, 0.f, 0.f, 0.f);
+  }
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+#pragma unroll
+  for (int j = 0; j < NSP_VECS; ++j) {
+    const int i = tid + j * NSP_THREADS;
+    v[j] = i < n4 ? ((const float4*)(x + m * H))[i] : make_float4(0.f, 0.f, 0.f, 0.f);
+  }
+  float ss = 0.f;
+#pragma unroll
+  for (int j = 0; j < NSP_VECS; ++j) ss += v[j].x * v[j].x + v[j].y * v[j].y + v[j].z * v[j].z + v[j].w * v[j].w;
+  const float rms = sqrtf(block_sum_f(ss, red) / (float)H + eps);
+  __nv_bfloat16* o3 = xs3 + m * 3 * H;
+#pragma unroll
+  for (int j = 0; j < NSP_VECS; ++j) {
+    const int i = tid + j * NSP_THREADS;
+    if (i >= n4) break;
+    const float in[4] = {v[j].x, v[j].y, v[j].z, v[j].w}, gg[4] = {g[j].x, g[j].y, g[j].z, g[j].w};
+    __nv_bfloat16 part[3][4];
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const float r0 = gamma ? in[e] / rms * (one + gg[e]) : in[e];
+      part[0][e] = __float2bfloat16_rn(r0);
+      const float r1 = r0 - __bfloat162float(part[0][e]);
+      part[1][e] = __float2bfloat16_rn(r1);
+      part[2][e] = __float2bfloat16_rn(r1 - __bfloat162float(part[1][e]));
+    }
+    uint2 w[3];
+#pragma unroll
+    for (int q = 0; q < 3; ++q) {
+      const __nv_bfloat162 lo = __halves2bfloat162(part[q][0], part[q][1]), hi = __halves2bfloat162(part[q][2], part[q][3]);
+      w[q] = make_uint2(*(const uint32_t*)&lo, *(const uint32_t*)&hi);
+      ((uint2*)(o3 + q * (int64_t)H))[i] = w[q];
+    }
+    ((uint2*)(xn + m * H))[i] = w[0];
+  }
+}
+
 // One warp per token: softmax over the router logits (or the sigmoid of each), top-k (ties -> lower expert
 // id), optional renormalisation, times scale.  With `correction` [E] the experts are chosen by probability + correction
 // and weighted by probability.  Dynamic shared memory: E floats per warp, 2 E with correction.
 constexpr uint32_t TAKEN = 0xFFFFFFFFu;  // a chosen expert's mark (a NaN no sum here produces)
-__global__ void k_moe_topk(const float* logits, int64_t M, int E, int k, int norm_topk, int sigmoid, const float* correction,
-                           float scale, uint32_t* ids, float* wts) {
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-  asm volatile("griddepcontrol.wait;" ::: "memory");
-  extern __shared__ float sm[];
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  const int64_t m = (int64_t)blockIdx.x * nw + wid;
-  if (m >= M) return;
-  float* pr = sm + (size_t)wid * E * (correction ? 2 : 1);
+// Lane r < k receives the expert of slot r and its weight; pr: the warp's shared memory.
+__device__ __forceinline__ void topk_of_row(const float* lg, int E, int k, int norm_topk, int sigmoid, const float* correction, float scale,
+                                            float* pr, uint32_t* id, float* weight) {
+  const int lane = threadIdx.x & 31;
   float* ch = correction ? pr + E : pr;  // what the choice goes by
-  const float* lg = logits + m * E;
   float mx = -3.4028234663852886e38f;
   for (int e = lane; e < E; e += 32) {
     const float v = lg[e];
@@ -244,22 +290,33 @@ __global__ void k_moe_topk(const float* logits, int64_t M, int E, int k, int nor
     __syncwarp();
   }
   total = sum_in_reference_order(chosen, k);  // bit-identical to the reference's sum over the k values
+  *id = chosen_id;
+  *weight = (norm_topk ? chosen / total : chosen) * scale;
+}
+__global__ void k_moe_topk(const float* logits, int64_t M, int E, int k, int norm_topk, int sigmoid, const float* correction,
+                           float scale, uint32_t* ids, float* wts) {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  extern __shared__ float sm[];
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  const int64_t m = (int64_t)blockIdx.x * nw + wid;
+  if (m >= M) return;
+  uint32_t id;
+  float w;
+  topk_of_row(logits + m * E, E, k, norm_topk, sigmoid, correction, scale, sm + (size_t)wid * E * (correction ? 2 : 1), &id, &w);
   if (lane < k) {
-    ids[m * k + lane] = chosen_id;
-    wts[m * k + lane] = (norm_topk ? chosen / total : chosen) * scale;
+    ids[m * k + lane] = id;
+    wts[m * k + lane] = w;
   }
 }
 
-// One block of at least El threads (El <= 1024).  Counts the pairs routed to experts
+// A block of at least El threads (El <= 1024; sh_i: 2 El ints).  Counts the pairs routed to experts
 // [e_lo, e_lo + El), lays the groups out back to back, lists the GEMM tiles (tn rows each,
 // never crossing a group) and gives every pair its row (or -1 when another rank owns its
 // expert).  Thread e owns expert e: two block-wide prefix sums give its first row and its
 // first tile.
-__global__ void k_moe_plan(const uint32_t* ids, int P, int e_lo, int El, int tn, int32_t* pos, int32_t* tile_expert,
-                           int32_t* tile_row0, int32_t* tile_rows, int32_t* n_tiles) {
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-  asm volatile("griddepcontrol.wait;" ::: "memory");
-  extern __shared__ int sh_i[];
+__device__ __forceinline__ void plan_block(const uint32_t* ids, int P, int e_lo, int El, int tn, int* sh_i, int32_t* pos, int32_t* tile_expert,
+                                           int32_t* tile_row0, int32_t* tile_rows, int32_t* n_tiles) {
   int* cnt = sh_i;          // [El]
   int* cur = sh_i + El;     // [El]
   __shared__ int wsum_rows[32], wsum_tiles[32];
@@ -306,6 +363,41 @@ __global__ void k_moe_plan(const uint32_t* ids, int P, int e_lo, int El, int tn,
     const int e = (int)ids[p] - e_lo;
     pos[p] = (e >= 0 && e < El) ? atomicAdd(&cur[e], 1) : -1;
   }
+}
+
+__global__ void k_moe_plan(const uint32_t* ids, int P, int e_lo, int El, int tn, int32_t* pos, int32_t* tile_expert,
+                           int32_t* tile_row0, int32_t* tile_rows, int32_t* n_tiles) {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  extern __shared__ int sh_i[];
+  plan_block(ids, P, e_lo, El, tn, sh_i, pos, tile_expert, tile_row0, tile_rows, n_tiles);
+}
+
+// Both in one block for a step's few tokens (a warp per token, then the plan out of shared memory): two dependent
+// launches of one small block each cost a step 2 us per layer more than one (with k_moe_combine_norm: four layers of the
+// Qwen3-30B-A3B shape, batch 8, 703 -> 688 us a step).
+__global__ void __launch_bounds__(1024)
+k_moe_topk_plan(const float* logits, int M, int E, int k, int norm_topk, int sigmoid, const float* correction, float scale,
+                uint32_t* ids, float* wts, int e_lo, int El, int tn, int32_t* pos, int32_t* tile_expert, int32_t* tile_row0,
+                int32_t* tile_rows, int32_t* n_tiles) {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  extern __shared__ float sm[];
+  int* sh_i = (int*)sm;                          // [2 El] the plan's
+  uint32_t* chosen = (uint32_t*)(sh_i + 2 * El);  // [M k]
+  float* pr = (float*)(chosen + M * k);          // [M][E or 2 E]
+  const int lane = threadIdx.x & 31, m = threadIdx.x >> 5;
+  if (m < M) {
+    uint32_t id;
+    float w;
+    topk_of_row(logits + (int64_t)m * E, E, k, norm_topk, sigmoid, correction, scale, pr + (size_t)m * E * (correction ? 2 : 1), &id, &w);
+    if (lane < k) {
+      ids[m * k + lane] = chosen[m * k + lane] = id;
+      wts[m * k + lane] = w;
+    }
+  }
+  __syncthreads();
+  plan_block(chosen, M * k, e_lo, El, tn, sh_i, pos, tile_expert, tile_row0, tile_rows, n_tiles);
 }
 
 // xg[pos[p], :] = xn[p / k, :] (bf16 rows of H elements, H % 8 == 0)
@@ -386,6 +478,56 @@ __global__ void k_moe_combine(const float* y, const int32_t* pos, const float* w
   }
 }
 
+// out[t, :] = x[t, :] + the sum of k_moe_combine, and the norm the next block starts with, bf16(out / rms * gamma)
+// (k_rmsnorm's arithmetic): a block per token, its row in registers.  One dependent launch less per layer of a step
+// (with k_moe_topk_plan 703 -> 688 us for four layers); a prompt saves the norm's read of the residual stream.
+constexpr int CN_THREADS = 256, CN_VECS = 8;
+__global__ void __launch_bounds__(CN_THREADS)
+k_moe_combine_norm(const float* y, const int32_t* pos, const float* wts, int k, int H, const float* x, float* out, const float* gamma,
+                   float eps, int plus_one, __nv_bfloat16* xn) {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  __shared__ float red[32], sw[32];
+  __shared__ int sp[32];
+  const int64_t t = blockIdx.x;
+  const int tid = threadIdx.x, per = H / 4;
+  if (tid < k) {
+    sp[tid] = pos[t * k + tid];
+    sw[tid] = wts[t * k + tid];
+  }
+  __syncthreads();
+  float4 v[CN_VECS];
+  float ss = 0.f;
+#pragma unroll
+  for (int i = 0; i < CN_VECS; ++i) {
+    const int j = tid + i * CN_THREADS;
+    if (j >= per) break;
+    const float4 b = ((const float4*)(x + t * H))[j];
+    float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 8
+    for (int s = 0; s < k; ++s) {
+      if (sp[s] < 0) continue;
+      const float4 u = ((const float4*)(y + (int64_t)sp[s] * H))[j];
+      const float w = sw[s];
+      acc.x += u.x * w; acc.y += u.y * w; acc.z += u.z * w; acc.w += u.w * w;
+    }
+    acc.x += b.x; acc.y += b.y; acc.z += b.z; acc.w += b.w;
+    v[i] = acc;
+    ((float4*)(out + t * H))[j] = acc;
+    ss += acc.x * acc.x + acc.y * acc.y + acc.z * acc.z + acc.w * acc.w;
+  }
+  const float rms = sqrtf(block_sum_f(ss, red) / (float)H + eps);
+#pragma unroll
+  for (int i = 0; i < CN_VECS; ++i) {
+    const int j = tid + i * CN_THREADS;
+    if (j >= per) break;
+    float4 g = ((const float4*)gamma)[j];
+    if (plus_one) { g.x += 1.f; g.y += 1.f; g.z += 1.f; g.w += 1.f; }
+    const __nv_bfloat162 a = __floats2bfloat162_rn(v[i].x / rms * g.x, v[i].y / rms * g.y), b = __floats2bfloat162_rn(v[i].z / rms * g.z, v[i].w / rms * g.w);
+    ((uint2*)(xn + t * H))[j] = make_uint2(*(const uint32_t*)&a, *(const uint32_t*)&b);
+  }
+}
+
 struct MoeGemmArgs {
   const int32_t* tile_expert;
   const int32_t* tile_row0;
@@ -448,6 +590,14 @@ k_moe_gemm(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CU
     *cta_abort = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    // weights of the first stages: no dependency, and no need for TMEM or the other warps
+    for (int i = 0; i < min(nkb, STAGES); ++i) {
+      const uint32_t full = bars + 8 * i;
+      const uint32_t a = base + i * STAGE_BYTES;
+      mbar_expect_tx(full, W_BYTES);
+      tma_load_2d(a, &map_w, i * BK, wrow, full);
+      if (DUAL) tma_load_2d(a + A_BYTES, &map_u, i * BK, wrow, full);
+    }
   }
   if (warp == 1) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32((const void*)tmem_slot)),
@@ -464,13 +614,6 @@ k_moe_gemm(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CU
   if (warp == 0) {
     if (lane == 0) {
       const int pre = min(nkb, STAGES);
-      for (int i = 0; i < pre; ++i) {  // weights of the first stages: no dependency
-        const uint32_t full = bars + 8 * i;
-        const uint32_t a = base + i * STAGE_BYTES;
-        mbar_expect_tx(full, W_BYTES);
-        tma_load_2d(a, &map_w, i * BK, wrow, full);
-        if (DUAL) tma_load_2d(a + A_BYTES, &map_u, i * BK, wrow, full);
-      }
       asm volatile("griddepcontrol.wait;" ::: "memory");
       for (int i = 0; i < nkb; ++i) {
         const int s = i % STAGES;
@@ -491,21 +634,28 @@ k_moe_gemm(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CU
   } else if (warp == 1) {
     if (lane == 0) {
       constexpr uint32_t idesc = umma_idesc(TN);
+      const uint64_t da0 = umma_desc(base), db0 = umma_desc(base + W_BYTES);  // of slot 0
+      constexpr uint64_t DK = UMMA_K * 2 >> 4, DUP = A_BYTES >> 4;
+      uint64_t off = 0;
+      int sl = 0;
+      uint32_t par = 0;
       bool ok = true;
-      for (int i = 0; i < nkb && ok; ++i) {
-        const int s = i % STAGES;
-        const uint32_t ph = (uint32_t)(i / STAGES) & 1u;
-        ok = mbar_wait(bars + 8 * s, ph, cta_abort, p.err);
+      for (int i = 0; i < nkb; ++i) {
+        ok = mbar_wait(bars + 8 * sl, par, cta_abort, p.err);
         if (!ok) break;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        const uint32_t a = base + s * STAGE_BYTES;
+        const uint64_t da = da0 + off, db = db0 + off;
+        umma_bf16(tmem_acc, da, db, idesc, i > 0 ? 1u : 0u);
 #pragma unroll
-        for (int kk = 0; kk < BK / UMMA_K; ++kk) {
-          const uint64_t db = umma_desc(a + W_BYTES + kk * UMMA_K * 2);
-          umma_bf16(tmem_acc, umma_desc(a + kk * UMMA_K * 2), db, idesc, (i > 0 || kk > 0) ? 1u : 0u);
-          if (DUAL) umma_bf16(tmem_acc + TN, umma_desc(a + A_BYTES + kk * UMMA_K * 2), db, idesc, (i > 0 || kk > 0) ? 1u : 0u);
+        for (int kk = 1; kk < BK / UMMA_K; ++kk) umma_bf16_acc(tmem_acc, da + kk * DK, db + kk * DK, idesc);
+        if (DUAL) {
+          umma_bf16(tmem_acc + TN, da + DUP, db, idesc, i > 0 ? 1u : 0u);
+#pragma unroll
+          for (int kk = 1; kk < BK / UMMA_K; ++kk) umma_bf16_acc(tmem_acc + TN, da + DUP + kk * DK, db + kk * DK, idesc);
         }
-        umma_commit(bars + 8 * (STAGES + s));
+        if (i + STAGES < nkb) umma_commit(bars + 8 * (STAGES + sl));  // (nobody waits for a slot's last use)
+        off += STAGE_BYTES >> 4;
+        if (++sl == STAGES) { sl = 0; par ^= 1u; off = 0; }
       }
       if (ok) umma_commit(bar_accum);
     }
@@ -658,6 +808,12 @@ int launch_moe_gemm(cg_ctx* c, const CUtensorMap& mw, const CUtensorMap& mu, con
 }  // namespace
 
 static int launch_combine(cg_ctx* c, const MoeArgs& a) {
+  if (a.next_gamma) {
+    CG_CUDA(c, launch_kernel(c, k_moe_combine_norm, dim3((unsigned)a.M), dim3(CN_THREADS), 0, 1, (const float*)a.w.y, (const int32_t*)a.w.pos,
+                             (const float*)a.w.wts, a.k, a.H, a.x, a.out, a.next_gamma, a.eps, a.plus_one, a.xn));
+    CG_LAUNCHED(c);
+    return CG_OK;
+  }
   const dim3 grid(grid_for(a.M * (a.H / 4), 256));
   if (a.push) {
     if (a.M * a.H > a.push->max_elems) return fail(c, CG_ERR_INVALID, "moe: rows do not fit the exchange area");
@@ -718,26 +874,52 @@ static int launch_plan(cg_ctx* c, const MoeArgs& a, int tn) {
   return CG_OK;
 }
 
-int moe_topk(cg_ctx* c, const MoeArgs& a) {
+// Choice and plan in one launch where one block has a warp for every token and a thread for every expert
+// (decode steps: at most 32 tokens; 1024 threads) and its rows fit the shared memory that needs no opt-in.
+static size_t ride_smem(const MoeArgs& a) {
+  return (size_t)2 * a.El * 4 + (size_t)a.M * a.k * 4 + (size_t)a.M * a.E * (a.correction ? 8 : 4);
+}
+static bool plan_rides(const MoeArgs& a) { return a.M <= 32 && ride_smem(a) <= 48 * 1024; }
+
+static int launch_choice(cg_ctx* c, const MoeArgs& a, int tn) {
+  if (!plan_rides(a)) {
+    CG_TRY(launch_topk(c, a));
+    return launch_plan(c, a, tn);
+  }
+  const unsigned threads = (unsigned)std::max<int64_t>({128, 32 * a.M, (a.El + 31) / 32 * 32});
+  CG_CUDA(c, launch_kernel(c, k_moe_topk_plan, dim3(1), dim3(threads), ride_smem(a), 1, (const float*)a.logits, (int)a.M, a.E, a.k, a.norm_topk,
+                           a.sigmoid, a.correction, a.router_scale, a.w.ids, a.w.wts, a.e_lo, a.El, tn, a.w.pos, a.w.tile_expert,
+                           a.w.tile_row0, a.w.tile_rows, a.w.n_tiles));
+  CG_LAUNCHED(c);
+  return CG_OK;
+}
+
+int moe_choose(cg_ctx* c, const MoeArgs& a, bool f32) {
   if (a.M == 0) return CG_OK;
   CG_TRY(check_moe(c, a));
-  return launch_topk(c, a);
+  return launch_choice(c, a, f32 ? MF_ROWS : moe_pick_tn(a.M * a.k, a.E));
 }
+
+bool moe_norms_behind(const MoeArgs& a) { return !a.push && a.add_residual && a.H <= CN_THREADS * CN_VECS * 4; }
 
 int moe_ffn(cg_ctx* c, const MoeArgs& a) {
   if (a.M == 0) return CG_OK;
   CG_TRY(check_moe(c, a));
+  if (a.next_gamma && !moe_norms_behind(a)) return fail(c, CG_ERR_INVALID, "moe: this form has no norm behind it");
   if (a.push && !a.router3) return fail(c, CG_ERR_INVALID, "moe: the pushed reduction needs the bf16 router path");
   if (a.router3) {
     if (a.push)
       CG_CUDA(c, launch_kernel(c, k_moe_norm_split<1>, dim3((unsigned)a.M), dim3(256), 0, 1, a.out, a.gamma, a.eps, a.plus_one, a.H,
                                a.xn, a.xs3, *a.push, c->core->dev_err));
+    else if (a.H <= NSP_THREADS * NSP_VECS * 4 && (((uintptr_t)a.x | (uintptr_t)a.gamma) & 15) == 0)
+      CG_CUDA(c, launch_kernel(c, k_moe_norm_split_vec, dim3((unsigned)a.M), dim3(NSP_THREADS), 0, 1, a.x, a.gamma, a.eps, a.plus_one, a.H,
+                               a.xn, a.xs3));
     else
       CG_CUDA(c, launch_kernel(c, k_moe_norm_split<0>, dim3((unsigned)a.M), dim3(256), 0, 1, const_cast<float*>(a.x), a.gamma, a.eps,
                                a.plus_one, a.H, a.xn, a.xs3, PeerPush{}, c->core->dev_err));
     CG_LAUNCHED(c);
     CG_TRY(router_logits(c, a, a.xs3, a.router3, 3 * (int64_t)a.H));
-    CG_TRY(launch_topk(c, a));
+    CG_TRY(moe_choose(c, a, false));
   } else {
     const size_t smem = (size_t)(a.H + a.E) * 4;
     static PerDeviceSize configured_on;
@@ -749,6 +931,7 @@ int moe_ffn(cg_ctx* c, const MoeArgs& a) {
     CG_CUDA(c, launch_kernel(c, k_moe_route, dim3((unsigned)a.M), dim3(256), smem, 1, a.x, a.gamma, a.eps, a.plus_one, a.router,
                              a.H, a.E, a.k, a.norm_topk, a.xn, a.w.ids, a.w.wts));
     CG_LAUNCHED(c);
+    CG_TRY(launch_plan(c, a, moe_pick_tn(a.M * a.k, a.E)));
   }
   CG_TRY(moe_experts(c, a));
   return launch_combine(c, a);
@@ -761,7 +944,6 @@ int moe_experts(cg_ctx* c, const MoeArgs& a) {
   const int tn = moe_pick_tn(P, a.E);
   const int64_t max_tiles = moe_max_tiles(P, a.El, tn);
   if (max_tiles > 65535) return fail(c, CG_ERR_UNSUPPORTED, "moe: too many tiles");
-  CG_TRY(launch_plan(c, a, tn));
   if (a.weigh_input)
     CG_CUDA(c, launch_kernel(c, k_moe_gather_weighted, dim3(grid_for(P * (a.H / 8), 256)), dim3(256), 0, 1, a.x, (const float*)a.w.wts,
                              (const int32_t*)a.w.pos, P, a.k, a.H, a.w.xg));
@@ -822,7 +1004,6 @@ int moe_experts(cg_ctx* c, const MoeArgs& a) {
 int moe_experts_f32(cg_ctx* c, const MoeArgs& a, const float* x, const float* w_gate, const float* w_up, const float* w_down, float* h) {
   if (a.M == 0) return CG_OK;
   CG_TRY(check_moe(c, a));
-  CG_TRY(launch_plan(c, a, MF_ROWS));
   const int64_t P = a.M * a.k, tiles = moe_max_tiles(P, a.El, MF_ROWS);
   if (tiles > 65535) return fail(c, CG_ERR_UNSUPPORTED, "moe: too many tiles");
   // rows in grouped order: which token each reads

@@ -61,6 +61,15 @@ def test_fused_moe_matches_op_stream(oracle, cuda_bf16, S, H, E, Fe, k, renorm):
     assert np.abs(got - want).max() <= 1e-2 * scale + 1e-6, float(np.abs(got - want).max() / scale)
 
 
+# choice and plan in one block: its last token count and the first of the two launches, more experts than tokens'
+# threads, rows that fill its shared memory and the first that do not, a hidden size that ends inside a block's walk
+@pytest.mark.gpu
+@pytest.mark.parametrize("S,H,E,Fe,k", [(31, 72, 16, 32, 3), (32, 72, 16, 32, 3), (33, 72, 16, 32, 3), (2, 64, 700, 8, 32), (32, 64, 340, 8, 2),
+                                        (32, 64, 372, 8, 2), (1, 1032, 8, 32, 8)])
+def test_fused_moe_choice_and_plan(oracle, cuda_bf16, S, H, E, Fe, k):
+    test_fused_moe_matches_op_stream(oracle, cuda_bf16, S, H, E, Fe, k, True)
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("S,H,E,Fe,k,renorm", [CASES[1], CASES[5]])
 def test_fused_moe_f32_router(oracle, cuda, S, H, E, Fe, k, renorm):
