@@ -351,6 +351,19 @@ bool use_push(cg_decoder* D, int64_t M, int64_t S) {
          M * D->H <= D->c->xchg.max_elems;
 }
 
+// x = the embeddings of M tokens, and where the table allows it the norm that the first layer starts with (xn_ready).
+int embed_rows(cg_decoder* D, const uint32_t* tokens, int64_t tok_ld, int64_t tok_off, int64_t S, int64_t M) {
+  const cg_decoder_config& cfg = D->cfg;
+  const float scale = cfg.embed_scale > 0.f ? cfg.embed_scale : 1.f;
+  const float* gamma = (const float*)D->layers[0].ln_in->data();
+  D->xn_ready = embed_norm_supported(D->embed->data(), D->embed->storage, gamma, D->H);
+  if (D->xn_ready)
+    return k_launch_embed_norm(D->c, tokens, tok_ld, tok_off, S, D->embed->data(), cfg.vocab, M, D->H, scale, gamma, cfg.rms_eps,
+                               cfg.norm_plus_one, (float*)D->x->data(), (__nv_bfloat16*)D->xn->data());
+  return k_launch_embed(D->c, tokens, tok_ld, tok_off, S, D->embed->data(), D->embed->storage, cfg.vocab, M, D->H, scale,
+                        (float*)D->x->data());
+}
+
 // All layers for M = B * S new tokens at positions [pos0, pos0 + S); x holds the embeddings
 // (embed_rows).
 int run_layers(cg_decoder* D, int64_t B, int64_t S, int64_t pos0, bool from_dev_pos) {
@@ -363,7 +376,6 @@ int run_layers(cg_decoder* D, int64_t B, int64_t S, int64_t pos0, bool from_dev_
   // norm hand-over between GEMMs: decode steps of pre-norm models on one GPU
   const bool handover = c->opt_handover && S == 1 && small_m(M, D->H) && cfg.tp_world == 1 && !cfg.post_norms;
   D->xn_raw = false;
-  D->xn_ready = false;
   for (int li = 0; li < cfg.num_layers; ++li) {
     Layer& L = D->layers[li];
     const bool small = small_m(M, D->H);
@@ -518,8 +530,7 @@ int run_head(cg_decoder* D, int64_t B, int64_t S, bool advance) {
 // One decode step for B rows reading position / count from device memory.
 int enqueue_step(cg_decoder* D, int64_t B) {
   if (D->mixed) return mixed_step(D);
-  CG_TRY(k_launch_embed(D->c, (const uint32_t*)D->cur->data(), 1, 0, 1, D->embed->data(), D->embed->storage, D->cfg.vocab, B,
-                        D->H, D->cfg.embed_scale > 0.f ? D->cfg.embed_scale : 1.f, (float*)D->x->data()));
+  CG_TRY(embed_rows(D, (const uint32_t*)D->cur->data(), 1, 0, 1, B));
   CG_TRY(run_layers(D, B, 1, 0, true));
   return run_head(D, B, 1, true);
 }
@@ -964,8 +975,7 @@ int prefill_at(cg_decoder* D, const cg_tensor* tokens, int64_t base, int64_t gen
   CG_TRY(ensure_workspace(D, B * Sc));
   for (int64_t p0 = 0; p0 < S; p0 += Sc) {
     const int64_t s = std::min(Sc, S - p0);
-    CG_TRY(k_launch_embed(c, (const uint32_t*)tk.t->data(), S, p0, s, D->embed->data(), D->embed->storage, D->cfg.vocab,
-                          B * s, D->H, D->cfg.embed_scale > 0.f ? D->cfg.embed_scale : 1.f, (float*)D->x->data()));
+    CG_TRY(embed_rows(D, (const uint32_t*)tk.t->data(), S, p0, s, B * s));
     // a one-token chunk would take the decode attention path, which reads the device position
     if (s == 1) CG_TRY(set_state(D, base + p0, generated));
     CG_TRY(run_layers(D, B, s, base + p0, s == 1));

@@ -13,6 +13,10 @@ namespace cg {
 // tokens[b * tok_ld + tok_off + s]: a window of S positions out of a [B, tok_ld] id matrix.
 int k_launch_embed(cg_ctx* c, const uint32_t* tokens, int64_t tok_ld, int64_t tok_off, int64_t S, const void* table,
                    int table_storage, int64_t vocab, int64_t M, int64_t H, float scale, float* out);
+// the same with the norm behind it: xn = bf16(out / rms * gamma)
+bool embed_norm_supported(const void* table, int st, const float* gamma, int64_t H);
+int k_launch_embed_norm(cg_ctx* c, const uint32_t* tokens, int64_t tok_ld, int64_t tok_off, int64_t S, const void* table, int64_t vocab,
+                        int64_t M, int64_t H, float scale, const float* gamma, float eps, int plus_one, float* out, __nv_bfloat16* xn);
 
 // RMSNorm of each row of x [M, H] (row stride ldx): out = x / sqrt(mean(x^2) + eps) * g, g = gamma or 1 + gamma.
 // out_bf16 selects the output element type (bf16 feeds the tensor-core GEMMs).
