@@ -233,16 +233,29 @@ __global__ void __launch_bounds__(256, RD_ROWS <= 8 ? 3 : 2) k_recur_decode(Recu
   const int lpr = a.dvs / 4, rpp = 256 / lpr;         // threads per state row, rows per pass
   const int rg = tid / lpr, cg = tid - rg * lpr;
   const bool act = rg < rpp;
-  asm volatile("griddepcontrol.wait;" ::: "memory");
-  const int64_t m = row, pos = row_pos0(a.rows, row);
+  // The state is on its way while the projection still runs.  Its last writer is this layer run's kernel of the step
+  // before, and the step counter is raised (behind its own dependency wait) only when that step's kernels are
+  // complete: if the counter read here is still the one behind the wait, what was read is what they left;
+  // else the step before was not over, and the state is read again.
   const int slot = a.rows.slot[row];
   float* Sg = a.S + ((int64_t)slot * a.H + h) * a.dk * a.dvs;
   float4 S[RD_ROWS];
+  auto load_state = [&](bool any) {
 #pragma unroll
-  for (int i = 0; i < RD_ROWS; ++i) {
-    const int r = rg + i * rpp;
-    S[i] = act && r < a.dk && pos > 0 ? *(const float4*)(Sg + (int64_t)r * a.dvs + 4 * cg) : make_float4(0.f, 0.f, 0.f, 0.f);
-  }
+    for (int i = 0; i < RD_ROWS; ++i) {
+      const int r = rg + i * rpp;
+      S[i] = act && r < a.dk && any ? __ldcg((const float4*)(Sg + (int64_t)r * a.dvs + 4 * cg)) : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+  };
+  int64_t step_early;
+  asm volatile("ld.acquire.gpu.global.s64 %0, [%1];" : "=l"(step_early) : "l"(a.rows.step) : "memory");
+  const int64_t pos_early = a.rows.pos0[row] + step_early;
+  load_state(pos_early > 0);
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  int64_t step_now;
+  asm volatile("ld.acquire.gpu.global.s64 %0, [%1];" : "=l"(step_now) : "l"(a.rows.step) : "memory");
+  const int64_t m = row, pos = a.rows.pos0[row] + step_now;
+  if (pos != pos_early) load_state(pos > 0);
   // short convolutions of this head's channels
   const float* p = a.proj + m * a.ldp;
   float* tail = a.tail + (int64_t)slot * a.taps * a.C;
