@@ -98,6 +98,13 @@ k_gemm_tc(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUt
     *cta_abort = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    // weights first: they depend neither on the preceding kernel nor on TMEM or the other warps
+    for (int i = 0; i < min(nkb, STAGES); ++i) {
+      const uint32_t full = bars + 8 * i;
+      mbar_expect_tx(full, W_BYTES);
+      tma_load_2d(base + i * STAGE_BYTES, &map_w, (kb0 + i) * BK, n0, full);
+      if (ACC2) tma_load_2d(base + i * STAGE_BYTES + A_BYTES, &map_w, (kb0 + i) * BK, n0 + p.row2_off, full);
+    }
   }
   if (warp == 1) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32((const void*)tmem_slot)),
@@ -113,14 +120,7 @@ k_gemm_tc(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUt
   bool acc_ok = false;  // epilogue warps: the accumulator is complete
   if (warp == 0) {
     if (lane == 0 && nkb > 0) {
-      // weights first: they do not depend on the preceding kernel
       const int pre = min(nkb, STAGES);
-      for (int i = 0; i < pre; ++i) {
-        const uint32_t full = bars + 8 * i;
-        mbar_expect_tx(full, W_BYTES);
-        tma_load_2d(base + i * STAGE_BYTES, &map_w, (kb0 + i) * BK, n0, full);
-        if (ACC2) tma_load_2d(base + i * STAGE_BYTES + A_BYTES, &map_w, (kb0 + i) * BK, n0 + p.row2_off, full);
-      }
       asm volatile("griddepcontrol.wait;" ::: "memory");
       for (int i = 0; i < nkb; ++i) {
         const int s = i % STAGES;
@@ -141,22 +141,27 @@ k_gemm_tc(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUt
   } else if (warp == 1) {
     if (lane == 0 && nkb > 0) {
       constexpr uint32_t idesc = umma_idesc(TN);
+      const uint64_t da0 = umma_desc(base), db0 = umma_desc(base + W_BYTES);  // of slot 0
+      constexpr uint64_t DK = UMMA_K * 2 >> 4, DUP = A_BYTES >> 4;
+      uint64_t off = 0;
+      int sl = 0;
+      uint32_t par = 0;
       bool ok = true;
-      for (int i = 0; i < nkb && ok; ++i) {
-        const int s = i % STAGES;
-        const uint32_t ph = (uint32_t)(i / STAGES) & 1u;
-        ok = mbar_wait(bars + 8 * s, ph, cta_abort, p.err);
+      for (int i = 0; i < nkb; ++i) {
+        ok = mbar_wait(bars + 8 * sl, par, cta_abort, p.err);
         if (!ok) break;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        const uint32_t a = base + s * STAGE_BYTES;
+        const uint64_t da = da0 + off, db = db0 + off;
+        umma_bf16(tmem_acc, da, db, idesc, i > 0 ? 1u : 0u);
+        if (ACC2) umma_bf16(tmem_acc + TN, da + DUP, db, idesc, i > 0 ? 1u : 0u);
 #pragma unroll
-        for (int kk = 0; kk < BK / UMMA_K; ++kk) {
-          const uint64_t da = umma_desc(a + kk * UMMA_K * 2);
-          const uint64_t db = umma_desc(a + W_BYTES + kk * UMMA_K * 2);
-          umma_bf16(tmem_acc, da, db, idesc, (i > 0 || kk > 0) ? 1u : 0u);
-          if (ACC2) umma_bf16(tmem_acc + TN, umma_desc(a + A_BYTES + kk * UMMA_K * 2), db, idesc, (i > 0 || kk > 0) ? 1u : 0u);
+        for (int kk = 1; kk < BK / UMMA_K; ++kk) {
+          umma_bf16_acc(tmem_acc, da + kk * DK, db + kk * DK, idesc);
+          if (ACC2) umma_bf16_acc(tmem_acc + TN, da + DUP + kk * DK, db + kk * DK, idesc);
         }
-        umma_commit(bars + 8 * (STAGES + s));  // slot reusable once these MMAs have read it
+        umma_commit(bars + 8 * (STAGES + sl));  // slot reusable once these MMAs have read it
+        off += STAGE_BYTES >> 4;
+        if (++sl == STAGES) { sl = 0; par ^= 1u; off = 0; }
       }
       if (ok) umma_commit(bar_accum);
     }
@@ -263,12 +268,12 @@ k_gemm_tc(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUt
     cluster_sync_all();
     if (warp >= 2 && !*cta_abort) {
       const int S = p.splits;
-      const int rows_per = BM / S;
+      const int lg = 31 - __clz(BM / S);  // (S is a power of two)
       const int cols = min(TN, p.M - m0);
       const uint32_t stage_u = base;
-      for (int e = tid - 64; e < rows_per * cols; e += 128) {
-        const int col = e / rows_per;
-        const int row = split * rows_per + (e - col * rows_per);
+      for (int e = tid - 64; e < cols << lg; e += 128) {
+        const int col = e >> lg;
+        const int row = (split << lg) + (e & ((1 << lg) - 1));
         const float acc = sum_cluster_f32(stage_u + (uint32_t)(col * BM + row) * 4u, S);
         const int n = n0 + row;
         if (n < p.N) store_out(p, m0 + col, n, acc);
@@ -301,6 +306,34 @@ __global__ void k_splitk_reduce(const float* partial, int splits, int64_t M, int
     if (out_mode == 0) ((float*)out)[o] = acc;
     else if (out_mode != 2) ((__nv_bfloat16*)out)[o] = __float2bfloat16_rn(bf16_out(out_mode, acc, residual, n));
     else ((float*)out)[o] = acc + residual[o];
+  }
+}
+
+// The same four columns at a time, a block per 1024 columns of a row: no 64-bit division per element, and up to
+// eight slices in flight at once.  (N and the row stride multiples of 4, 16-byte aligned bases.)
+__global__ void __launch_bounds__(256) k_splitk_reduce_vec(const float* partial, int splits, int64_t M, int64_t N, void* out, int64_t ldo,
+                                                           const float* residual, int out_mode) {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  const int64_t m = blockIdx.y, n = 4 * ((int64_t)blockIdx.x * 256 + threadIdx.x), total = M * N;
+  if (n >= N) return;
+  const float* src = partial + m * N + n;
+  float4 acc = make_float4(0.f, 0.f, 0.f, 0.f), res = acc;
+  if (out_mode == 2) res = *(const float4*)(residual + m * ldo + n);
+#pragma unroll 8
+  for (int s = 0; s < splits; ++s) {
+    const float4 v = __ldcg((const float4*)(src + (int64_t)s * total));
+    acc.x += v.x; acc.y += v.y; acc.z += v.z; acc.w += v.w;
+  }
+  const int64_t o = m * ldo + n;
+  if (out_mode == 0) {
+    *(float4*)((float*)out + o) = acc;
+  } else if (out_mode == 2) {
+    *(float4*)((float*)out + o) = make_float4(acc.x + res.x, acc.y + res.y, acc.z + res.z, acc.w + res.w);
+  } else {
+    const __nv_bfloat162 a = __floats2bfloat162_rn(bf16_out(out_mode, acc.x, residual, n), bf16_out(out_mode, acc.y, residual, n + 1)),
+                         b = __floats2bfloat162_rn(bf16_out(out_mode, acc.z, residual, n + 2), bf16_out(out_mode, acc.w, residual, n + 3));
+    *(uint2*)((__nv_bfloat16*)out + o) = make_uint2(*(const uint32_t*)&a, *(const uint32_t*)&b);
   }
 }
 
@@ -428,7 +461,12 @@ int gemm_tc(cg_ctx* c, const __nv_bfloat16* x, int64_t ldx, const __nv_bfloat16*
     case 128: CG_TRY((launch<128, 6, 1>(c, mw, mx, a, grid))); break;
     default: CG_TRY((launch<256, 4, 1>(c, mw, mx, a, grid))); break;
   }
-  if (splits > 1 && !cluster) {
+  const bool aligned = ((uintptr_t)workspace % 16) == 0 && ((uintptr_t)out % 16) == 0 && (out_mode != 2 || ((uintptr_t)residual % 16) == 0);
+  if (splits > 1 && !cluster && aligned && N % 4 == 0 && ldo % 4 == 0 && M <= 65535) {
+    CG_CUDA(c, launch_kernel(c, k_splitk_reduce_vec, dim3((unsigned)((N + 1023) / 1024), (unsigned)M), dim3(256), 0, 1, (const float*)workspace, splits,
+                             M, N, out, ldo, residual, out_mode));
+    CG_LAUNCHED(c);
+  } else if (splits > 1 && !cluster) {
     CG_CUDA(c, launch_kernel(c, k_splitk_reduce, dim3(grid_for(M * N, 256)), dim3(256), 0, 1, (const float*)workspace, splits,
                              M, N, out, ldo, residual, out_mode));
     CG_LAUNCHED(c);
