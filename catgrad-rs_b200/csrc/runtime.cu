@@ -96,18 +96,17 @@ static bool mostly_new_pages(const void* dst, size_t bytes) {
 
 // `bytes` from the device to host memory, complete on return.  The driver copies to pageable memory on the
 // calling thread, 3 to 4 GB/s where the destination's pages are new.  Reads of a megabyte and more (a batch's
-// logits) into new pages, and of 12 MB and more into any, come through pinned segments instead, which four
-// threads empty into the destination while the next ones arrive: segment k waits in slot k mod 16, and the
-// thread that empties a slot asks for the segment 16 further on.  Into pages in use / new pages, before -> now:
-// 16.8 MB 1335 -> 930 / 4902 -> 2218 us; 7.8 MB new 2513 -> 1138 us.  Into 7.8 MB in use the threads can cost
-// more than they save (a forward of 2.2 ms that reads its logits: +0.3 ms), so those stay with the driver.
+// logits) into new pages come through pinned segments instead, which four threads empty into the destination
+// while the next ones arrive: segment k waits in slot k mod 16, and the thread that empties a slot asks for the
+// segment 16 further on.  Before -> now: 7.8 MB 2513 -> 1177 us, 16.8 MB 4902 -> 2137 us.  Into pages in use the
+// driver is as fast as the threads (a forward of 2.2 ms that reads 7.8 MB of logits: 0.3 ms longer with them).
 cudaError_t Core::copy_out(void* dst, const void* src, size_t bytes) {
   const int n = (int)((bytes + OUT_SEG - 1) / OUT_SEG);
   cudaPointerAttributes at;
   const bool pageable = cudaPointerGetAttributes(&at, dst) == cudaSuccess && at.type == cudaMemoryTypeUnregistered;
   cudaGetLastError();
   std::unique_lock<std::mutex> lock(out_mu, std::defer_lock);
-  if (n >= 2 && n <= (1 << 24) && pageable && (n >= 24 || mostly_new_pages(dst, bytes))) lock.lock();
+  if (n >= 2 && n <= (1 << 24) && pageable && mostly_new_pages(dst, bytes)) lock.lock();
   if (lock.owns_lock() && !out_stage && !out_failed) {
     int current = device;
     cudaGetDevice(&current);
