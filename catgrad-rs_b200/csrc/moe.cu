@@ -315,6 +315,7 @@ __global__ void k_moe_topk(const float* logits, int64_t M, int E, int k, int nor
 // never crossing a group) and gives every pair its row (or -1 when another rank owns its
 // expert).  Thread e owns expert e: two block-wide prefix sums give its first row and its
 // first tile.
+constexpr size_t PLAN_SMEM = 2 * 32 * sizeof(int);  // wsum_rows, wsum_tiles
 __device__ __forceinline__ void plan_block(const uint32_t* ids, int P, int e_lo, int El, int tn, int* sh_i, int32_t* pos, int32_t* tile_expert,
                                            int32_t* tile_row0, int32_t* tile_rows, int32_t* n_tiles) {
   int* cnt = sh_i;          // [El]
@@ -875,11 +876,12 @@ static int launch_plan(cg_ctx* c, const MoeArgs& a, int tn) {
 }
 
 // Choice and plan in one launch where one block has a warp for every token and a thread for every expert
-// (decode steps: at most 32 tokens; 1024 threads) and its rows fit the shared memory that needs no opt-in.
+// (decode steps: at most 32 tokens; 1024 threads) and its rows fit the shared memory that needs no opt-in: 48 KB
+// less what plan_block has of its own.
 static size_t ride_smem(const MoeArgs& a) {
   return (size_t)2 * a.El * 4 + (size_t)a.M * a.k * 4 + (size_t)a.M * a.E * (a.correction ? 8 : 4);
 }
-static bool plan_rides(const MoeArgs& a) { return a.M <= 32 && ride_smem(a) <= 48 * 1024; }
+static bool plan_rides(const MoeArgs& a) { return a.M <= 32 && ride_smem(a) + PLAN_SMEM <= 48 * 1024; }
 
 static int launch_choice(cg_ctx* c, const MoeArgs& a, int tn) {
   if (!plan_rides(a)) {

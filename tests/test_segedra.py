@@ -216,6 +216,19 @@ def test_loops(backends, loop, prec):
 
 
 @gpu
+@pytest.mark.parametrize("experts", [184, 185, 186])
+def test_corrected_choice_and_plan_in_one_block(backends, experts):
+    """32 tokens with as many experts as the choice and the plan in one block have shared memory for (two values per token
+    and expert where the choice is corrected), and the first counts that take two launches."""
+    cfg = model([moe(att(window=0), experts, 2, 8)])
+    W, seq = weights(cfg, 8), toks(32, 8)
+    dec = decoder(backends["f32"], cfg, W)
+    want, ok = expected(cfg, W, seq)
+    assert agrees(everything(dec, seq), want, ok, "f32")
+    dec.close()
+
+
+@gpu
 def test_wide_rows_take_the_persistent_kernels(backends):
     """Sizes at which the projections, the squared relu and the experts run on the persistent GEMMs."""
     for seed, n, ff in ((6, 600, 9216), (7, 1100, 8192)):
