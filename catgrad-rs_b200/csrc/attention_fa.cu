@@ -463,17 +463,20 @@ k_attn_fa(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUt
 //     the same key tiles: while one group exponentiates, the other's products run;
 //   * P is written back over its scores in TMEM (bf16, two to a column) and is the A operand of P V from there:
 //     no shared memory, no proxy fence, and room for two query tiles beside the key and value ring;
-//   * O stays in TMEM and is accumulated there.  It is rescaled only where a row's maximum has grown by more than
-//     2^8 since the last time: until then the exponentials are taken against the old maximum, which at
-//     most makes them 2^8 times larger (bf16 and f32 keep their relative precision).
+//   * O stays in TMEM and is accumulated there.  A warp rescales it where a row's maximum has grown.  Every time: the
+//     largest probability of a row is then exactly 1 and loses nothing in bf16.  Exponentials against a
+//     maximum that may lag by 2^8 save most of the rescaling (below: 636 us and 146), but turn the probabilities that
+//     decide into arbitrary numbers to be rounded (error against 64 bits 4 % larger where scores spread by a few units, 17 %
+//     where by many).
+//   * the denominator sums the probabilities as bf16 holds them, so that of their rounding only what differs
+//     between the keys of a row is left.
+// The two query tiles that take turns and P in its scores' place are FlashAttention-4's, as published.
 // Head size 256 (with or without soft-cap) has one query tile (its outputs fill half of the TMEM) and two score
 // buffers instead, so that the next scores are computed while this tile's softmax runs.
 // Columns: scores of slot s at s BK (two slots), then O of group w.
 // One layer, before (k_attn_fa; head size 256 k_attn_prefill on mma.sync) -> now: 1 x 8191 tokens, 32 heads of 128: 1196 ->
 // 636 us (864 TFLOP/s); 32 x 509: 321 -> 194; 8 x 512, 32 heads of 64: 56 -> 48; 13 x 389: 79 -> 73; 4 x 2048, 8 heads of
 // 256, soft-cap: 780 -> 145 us (473 TFLOP/s).
-constexpr float FQ_SLACK = 8.f;  // log2 of how far a maximum may grow before the outputs are rescaled
-
 __device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t* v) {
   asm volatile(
       "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};" ::"r"(taddr),
@@ -726,7 +729,7 @@ k_attn_fq(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUt
       if (j == 0) {
         m = mx;
       } else {
-        const bool grown = mx > m + FQ_SLACK;
+        const bool grown = mx > m;
         if (__any_sync(0xffffffffu, grown)) {
           const float m_new = grown ? mx : m;
           const float corr = grown ? fast_exp2(m - m_new) : 1.f;  // 0 while m is -inf
@@ -736,13 +739,13 @@ k_attn_fq(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUt
           if (!__all_sync(0xffffffffu, ok)) { ok = false; break; }
           asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 #pragma unroll 1
-          for (int c = 0; c < D; c += 16) {
-            uint32_t t[16];
-            tmem_ld16(o_addr + c, t);
+          for (int c = 0; c < D; c += 32) {
+            tmem_ld32(o_addr + c, vb);
             asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
-            for (int i = 0; i < 16; ++i) t[i] = __float_as_uint(__uint_as_float(t[i]) * corr);
-            tmem_st16(o_addr + c, t);
+            for (int i = 0; i < 32; ++i) vb[i] = __float_as_uint(__uint_as_float(vb[i]) * corr);
+            tmem_st16(o_addr + c, vb);
+            tmem_st16(o_addr + c + 16, vb + 16);
           }
           l *= corr;
           m = m_new;
@@ -763,10 +766,11 @@ k_attn_fq(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUt
             if (CAP) e[t] = fast_exp2(fmaf(2.f * p.cap_log2e, fast_rcp(1.f + fast_exp2(x * p.cap_unit)), -p.cap_log2e - mc));
             else e[t] = fast_exp2(fmaf(x, p.scale_log2e, -mc));
             if (masked.value) e[t] = vis & (1u << (i + t)) ? e[t] : 0.f;
-            ls[t] += e[t];
           }
           const __nv_bfloat162 pr = __floats2bfloat162_rn(e[0], e[1]);
           pk[i / 2] = *(const uint32_t*)&pr;
+          ls[0] += __uint_as_float(pk[i / 2] << 16);
+          ls[1] += __uint_as_float(pk[i / 2] & 0xffff0000u);
         }
         tmem_st16(s_addr + (uint32_t)c * 16u, pk);
       };
