@@ -111,8 +111,6 @@ k_attn_fa(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUt
   constexpr uint32_t O_COL = 2 * S_COLS;            // O_t after the two score buffers
   constexpr uint32_t NCOLS = 2 * S_COLS + D <= 256 ? 256 : 512;  // two CTAs per SM share 512 columns
 
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   const uint32_t raw = smem_u32(smem_raw);
   const uint32_t base = (raw + 1023u) & ~1023u;
@@ -173,6 +171,11 @@ k_attn_fa(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUt
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   }
+  // q and the cache are written by the preceding kernels
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  // TMEM between the dependency and the trigger: all kernels before have given their columns back, and none
+  // behind can take columns that this one still waits for (a CTA of theirs that held some would wait for this kernel to
+  // end, and this kernel for the columns).
   if (warp == 1) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32((const void*)tmem_slot)),
                  "r"(NCOLS)
@@ -183,9 +186,7 @@ k_attn_fa(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUt
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem_base = *tmem_slot;
-
-  // q and the cache are written by the preceding kernels
-  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 
   if (warp == 0) {
     if (lane == 0) {
@@ -509,7 +510,6 @@ k_attn_fq(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUt
   constexpr uint32_t O_COL = 2 * BK, NCOLS = 512;
   static_assert(O_COL + NQ * D <= NCOLS, "TMEM");
 
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   const uint32_t raw = smem_u32(smem_raw);
   const uint32_t base = (raw + 1023u) & ~1023u;
@@ -563,6 +563,9 @@ k_attn_fq(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUt
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   }
+  // q and the cache are written by the preceding kernels
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  // (TMEM between the dependency and the trigger, as in k_attn_fa)
   if (warp == 1) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32((const void*)tmem_slot)),
                  "r"(NCOLS)
@@ -573,9 +576,7 @@ k_attn_fq(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUt
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem_base = *tmem_slot;
-
-  // q and the cache are written by the preceding kernels
-  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 
   if (warp == 0) {
     if (lane == 0) {
