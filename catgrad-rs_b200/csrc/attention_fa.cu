@@ -494,10 +494,13 @@ __device__ __forceinline__ void umma_bf16_ts(uint32_t tmem_d, uint32_t tmem_a, u
       ::"r"(tmem_d), "r"(tmem_a), "l"(db), "r"(idesc), "r"(accumulate)
       : "memory");
 }
-__device__ __forceinline__ float fast_rcp(float x) {
+// 1 / x for x >= 1 (as good as 0 above 1e37): the approximation and one step of Newton's iteration, so that a soft-capped
+// score keeps its 24 bits.  (2048 tokens, 8 heads of 256: 183 us without the step, 189 with it, 455 with a division.)
+__device__ __forceinline__ float rcp_newton(float x) {
   float y;
+  x = x > 1e37f ? 1e37f : x;  // (a NaN stays one)
   asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-  return y;
+  return fmaf(y, fmaf(-x, y, 1.f), y);
 }
 
 template <int D, int BK, int NQ, bool CAP>
@@ -725,7 +728,7 @@ k_attn_fq(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUt
       }
       const float raw_max = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3]));
       float mx;  // (the soft-cap is monotone)
-      if (CAP) mx = raw_max == -INFINITY ? -INFINITY : fmaf(2.f * p.cap_log2e, fast_rcp(1.f + fast_exp2(raw_max * p.cap_unit)), -p.cap_log2e);
+      if (CAP) mx = raw_max == -INFINITY ? -INFINITY : fmaf(2.f * p.cap_log2e, rcp_newton(1.f + fast_exp2(raw_max * p.cap_unit)), -p.cap_log2e);
       else mx = raw_max * p.scale_log2e;
       if (j == 0) {
         m = mx;
@@ -764,7 +767,7 @@ k_attn_fq(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUt
 #pragma unroll
           for (int t = 0; t < 2; ++t) {
             const float x = __uint_as_float(cur[i + t]);
-            if (CAP) e[t] = fast_exp2(fmaf(2.f * p.cap_log2e, fast_rcp(1.f + fast_exp2(x * p.cap_unit)), -p.cap_log2e - mc));
+            if (CAP) e[t] = fast_exp2(fmaf(2.f * p.cap_log2e, rcp_newton(1.f + fast_exp2(x * p.cap_unit)), -p.cap_log2e - mc));
             else e[t] = fast_exp2(fmaf(x, p.scale_log2e, -mc));
             if (masked.value) e[t] = vis & (1u << (i + t)) ? e[t] : 0.f;
           }

@@ -350,3 +350,22 @@ def test_fused_attention_rounds_against_the_running_maximum(cuda, d, window, cap
     rounded = synth.bf16_round((pb @ v / pb.sum(-1, keepdims=True)).astype(np.float32))
     error = lambda x: np.linalg.norm(x - want) / np.linalg.norm(want)
     assert error(got) <= 1.02 * error(rounded)
+
+
+@pytest.mark.parametrize("d", [64, 128, 256])
+def test_fused_attention_soft_cap_extremes(cuda, d):
+    """Scores far beyond the soft-cap on both sides (each +-cap to 24 bits, so keys of one sign weigh the same and those of the
+    other nothing), and a NaN: rows that see it are NaN, rows before it are what they were."""
+    s, cap = 200, 50.0
+    sign = np.where(np.arange(s) % 3 == 0, 1.0, -1.0).astype(np.float32)
+    q = np.full((1, 1, s, d), 100.0, np.float32)
+    k = np.broadcast_to(sign[:, None] * 3e30, (1, 1, s, d)).astype(np.float32)
+    v = synth.bf16_round(rnd((1, 1, s, d)))
+    run = lambda q, k, v: cuda.to_numpy(cuda.fused_attention(cuda.from_numpy(q), cuda.from_numpy(k), cuda.from_numpy(v), 0, cap))[0, 0]
+    got = run(q, k, v)
+    up = np.cumsum(sign > 0)
+    want = np.cumsum(np.where(sign[:, None] > 0, v[0, 0], 0).astype(np.float64), 0) / up[:, None]
+    np.testing.assert_allclose(got, want, rtol=2.0 ** -8, atol=2.0 ** -8 * 1e-3)
+    k[0, 0, 150, 0] = np.nan
+    bad = run(q, k, v)
+    assert np.isnan(bad[150:]).all() and (bad[:150] == got[:150]).all()
