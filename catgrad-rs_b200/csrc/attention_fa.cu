@@ -1,6 +1,6 @@
 // attention_fa.cu — causal prefill attention on the Blackwell tensor cores (tcgen05 + TMEM): k_attn_fq for head
 // sizes 64, 128 and 256 with or without soft-cap, k_attn_fa for distance biases and gates per value (head
-// sizes 64 and 128) and as the 64-key variant.
+// sizes 64 and 128) and where the option asks for it.
 //
 // Same mathematics as attention.cu (catgrad-llm/src/models/llama.rs:97-108 after repeat_kv,
 // catgrad-llm/src/helpers.rs:147-161, as an online-softmax pass over key tiles); what changes
@@ -456,28 +456,33 @@ k_attn_fa(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUt
   }
 }
 
-// ---- two query tiles per CTA, probabilities and outputs in TMEM -----------------------------------
+// ---- probabilities and outputs in TMEM ------------------------------------------------------------
 //
-// k_attn_fa above is one softmax warpgroup deep: its chain (scores -> maximum -> exponentials -> P V -> fold into
-// registers) leaves the tensor cores idle four fifths of the time.  Here
-//   * NQ = 2 groups of four softmax warps, each with its own 128 queries, take turns on the tensor cores over
-//     the same key tiles: while one group exponentiates, the other's products run;
+// k_attn_fa above folds every tile's P V into registers behind a chain (scores -> maximum -> exponentials -> P through
+// shared memory -> P V -> fold) that leaves the tensor cores idle four fifths of the time.  Here
 //   * P is written back over its scores in TMEM (bf16, two to a column) and is the A operand of P V from there:
-//     no shared memory, no proxy fence, and room for two query tiles beside the key and value ring;
+//     no shared memory, no proxy fence;
 //   * O stays in TMEM and is accumulated there.  A warp rescales it where a row's maximum has grown.  Every time: the
 //     largest probability of a row is then exactly 1 and loses nothing in bf16.  Exponentials against a
-//     maximum that may lag by 2^8 save most of the rescaling (below: 636 us and 146), but turn the probabilities that
-//     decide into arbitrary numbers to be rounded (error against 64 bits 4 % larger where scores spread by a few units, 17 %
-//     where by many).
+//     maximum that may lag by 2^8 save most of the rescaling (4 x 2048, 8 heads of 256: 146 us instead of 189), but turn
+//     the probabilities that decide into arbitrary numbers to be rounded (error against 64 bits 4 % larger where scores
+//     spread by a few units, 17 % where by many);
 //   * the denominator sums the probabilities as bf16 holds them, so that of their rounding only what differs
-//     between the keys of a row is left.
-// The two query tiles that take turns and P in its scores' place are FlashAttention-4's, as published.
-// Head size 256 (with or without soft-cap) has one query tile (its outputs fill half of the TMEM) and two score
-// buffers instead, so that the next scores are computed while this tile's softmax runs.
-// Columns: scores of slot s at s BK (two slots), then O of group w.
-// One layer, before (k_attn_fa; head size 256 k_attn_prefill on mma.sync) -> now: 1 x 8191 tokens, 32 heads of 128: 1196 ->
-// 636 us (864 TFLOP/s); 32 x 509: 321 -> 194; 8 x 512, 32 heads of 64: 56 -> 48; 13 x 389: 79 -> 73; 4 x 2048, 8 heads of
-// 256, soft-cap: 780 -> 145 us (473 TFLOP/s).
+//     between the keys of a row is left;
+//   * there are two score buffers, so that the next scores are computed while this tile's softmax runs.
+// P in its scores' place is FlashAttention-4's, as published.
+// A CTA has 128 queries and 64-key tiles.  Up to head size 128 it takes 256 columns and half of an SM, so that one CTA's
+// products run under the other's exponentials.  (Two query tiles and 128-key tiles in one CTA of a whole SM
+// were slower nearly everywhere: 1 x 8191 tokens, 32 heads of 128: 738 us against 710; 8 x 512, 32 heads of 64: 51 against 44; and
+// where there are fewer tiles than SMs, or the second tile is empty, slower than k_attn_fa.)  At head size 256 the
+// outputs fill half of the TMEM, and there is one CTA per SM.
+// Columns: scores of buffer s at 64 s, then O.
+// One layer, before (k_attn_fa; head size 256, soft-caps and rows of less than 64 tokens k_attn_prefill on mma.sync) -> now:
+// 1 x 8191 tokens, 32 heads of 128: 1188 -> 710 us (774 TFLOP/s); 32 x 509: 319 -> 183; 8 x 512, 32 heads of 64: 56 -> 44;
+// 13 x 389: 78 -> 63; 4 x 2048, 8 heads of 256, soft-cap: 768 -> 189 (364 TFLOP/s).  Over 456 shapes (17 to 2000 tokens, 8 to
+// 416 rows x heads, windows of 64 to 512, with and without soft-cap) it takes 0.14 to 0.95 of the time, 0.57 in the mean.
+constexpr int FQ_BK = 64;  // keys per tile
+
 __device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t* v) {
   asm volatile(
       "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};" ::"r"(taddr),
@@ -503,25 +508,26 @@ __device__ __forceinline__ float rcp_newton(float x) {
   return fmaf(y, fmaf(-x, y, 1.f), y);
 }
 
-template <int D, int BK, int NQ, bool CAP>
-__global__ void __launch_bounds__(128 + NQ * 128, 1)
+template <int D, bool CAP>
+__global__ void __launch_bounds__(256, D <= 128 ? 2 : 1)
 k_attn_fq(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
           const __grid_constant__ CUtensorMap map_v, FaArgs p) {
   constexpr int SUB = D / 64;
+  constexpr int BK = FQ_BK;
   constexpr uint32_t BOX = 128 * 128, KBOX = BK * 128;
   constexpr uint32_t Q_BYTES = SUB * BOX, KV_BYTES = SUB * KBOX;
-  constexpr uint32_t O_COL = 2 * BK, NCOLS = 512;
-  static_assert(O_COL + NQ * D <= NCOLS, "TMEM");
+  constexpr uint32_t O_COL = 2 * BK, NCOLS = D <= 128 ? 256 : 512;
+  static_assert(O_COL + D <= NCOLS, "TMEM");
 
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   const uint32_t raw = smem_u32(smem_raw);
   const uint32_t base = (raw + 1023u) & ~1023u;
   uint8_t* gen = smem_raw + (base - raw);
-  const uint32_t sq = base, sk = sq + NQ * Q_BYTES, sv = sk + 2 * KV_BYTES, bars = sv + 2 * KV_BYTES;
+  const uint32_t sq = base, sk = sq + Q_BYTES, sv = sk + 2 * KV_BYTES, bars = sv + 2 * KV_BYTES;
   const uint32_t b_q_full = bars, b_k_full = bars + 8, b_v_full = bars + 24, b_k_empty = bars + 40, b_v_empty = bars + 56,
-                 b_s_full = bars + 72, b_p_full = bars + 88, b_o_full = bars + 104, b_v_last = bars + 120, b_v_ready = bars + 128;
-  volatile uint32_t* tmem_slot = (volatile uint32_t*)(gen + (bars - base) + 136);
-  volatile int* cta_abort = (volatile int*)(gen + (bars - base) + 140);
+                 b_s_full = bars + 72, b_p_full = bars + 88, b_o_full = bars + 104, b_v_last = bars + 112, b_v_ready = bars + 120;
+  volatile uint32_t* tmem_slot = (volatile uint32_t*)(gen + (bars - base) + 128);
+  volatile int* cta_abort = (volatile int*)(gen + (bars - base) + 132);
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int qt = (int)gridDim.x - 1 - (int)blockIdx.x, h = blockIdx.y;  // longest tiles first
@@ -534,19 +540,17 @@ k_attn_fq(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUt
     b = p.rows.slot[row];
   }
   const int kvh = h / (p.nh / p.nkv);
-  const int64_t q0 = (int64_t)qt * (128 * NQ);
+  const int64_t q0 = (int64_t)qt * 128;
   if (q0 >= len) return;  // uniform over the CTA, before anything is allocated
-  // key tiles: nk of kept first tokens, then from tile j0 on; group w needs the first nt[w] of them
+  const int64_t last_q = start_pos + std::min<int64_t>(len, q0 + 128) - 1;  // position of the last query
+  // key tiles: nk of kept first tokens, then from tile j0 on
   const int j0 = p.window > 0 ? (int)(std::max<int64_t>(0, start_pos + q0 - p.window + 1) / BK) : 0;
   const int nk = (int)std::min<int64_t>(j0, (p.keep + BK - 1) / BK);
-  auto tiles_to = [&](int64_t q_end) { return nk + (int)((start_pos + std::min<int64_t>(len, q_end) - 1) / BK) + 1 - j0; };
-  const int nt0 = tiles_to(q0 + 128);
-  const int nt1 = NQ == 2 && q0 + 128 < len ? tiles_to(q0 + 256) : 0;
-  const int nt = nt1 > nt0 ? nt1 : nt0;
+  const int nt = nk + (int)(last_q / BK) + 1 - j0;
   // keys of the last tile that some query of this CTA sees.  What lies behind them (rows of the cache that
   // nothing or another sequence wrote) is cleared in shared memory: a probability of 0 times an infinity
   // would not be 0
-  const int seen = (int)(start_pos + std::min<int64_t>(len, q0 + 128 * NQ) - (int64_t)(j0 + nt - 1 - nk) * BK);
+  const int seen = (int)(last_q % BK) + 1;
   auto tile_of = [&](int j) { return j < nk ? j : j0 + j - nk; };
 
   if (tid == 0) {
@@ -558,8 +562,8 @@ k_attn_fq(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUt
       mbar_init(b_v_empty + 8 * i, 1);
       mbar_init(b_s_full + 8 * i, 1);
       mbar_init(b_p_full + 8 * i, 4);  // (a warp each: 128 arrivals on one address take turns)
-      mbar_init(b_o_full + 8 * i, 1);
     }
+    mbar_init(b_o_full, 1);
     mbar_init(b_v_last, 1);
     mbar_init(b_v_ready, 1);
     *cta_abort = 0;
@@ -583,10 +587,8 @@ k_attn_fq(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUt
 
   if (warp == 0) {
     if (lane == 0) {
-      const int groups = nt1 > 0 ? 2 : 1;
-      mbar_expect_tx(b_q_full, groups * Q_BYTES);
-      for (int w = 0; w < groups; ++w)
-        for (int s = 0; s < SUB; ++s) tma_load_2d(sq + w * Q_BYTES + s * BOX, &map_q, h * D + s * 64, (int)(tok0 + q0) + w * 128, b_q_full);
+      mbar_expect_tx(b_q_full, Q_BYTES);
+      for (int s = 0; s < SUB; ++s) tma_load_2d(sq + s * BOX, &map_q, h * D + s * 64, (int)(tok0 + q0), b_q_full);
       const int64_t kvrow0 = p.token_major ? b * p.Tmax : (b * p.nkv + kvh) * p.Tmax;
       const int kx = p.token_major ? kvh * D : 0;
       for (int j = 0; j < nt; ++j) {
@@ -604,56 +606,42 @@ k_attn_fq(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUt
     if (lane == 0) {
       constexpr uint32_t idesc_s = umma_idesc(BK), idesc_o = umma_idesc(D) | (1u << 16);  // (V: MN-major)
       const uint64_t dq = umma_desc(sq), dk = umma_desc(sk), dv = umma_desc_mn(sv, KBOX);
-      // the last group that reads tile j frees its buffer (products complete in the order they are issued)
-      auto last = [&](int j) { return j < nt1 ? 1 : 0; };
-      auto slot_of = [&](int w, int j) { return NQ == 2 ? w : j & 1; };
-      auto slot_phase = [&](int j) { return (uint32_t)(NQ == 2 ? j : j >> 1) & 1u; };
-      auto qk = [&](int w, int j) {
-        const uint32_t buf = (uint32_t)j & 1u;
-        if (!mbar_wait(b_k_full + 8 * buf, ((uint32_t)j >> 1) & 1u, cta_abort, p.err)) return false;
+      auto qk = [&](int j) {
+        const uint32_t buf = (uint32_t)j & 1u, ph = ((uint32_t)j >> 1) & 1u;
+        if (!mbar_wait(b_k_full + 8 * buf, ph, cta_abort, p.err)) return false;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        const int slot = slot_of(w, j);
 #pragma unroll
         for (int kk = 0; kk < D / UMMA_K; ++kk) {
           const uint64_t oq = ((uint32_t)(kk / 4) * BOX + (uint32_t)(kk % 4) * 32u) >> 4, ok = ((uint32_t)(kk / 4) * KBOX + (uint32_t)(kk % 4) * 32u) >> 4;
-          umma_bf16(tmem_base + slot * BK, dq + ((w * Q_BYTES) >> 4) + oq, dk + ((buf * KV_BYTES) >> 4) + ok, idesc_s, kk > 0 ? 1u : 0u);
+          umma_bf16(tmem_base + buf * BK, dq + oq, dk + ((buf * KV_BYTES) >> 4) + ok, idesc_s, kk > 0 ? 1u : 0u);
         }
-        umma_commit(b_s_full + 8 * slot);
-        if (w == last(j)) umma_commit(b_k_empty + 8 * buf);
+        umma_commit(b_s_full + 8 * buf);
+        umma_commit(b_k_empty + 8 * buf);
         return true;
       };
-      auto pv = [&](int w, int j) {
-        const uint32_t buf = (uint32_t)j & 1u;
-        const int slot = slot_of(w, j);
-        if (!mbar_wait(b_v_full + 8 * buf, ((uint32_t)j >> 1) & 1u, cta_abort, p.err)) return false;
+      auto pv = [&](int j) {
+        const uint32_t buf = (uint32_t)j & 1u, ph = ((uint32_t)j >> 1) & 1u;
+        if (!mbar_wait(b_v_full + 8 * buf, ph, cta_abort, p.err)) return false;
         if (j == nt - 1 && seen < BK) {
           // (warp 2 clears what no query sees while the softmax runs)
-          if (w == 0 || nt0 < nt) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(b_v_last) : "memory");
+          asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(b_v_last) : "memory");
           if (!mbar_wait(b_v_ready, 0, cta_abort, p.err)) return false;
         }
-        if (!mbar_wait(b_p_full + 8 * slot, slot_phase(j), cta_abort, p.err)) return false;
+        if (!mbar_wait(b_p_full + 8 * buf, ph, cta_abort, p.err)) return false;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 #pragma unroll
         for (int kk = 0; kk < BK / UMMA_K; ++kk)
-          umma_bf16_ts(tmem_base + O_COL + w * D, tmem_base + slot * BK + kk * (UMMA_K / 2), dv + ((buf * KV_BYTES + (uint32_t)kk * (UMMA_K * 128u)) >> 4),
+          umma_bf16_ts(tmem_base + O_COL, tmem_base + buf * BK + kk * (UMMA_K / 2), dv + ((buf * KV_BYTES + (uint32_t)kk * (UMMA_K * 128u)) >> 4),
                        idesc_o, j > 0 || kk > 0 ? 1u : 0u);
-        umma_commit(b_o_full + 8 * w);
-        if (w == last(j)) umma_commit(b_v_empty + 8 * buf);
+        umma_commit(b_o_full);
+        umma_commit(b_v_empty + 8 * buf);
         return true;
       };
       // Scores overwrite the probabilities that lay in their columns, and products with different accumulators are not
-      // ordered among themselves: the product that reads them is waited for, phase by phase.
-      auto done = [&](int w, int j) { return mbar_wait(b_o_full + 8 * w, (uint32_t)j & 1u, cta_abort, p.err); };
-      bool ok = mbar_wait(b_q_full, 0, cta_abort, p.err) && qk(0, 0);
-      if (NQ == 2) {
-        if (ok && nt1 > 0) ok = qk(1, 0);
-        for (int j = 0; j < nt && ok; ++j) {
-          if (j < nt0) ok = pv(0, j) && (j + 1 >= nt0 || (done(0, j) && qk(0, j + 1)));
-          if (ok && j < nt1) ok = pv(1, j) && (j + 1 >= nt1 || (done(1, j) && qk(1, j + 1)));
-        }
-      } else {
-        for (int j = 0; j < nt && ok; ++j) ok = (j + 1 >= nt || ((j == 0 || done(0, j - 1)) && qk(0, j + 1))) && pv(0, j);
-      }
+      // ordered among themselves: the product that reads them is waited for.
+      auto done = [&](int j) { return mbar_wait(b_o_full, (uint32_t)j & 1u, cta_abort, p.err); };
+      bool ok = mbar_wait(b_q_full, 0, cta_abort, p.err) && qk(0);
+      for (int j = 0; j < nt && ok; ++j) ok = (j + 1 >= nt || ((j == 0 || done(j - 1)) && qk(j + 1))) && pv(j);
     }
   } else if (warp == 2) {
     if (seen < BK) {
@@ -670,18 +658,16 @@ k_attn_fq(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUt
       }
     }
   } else if (warp >= 4) {
-    const int w = (warp - 4) >> 2, q = warp & 3;
+    const int q = warp & 3;
     const int r = q * 32 + lane;  // query row of this thread = TMEM lane
-    const int mine = w ? nt1 : nt0;
     const uint32_t lane_base = tmem_base + ((uint32_t)(q * 32) << 16);
-    const uint32_t o_addr = lane_base + O_COL + w * D;
-    const int64_t qw = q0 + w * 128, qi = qw + r, qpos = start_pos + qi;
-    const int64_t last_q = start_pos + std::min<int64_t>(len, qw + 128) - 1;
+    const uint32_t o_addr = lane_base + O_COL;
+    const int64_t qi = q0 + r, qpos = start_pos + qi;
     float m = -INFINITY, l = 0.f;  // (m in units of log2: what a score is in the exponent of 2)
     bool ok = true;
-    for (int j = 0; j < mine && ok; ++j) {
-      const int slot = NQ == 2 ? w : j & 1;
-      ok = mbar_wait(b_s_full + 8 * slot, (uint32_t)(NQ == 2 ? j : j >> 1) & 1u, cta_abort, p.err);
+    for (int j = 0; j < nt && ok; ++j) {
+      const int buf = j & 1;
+      ok = __all_sync(0xffffffffu, mbar_wait(b_s_full + 8 * buf, (uint32_t)(j >> 1) & 1u, cta_abort, p.err));  // (a warp leaves whole)
       if (!ok) break;
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       const int k0 = tile_of(j) * BK;
@@ -697,14 +683,11 @@ k_attn_fq(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUt
         return bits_below(lim + 1 - c * 32) & (~bits_below(low - c * 32) | bits_below(kept - c * 32));
       };
       // uniform: some key may be masked for some row
-      const bool diag = (int64_t)k0 + BK - 1 > start_pos + qw || (p.window > 0 && k0 <= last_q - p.window && kept < BK);
-      const uint32_t s_addr = lane_base + slot * BK;
-      constexpr int NCH = BK / 32;
+      const bool diag = (int64_t)k0 + BK - 1 > start_pos + q0 || (p.window > 0 && k0 <= last_q - p.window && kept < BK);
+      const uint32_t s_addr = lane_base + buf * BK;
       uint32_t va[32], vb[32];
-      // pass 1: row maximum of the visible scores (four chains; chunk c + 1 is in flight while chunk c is reduced)
+      // pass 1: row maximum of the visible scores (four chains; the second half is in flight while the first is reduced)
       float mx4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
-      // (Both passes are rolled over pairs of chunks: unrolled, with a masked and a plain form each, the loop body left
-      // the instruction cache and prompts of 512 took 21 % longer.)
       auto largest = [&](int c, const uint32_t* cur) {
         if (!diag) {
 #pragma unroll
@@ -717,15 +700,12 @@ k_attn_fq(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUt
       };
       tmem_ld32(s_addr, va);
       asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-#pragma unroll 1
-      for (int c = 0; c < NCH; c += 2) {
-        tmem_ld32(s_addr + (uint32_t)(c + 1) * 32u, vb);
-        largest(c, va);
-        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-        tmem_ld32(s_addr + (uint32_t)(c + 2 < NCH ? c + 2 : 0) * 32u, va);  // (pass 2 starts from the first chunk again)
-        largest(c + 1, vb);
-        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-      }
+      tmem_ld32(s_addr + 32u, vb);
+      largest(0, va);
+      asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+      tmem_ld32(s_addr, va);  // (pass 2 starts from the first half again)
+      largest(1, vb);
+      asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
       const float raw_max = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3]));
       float mx;  // (the soft-cap is monotone)
       if (CAP) mx = raw_max == -INFINITY ? -INFINITY : fmaf(2.f * p.cap_log2e, rcp_newton(1.f + fast_exp2(raw_max * p.cap_unit)), -p.cap_log2e);
@@ -739,7 +719,7 @@ k_attn_fq(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUt
           const float corr = grown ? fast_exp2(m - m_new) : 1.f;  // 0 while m is -inf
           // (the product before the last was complete before this tile's scores could be issued, so the parity is that
           // of the last)
-          ok = mbar_wait(b_o_full + 8 * w, (uint32_t)(j - 1) & 1u, cta_abort, p.err);
+          ok = mbar_wait(b_o_full, (uint32_t)(j - 1) & 1u, cta_abort, p.err);
           if (!__all_sync(0xffffffffu, ok)) { ok = false; break; }
           asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 #pragma unroll 1
@@ -778,66 +758,53 @@ k_attn_fq(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUt
         }
         tmem_st16(s_addr + (uint32_t)c * 16u, pk);
       };
+      tmem_ld32(s_addr + 32u, vb);
       if (diag) {
-#pragma unroll 1
-        for (int c = 0; c < NCH; c += 2) {
-          tmem_ld32(s_addr + (uint32_t)(c + 1) * 32u, vb);
-          chunk(c, va, std::true_type{});
-          asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-          if (c + 2 < NCH) tmem_ld32(s_addr + (uint32_t)(c + 2) * 32u, va);
-          chunk(c + 1, vb, std::true_type{});
-          if (c + 2 < NCH) asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-        }
+        chunk(0, va, std::true_type{});
+        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+        chunk(1, vb, std::true_type{});
       } else {
-#pragma unroll 1
-        for (int c = 0; c < NCH; c += 2) {
-          tmem_ld32(s_addr + (uint32_t)(c + 1) * 32u, vb);
-          chunk(c, va, std::false_type{});
-          asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-          if (c + 2 < NCH) tmem_ld32(s_addr + (uint32_t)(c + 2) * 32u, va);
-          chunk(c + 1, vb, std::false_type{});
-          if (c + 2 < NCH) asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-        }
+        chunk(0, va, std::false_type{});
+        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+        chunk(1, vb, std::false_type{});
       }
-      // (With one group this warp may be a whole product ahead of the tensor core, and a parity tells only neighbouring
-      // phases apart: the last product but one is waited for here, where the last cannot have been issued.)
-      if (NQ == 1 && j > 0 && j + 1 == mine) ok = mbar_wait(b_o_full + 8 * w, (uint32_t)(j - 1) & 1u, cta_abort, p.err);
+      // (This warp may be a whole product ahead of the tensor core, and a parity tells only neighbouring phases apart: the
+      // last product but one is waited for here, where the last cannot have been issued.)
+      if (j > 0 && j + 1 == nt) ok = mbar_wait(b_o_full, (uint32_t)(j - 1) & 1u, cta_abort, p.err);
       asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
       asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
       __syncwarp();
-      if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(b_p_full + 8 * slot) : "memory");
+      if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(b_p_full + 8 * buf) : "memory");
       l += ls[0] + ls[1];
     }
-    if (mine > 0) {
-      ok = ok && mbar_wait(b_o_full + 8 * w, (uint32_t)(mine - 1) & 1u, cta_abort, p.err);
-      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      float inv = l > 0.f ? 1.f / l : 0.f;
-      if (p.sink) {
-        // one more term of the denominator, without a value
-        const float sk2 = p.sink[h] * LOG2E, top = fmaxf(m, sk2);
-        const float f = fast_exp2(m - top);
-        inv = f / (l * f + fast_exp2(sk2 - top));
-      }
-      const bool out = ok && qi < len;
-      inv *= p.out_scale;
-      if (p.gate && out) inv *= 1.f / (1.f + expf(-p.gate[(tok0 + qi) * p.ld_gate + h]));
-      __nv_bfloat16* dst = p.out + (tok0 + qi) * p.ld_out + (int64_t)h * D;
+    ok = ok && mbar_wait(b_o_full, (uint32_t)(nt - 1) & 1u, cta_abort, p.err);
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    float inv = l > 0.f ? 1.f / l : 0.f;
+    if (p.sink) {
+      // one more term of the denominator, without a value
+      const float sk2 = p.sink[h] * LOG2E, top = fmaxf(m, sk2);
+      const float f = fast_exp2(m - top);
+      inv = f / (l * f + fast_exp2(sk2 - top));
+    }
+    const bool out = ok && qi < len;
+    inv *= p.out_scale;
+    if (p.gate && out) inv *= 1.f / (1.f + expf(-p.gate[(tok0 + qi) * p.ld_gate + h]));
+    __nv_bfloat16* dst = p.out + (tok0 + qi) * p.ld_out + (int64_t)h * D;
 #pragma unroll 1
-      for (int c0 = 0; c0 < D; c0 += 32) {
-        uint32_t v[32];
-        tmem_ld32(o_addr + c0, v);
-        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-        if (out) {
+    for (int c0 = 0; c0 < D; c0 += 32) {
+      uint32_t v[32];
+      tmem_ld32(o_addr + c0, v);
+      asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+      if (out) {
 #pragma unroll
-          for (int t = 0; t < 4; ++t) {
-            uint32_t x[4];
+        for (int t = 0; t < 4; ++t) {
+          uint32_t x[4];
 #pragma unroll
-            for (int i = 0; i < 4; ++i) {
-              const __nv_bfloat162 pr = __floats2bfloat162_rn(__uint_as_float(v[8 * t + 2 * i]) * inv, __uint_as_float(v[8 * t + 2 * i + 1]) * inv);
-              x[i] = *(const uint32_t*)&pr;
-            }
-            *(uint4*)(dst + c0 + 8 * t) = make_uint4(x[0], x[1], x[2], x[3]);
+          for (int i = 0; i < 4; ++i) {
+            const __nv_bfloat162 pr = __floats2bfloat162_rn(__uint_as_float(v[8 * t + 2 * i]) * inv, __uint_as_float(v[8 * t + 2 * i + 1]) * inv);
+            x[i] = *(const uint32_t*)&pr;
           }
+          *(uint4*)(dst + c0 + 8 * t) = make_uint4(x[0], x[1], x[2], x[3]);
         }
       }
     }
@@ -879,20 +846,20 @@ int fa_args(cg_ctx* c, const AttnArgs& a, int D, int BK, CUtensorMap* mq, CUtens
   return CG_OK;
 }
 
-template <int D, int BK, int NQ, bool CAP>
+template <int D, bool CAP>
 int launch_fq(cg_ctx* c, const AttnArgs& a) {
-  constexpr size_t smem = (size_t)(D / 64) * (NQ * 128 + 4 * BK) * 128 + 1024 + 144;
+  constexpr size_t smem = (size_t)(D / 64) * (128 + 4 * FQ_BK) * 128 + 1024 + 136;
   static PerDeviceFlag configured_on;
   bool& configured = configured_on.at(c->core->device);
   if (!configured) {
-    CG_CUDA(c, cudaFuncSetAttribute(k_attn_fq<D, BK, NQ, CAP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    CG_CUDA(c, cudaFuncSetAttribute(k_attn_fq<D, CAP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     configured = true;
   }
   CUtensorMap mq, mk, mv;
   FaArgs p;
-  CG_TRY(fa_args(c, a, D, BK, &mq, &mk, &mv, &p));
-  dim3 grid((unsigned)((a.S + 128 * NQ - 1) / (128 * NQ)), (unsigned)a.nh, (unsigned)(a.rows.rows ? a.rows.rows : a.B));
-  CG_CUDA(c, launch_kernel(c, k_attn_fq<D, BK, NQ, CAP>, grid, dim3(128 + NQ * 128), smem, 1, mq, mk, mv, p));
+  CG_TRY(fa_args(c, a, D, FQ_BK, &mq, &mk, &mv, &p));
+  dim3 grid((unsigned)((a.S + 127) / 128), (unsigned)a.nh, (unsigned)(a.rows.rows ? a.rows.rows : a.B));
+  CG_CUDA(c, launch_kernel(c, k_attn_fq<D, CAP>, grid, dim3(256), smem, 1, mq, mk, mv, p));
   CG_LAUNCHED(c);
   return CG_OK;
 }
@@ -922,6 +889,9 @@ int launch_fa(cg_ctx* c, const AttnArgs& a) {
 // what only k_attn_fa<EXTRA> does
 static bool plain_only(const AttnArgs& a) { return a.bias || (a.gate && a.wide_gate); }
 
+// Rows of 17 tokens and more: against the mma.sync kernel 17 to 63 tokens take 5.3 us for 6.5 (128 rows x heads, head size
+// 64), 10.5 for 26 (416, 128), 7 for 16 (128, 256).  Shorter rows, 5 to 10 us in either, stay there.  With distance
+// biases k_attn_fa takes 64 tokens and more.
 bool attn_fa_supported(const AttnArgs& a) {
   return (a.d == 64 || a.d == 128 || a.d == 256) && !(plain_only(a) && (a.softcap > 0.f || a.d == 256)) && !a.pos_dev && a.S >= (plain_only(a) ? 64 : 17) &&
          (a.rows.rows ? a.rows.M : a.B * a.S) < 2147483647ll && a.B * a.nkv * a.Tmax < 2147483647ll && ((uintptr_t)a.q % 16) == 0 &&
@@ -932,19 +902,16 @@ bool attn_fa_supported(const AttnArgs& a) {
 int k_launch_attn_fa(cg_ctx* c, const AttnArgs& a) {
   if (a.B == 0 || a.S == 0) return CG_OK;
   const bool cap = a.softcap > 0.f;
-  // 64-key tiles: two CTAs per SM (asked for by the option; with biases and wide gates head size 64 gains from it)
+  // k_attn_fa with 64-key tiles: two CTAs per SM (with biases and wide gates head size 64 gains from it)
   const bool k64 = c->opt_fa == 2 || a.d == 64;
   if (plain_only(a)) {
     if (a.d == 64) return launch_fa<64, 64, true>(c, a);
     return k64 ? launch_fa<128, 64, true>(c, a) : launch_fa<128, 128, true>(c, a);
   }
-  // 256 queries that share three 128-key tiles see half of each with a short window: 64-key tiles and 128 queries
-  // waste less (8 x 1024 tokens, 64 heads of 64, window 128: 159 us against 175)
-  const bool narrow = a.d == 64 && !cap && a.window > 0 && a.window <= 256;
-  if (narrow || (c->opt_fa == 2 && a.d <= 128 && !cap)) return a.d == 64 ? launch_fa<64, 64, false>(c, a) : launch_fa<128, 64, false>(c, a);
-  if (a.d == 64) return cap ? launch_fq<64, 128, 2, true>(c, a) : launch_fq<64, 128, 2, false>(c, a);
-  if (a.d == 128) return cap ? launch_fq<128, 128, 2, true>(c, a) : launch_fq<128, 128, 2, false>(c, a);
-  return cap ? launch_fq<256, 64, 1, true>(c, a) : launch_fq<256, 64, 1, false>(c, a);
+  if (c->opt_fa == 2 && a.d <= 128 && !cap) return a.d == 64 ? launch_fa<64, 64, false>(c, a) : launch_fa<128, 64, false>(c, a);
+  if (a.d == 64) return cap ? launch_fq<64, true>(c, a) : launch_fq<64, false>(c, a);
+  if (a.d == 128) return cap ? launch_fq<128, true>(c, a) : launch_fq<128, false>(c, a);
+  return cap ? launch_fq<256, true>(c, a) : launch_fq<256, false>(c, a);
 }
 
 }  // namespace cg

@@ -308,7 +308,7 @@ def test_fused_attention_tcgen05(cuda, b, nh, nkv, s, d, variant):
                                           (256, 100, 50.0), (128, 100, 0.0)])
 @pytest.mark.parametrize("s", [17, 40, 64, 127, 128, 129, 256, 257, 600])
 def test_fused_attention_query_tiles(cuda, d, window, cap, s):
-    """The two-query-tile prefill attention where its tiles end: one tile and none beside it, one row of the second, whole
+    """The prefill attention where its tiles (128 queries, 64 keys) end: one tile, one row of the second, whole
     tiles, windows that end inside a tile, growing scores (the outputs' rescaling), against float64.  Each probability and
     the result are rounded to bf16, 2^-9 of itself: an output, a mean of values, is off by at most 2^-8 of the largest value."""
     b, nh, nkv = 2, 2, 1
@@ -333,7 +333,7 @@ def test_fused_attention_rounds_against_the_running_maximum(cuda, d, window, cap
     """Peaked scores: what the result may lose is what rounding costs, each probability to bf16 against its row's largest
     score so far (tile by tile) and the result to bf16.  That error, emulated in float64, is the bound; 2 % more for the order
     of sums and exponentials of 32 bits.  Probabilities against a maximum left behind cost 4 to 17 % more."""
-    s, nh, tile = 700, 4, 64 if d == 256 else 128
+    s, nh, tile = 700, 4, 64
     q, k, v = (synth.bf16_round(rnd((1, nh, s, d))) for _ in range(3))
     q = synth.bf16_round(q * spread)
     got = cuda.to_numpy(cuda.fused_attention(cuda.from_numpy(q), cuda.from_numpy(k), cuda.from_numpy(v), window, cap))
