@@ -461,7 +461,7 @@ k_gemm_dec(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CU
     asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
   }
   // with split-K a CTA whose accumulator never came pushes all the same: its peers count on the bytes
-  // (the error word is set, and nothing is written from them)
+  // (the error word is set: what a peer makes of them is not a result)
   if (warp >= 2 && (acc_ok || cluster)) {
     const int q = warp & 3;
     const int row = q * 32 + lane;
@@ -588,7 +588,7 @@ k_gemm_dec(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CU
     }
     __syncwarp();
     asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
-    if (*cta_abort) mbar_wait_cluster(bar_x, 0, cta_abort, p.err);  // (what is still on its way, after a wait gave up)
+    if (*cta_abort) mbar_drain(bar_x, 0, p.err);  // (issued is not arrived: what is still on its way, after a wait gave up)
   }
 
   if (p.out_mode == 3) {

@@ -93,6 +93,21 @@ __device__ __forceinline__ bool mbar_wait_cluster(uint32_t bar, uint32_t parity,
   *err = DEV_TIMEOUT;
   return false;
 }
+// Where a wait has given up: polls for a phase that is certain to come (every byte it counts has been sent), whatever has
+// been reported, so that a CTA does not leave shared memory that others still write to.  Bounded like every wait.
+__device__ __forceinline__ void mbar_drain(uint32_t bar, uint32_t parity, const int32_t* err) {
+  const uint64_t t0 = globaltimer(), limit = wait_limit_ns(err);
+  uint32_t done = 0;
+  do {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(done)
+        : "r"(bar), "r"(parity)
+        : "memory");
+  } while (!done && globaltimer() - t0 <= limit);
+}
 __device__ __forceinline__ uint32_t cluster_ctarank() {
   uint32_t r;
   asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));

@@ -26,3 +26,16 @@ def test_prompt_attention_takes_tmem_between_its_dependency_and_its_trigger():
     for name in ("k_attn_fa", "k_attn_fq"):
         wait, alloc, trigger = places(kernel("attention_fa.cu", name), "griddepcontrol.wait;", "tcgen05.alloc.", "griddepcontrol.launch_dependents;")
         assert wait < alloc < trigger
+
+
+def test_pushes_to_a_cta_that_gave_up_are_counted_out_before_it_leaves():
+    """A CTA of the decode GEMM that has given up on a wait may still be pushed to when every peer has passed the last cluster
+    barrier (issued is not arrived).  It polls for the bytes whatever has been reported: a wait that ends early because the
+    error is known would let it leave."""
+    body = kernel("gemm_dec.cu", "k_gemm_dec")
+    last = body.rindex("barrier.cluster.wait.acquire.aligned")
+    assert "if (*cta_abort) mbar_drain(bar_x, 0, p.err);" in body[last:] and "mbar_wait" not in body[last:]
+    common = open(os.path.join(CSRC, "tc_common.cuh")).read()
+    drain = common[common.index("void mbar_drain("):]
+    drain = drain[:drain.index("\n}\n")]
+    assert "abort" not in drain and "DEV_TIMEOUT" not in drain and "limit" in drain
