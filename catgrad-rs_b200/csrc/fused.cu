@@ -711,6 +711,12 @@ k_argmax_part_vec(float* logits, int64_t Vp, float softcap, unsigned long long* 
     atomicMax(best_out + b, best);
   }
 }
+// One more cached position.  Released: kernels of the next step read the counter before their dependency wait (with
+// ld.acquire) and conclude from it that the states which this step's kernels wrote are complete; this kernel's own
+// wait has ordered their stores before it.
+__device__ __forceinline__ void step_done(int64_t* pos_dev) {
+  asm volatile("st.release.gpu.global.s64 [%0], %1;" ::"l"(pos_dev), "l"(*pos_dev + 1) : "memory");
+}
 // publish the tokens, clear the merge slots for the next step and, when asked, count one
 // more generated token and one more cached position
 __global__ void k_argmax_finish(unsigned long long* best, int64_t B, uint32_t* tokens, uint32_t* history, int64_t hist_ld,
@@ -727,7 +733,7 @@ __global__ void k_argmax_finish(unsigned long long* best, int64_t B, uint32_t* t
   __syncthreads();
   if (threadIdx.x == 0 && advance) {
     *count_dev = count + 1;
-    *pos_dev += 1;
+    step_done(pos_dev);
   }
 }
 
@@ -799,7 +805,7 @@ __global__ void k_argmax_finish_tp(PeerPush px, unsigned long long* best, int64_
   __syncthreads();
   if (threadIdx.x == 0 && advance) {
     *count_dev = count + 1;
-    *pos_dev += 1;
+    step_done(pos_dev);
   }
 }
 

@@ -236,7 +236,8 @@ __global__ void __launch_bounds__(256, RD_ROWS <= 8 ? 3 : 2) k_recur_decode(Recu
   // The state is on its way while the projection still runs.  Its last writer is this layer run's kernel of the step
   // before, and the step counter is raised (behind its own dependency wait) only when that step's kernels are
   // complete: if the counter read here is still the one behind the wait, what was read is what they left;
-  // else the step before was not over, and the state is read again.
+  // else the step before was not over, and the state is read again.  (Prompts and row tables lie behind copies, which no
+  // early launch passes.)
   const int slot = a.rows.slot[row];
   float* Sg = a.S + ((int64_t)slot * a.H + h) * a.dk * a.dvs;
   float4 S[RD_ROWS];

@@ -39,3 +39,18 @@ def test_pushes_to_a_cta_that_gave_up_are_counted_out_before_it_leaves():
     drain = common[common.index("void mbar_drain("):]
     drain = drain[:drain.index("\n}\n")]
     assert "abort" not in drain and "DEV_TIMEOUT" not in drain and "limit" in drain
+
+
+def test_the_step_counter_is_released_to_early_readers():
+    """k_recur_decode reads its state before its dependency wait and trusts it if the step counter (ld.acquire) has not moved:
+    whoever raises the counter has to release what the step wrote."""
+    early = open(os.path.join(CSRC, "recurrent.cu")).read()
+    assert early.count("ld.acquire.gpu.global.s64") == 2
+    text = open(os.path.join(CSRC, "fused.cu")).read()
+    assert "*pos_dev +=" not in text and "++*pos_dev" not in text
+    raised = text[text.index("void step_done("):]
+    assert "st.release.gpu.global.s64" in raised[:raised.index("\n}\n")]
+    for name in ("k_argmax_finish", "k_argmax_finish_tp"):
+        body = text[text.index(f" {name}("):]
+        body = body[:body.index("\n}\n")]
+        assert body.index("griddepcontrol.wait;") < body.index("step_done(pos_dev);")
