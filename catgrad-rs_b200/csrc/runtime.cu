@@ -95,11 +95,13 @@ static bool mostly_new_pages(const void* dst, size_t bytes) {
 }
 
 // `bytes` from the device to host memory, complete on return.  The driver copies to pageable memory on the
-// calling thread, 3 to 4 GB/s where the destination's pages are new.  Reads of a megabyte and more (a batch's
-// logits) into new pages come through pinned segments instead, which four threads empty into the destination
-// while the next ones arrive: segment k waits in slot k mod 16, and the thread that empties a slot asks for the
-// segment 16 further on.  Before -> now: 7.8 MB 2513 -> 1177 us, 16.8 MB 4902 -> 2137 us.  Into pages in use the
-// driver is as fast as the threads (a forward of 2.2 ms that reads 7.8 MB of logits: 0.3 ms longer with them).
+// calling thread, 3 to 4 GB/s where the destination's pages are new.  Reads of more than one segment (512 KB: a
+// batch's logits) into new pages come through pinned segments instead, which four threads (one for two segments) empty
+// into the destination while the next ones arrive: segment k waits in slot k mod 16, and the thread that empties a slot
+// asks for the segment 16 further on.  Before -> now: 1.05 MB 573 -> 330 us, 6.7 MB 3400 -> 1390, 16.8 MB 8500 -> 2880; the
+// context's first such read pays 5 ms for the pinned memory.  Into pages in use the driver is as fast as the threads
+// (6.7 MB: 415 us).  Threads that read from one context take turns, as they do in the driver (two of 6.7 MB: 6.8 -> 2.9 ms;
+// going the driver's way while another has the segments: 3.9).
 cudaError_t Core::copy_out(void* dst, const void* src, size_t bytes) {
   const int n = (int)((bytes + OUT_SEG - 1) / OUT_SEG);
   cudaPointerAttributes at;

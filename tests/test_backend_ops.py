@@ -2,6 +2,9 @@
 seeded inputs, through the C ABI.  Integer / index / byte-moving results must be
 bit-exact; f32 arithmetic that only moves or compares values too; pow/sin/cos within one
 ulp; sums and GEMMs within 1e-5 relative (summation order differs)."""
+import mmap
+import threading
+
 import numpy as np
 import pytest
 
@@ -270,3 +273,55 @@ def test_to_vec_and_shape_are_host_metadata(cuda):
     before = cuda.launch_count()
     _ = cuda.broadcast(cuda.slice(cuda.transpose(x, 0, 1), 0, 1, 2), (5, 2, 3)).shape
     assert cuda.launch_count() == before  # views launch nothing
+
+
+# one segment of the pinned way and the first size beyond it, two and three, all slots, slots used again, a short last one
+READ_SIZES = [n for seg in (1, 2, 3, 16, 17, 39) for n in (seg * 131072, seg * 131072 + 1)]
+
+
+def read_into(B, t, n, address):
+    B._check(B._f("to_vec_u32")(B._ctx, t._h, address, n))
+
+
+def fresh(nbytes):
+    """Memory whose pages nothing has touched."""
+    m = mmap.mmap(-1, nbytes + 4096)
+    return m, np.frombuffer(m, np.uint32)
+
+
+@pytest.mark.parametrize("n", READ_SIZES)
+@pytest.mark.parametrize("touched", [False, True], ids=["new pages", "pages in use"])
+def test_large_reads(cuda, n, touched):
+    """Results read into memory of any kind and size come whole: pinned segments for new pages, the driver's copy else."""
+    want = (np.arange(n, dtype=np.uint32) * np.uint32(2654435761)) ^ np.uint32(n)
+    t = cuda.from_numpy(want)
+    for offset in (0, 5):   # of the first value in its page
+        m, view = fresh(4 * n)
+        if touched:
+            view.fill(1)
+        read_into(cuda, t, n, view.ctypes.data + 4 * offset)
+        np.testing.assert_array_equal(view[offset:offset + n], want)
+        assert touched or (not view[:offset].any() and not view[offset + n:].any())
+
+
+def test_large_reads_of_several_threads(cuda):
+    """They share one context's pinned segments."""
+    sizes = [1953000, 1667328, 4194304, 300001]
+    want = [np.arange(n, dtype=np.uint32) * np.uint32(40503 + 2 * i) for i, n in enumerate(sizes)]
+    tensors = [cuda.from_numpy(w) for w in want]
+    cuda.sync()
+    wrong = []
+
+    def read(i):
+        for _ in range(4):
+            m, view = fresh(4 * sizes[i])
+            read_into(cuda, tensors[i], sizes[i], view.ctypes.data)
+            if not np.array_equal(view[:sizes[i]], want[i]):
+                wrong.append(i)
+
+    threads = [threading.Thread(target=read, args=(i,)) for i in range(len(sizes))]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not wrong
