@@ -63,7 +63,6 @@ struct DecArgs {
   int lg_rows_per;  // log2 of the rows of a tile that a split finishes (128 / splits)
   int x_rows;       // activation rows per k block in the ring (8 or TN)
   int xstage_cols;  // split-K: token columns of the exchange area (>= min(TN, M)); 0 without split-K
-  int quads;        // TN 32: groups of four tokens
   int xstage_in_ring;  // the exchange area lies over the ring (more than 16 tokens: it would cost the ring a
                        // stage): then a first cluster barrier says every CTA's ring is idle before anyone pushes
   int32_t* err;
@@ -138,77 +137,6 @@ __device__ __forceinline__ void st_async(uint32_t addr, uint32_t v, uint32_t bar
                : "memory");
 }
 
-__device__ __forceinline__ void st_async4(uint32_t addr, const uint32_t* v, uint32_t bar) {
-  asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.v4.b32 [%0], {%1, %2, %3, %4}, [%5];" ::"r"(addr), "r"(v[0]), "r"(v[1]),
-               "r"(v[2]), "r"(v[3]), "r"(bar)
-               : "memory");
-}
-
-// Above 16 tokens: the quads (four tokens' row) a CTA finishes behind the exchange, the splits' partial sums in rank
-// order.  S is the number of splits, so there are exactly as many loads; a thread has up to sixteen
-// turns here, and one value per turn with sixteen predicated loads each cost the paired GEMM of the
-// Llama-3-8B shape 14 us of 58.
-template <int S>
-__device__ __forceinline__ void finish_quads(const DecArgs& p, const float* xs, float* sq, const float* sc, bool got, int et, int split, int n0,
-                                             uint32_t parity, const Prefetched* pre) {
-  constexpr int LG = S == 2 ? 6 : S == 4 ? 5 : S == 8 ? 4 : 3;  // log2 of the rows this CTA finishes
-  constexpr int CH = S < 4 ? S : 4;                             // splits at a time: what the registers hold
-  const int groups = p.quads, stride4 = (groups * (p.dual ? 2 : 1)) | 1;
-  const int todo = groups << LG;
-#pragma unroll 1
-  for (int e = et; e < todo + et; e += 128) {  // (the same number of turns for every thread)
-    const int grp = e >> LG, rl = e & ((1 << LG) - 1);
-    const bool in = got && e < todo;
-    const int n = n0 + (split << LG) + rl;
-    float r2[4] = {0.f, 0.f, 0.f, 0.f};
-    if (in && n < p.N) {
-      Prefetched q[4];
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        q[j] = e == et ? pre[j] : Prefetched{false, 0.f, 0.f};
-        if (!q[j].have && p.out_mode == 2 && grp * 4 + j < p.M) {
-          q[j].have = true;
-          q[j].res = p.residual[(int64_t)(grp * 4 + j) * p.ldo + n];
-          if (p.xb_out) q[j].gain = p.g_next[n];
-        }
-      }
-      const float4* x0 = (const float4*)xs + rl * stride4 + grp;
-      float4 a = make_float4(0.f, 0.f, 0.f, 0.f), b = a;
-#pragma unroll
-      for (int t0 = 0; t0 < S; t0 += CH) {
-        float4 pg[CH], pu[CH];
-#pragma unroll
-        for (int t = 0; t < CH; ++t) pg[t] = x0[((t0 + t) << LG) * stride4];
-        if (p.dual)
-#pragma unroll
-          for (int t = 0; t < CH; ++t) pu[t] = x0[((t0 + t) << LG) * stride4 + groups];
-#pragma unroll
-        for (int t = 0; t < CH; ++t) { a.x += pg[t].x; a.y += pg[t].y; a.z += pg[t].z; a.w += pg[t].w; }
-        if (p.dual)
-#pragma unroll
-          for (int t = 0; t < CH; ++t) { b.x += pu[t].x; b.y += pu[t].y; b.z += pu[t].z; b.w += pu[t].w; }
-      }
-      const float g[4] = {a.x, a.y, a.z, a.w}, u[4] = {b.x, b.y, b.z, b.w};
-#pragma unroll
-      for (int j = 0; j < 4; ++j)
-        if (grp * 4 + j < p.M) r2[j] = finish(p, grp * 4 + j, n, g[j], u[j], parity, sc, q[j]);
-    }
-    if (p.ss_out) {
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        if (LG <= 5) {
-          // a token's rows are neighbouring lanes
-#pragma unroll
-          for (int o = 1 << LG >> 1; o; o >>= 1) r2[j] += __shfl_xor_sync(0xffffffffu, r2[j], o);
-          if (in && rl == 0 && grp * 4 + j < p.M) p.ss_out[((int64_t)blockIdx.x * S + split) * 32 + grp * 4 + j] = r2[j];
-        } else if (in) {
-          sq[((grp * 4 + j) << LG) + rl] = r2[j];
-        }
-      }
-    }
-  }
-}
-
 // Activation chunks (16 bytes) of the first k blocks: chunk id = ((k block * x_rows) + row) * 8 + place.
 // Rows past M are not read (they feed unused columns); places past K are zero.
 constexpr int XCH = 4;
@@ -254,15 +182,10 @@ k_gemm_dec(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CU
   const int STAGES = p.stages;
   const uint32_t wbytes = p.dual ? 2 * A_BYTES : A_BYTES;
   const uint32_t stage_bytes = wbytes + X_TILE;
-  // split-K exchange area.  Up to 16 tokens [splits][(1 + dual) * xstage_cols][128 / splits] f32
+  // split-K exchange area [splits][(1 + dual) * xstage_cols][128 / splits] f32.  Up to 16 tokens it lies
   // behind the ring (not inside it: the other CTAs of the cluster write here while this CTA may
-  // still be streaming).  Above [splits][128 / splits][quads of gate, quads of up] of four tokens each, a row
-  // an odd number of quads long so that eight neighbouring rows lie in different banks, inside the ring,
-  // guarded by one more cluster barrier.
-  constexpr bool QUAD = TN == 32;
-  const int stride4 = (p.quads * (p.dual ? 2 : 1)) | 1;
-  const uint32_t xbytes =
-      p.splits == 1 ? 0u : QUAD ? (uint32_t)stride4 * 16u * BM : (uint32_t)((p.dual ? 2 : 1) * p.xstage_cols) * BM * 4u;
+  // still be streaming); above, inside the ring, guarded by one more cluster barrier.
+  const uint32_t xbytes = (uint32_t)((p.dual ? 2 : 1) * p.xstage_cols) * BM * 4u;
   const uint32_t xoff = p.xstage_in_ring ? 0u : STAGES * stage_bytes;
   const uint32_t boff = STAGES * stage_bytes + (p.xstage_in_ring ? 0u : xbytes);
   const uint32_t bars = base + boff;  // full[STAGES], empty[STAGES], accum
@@ -293,7 +216,7 @@ k_gemm_dec(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CU
     if (cluster) {
       // all 128 rows / splits rows of every split, M tokens of one or two accumulators
       mbar_init(bar_x, 1);
-      mbar_expect_tx(bar_x, (uint32_t)((p.dual ? 2 : 1) * (QUAD ? 4 * p.quads : p.M)) * BM * 4u);
+      mbar_expect_tx(bar_x, (uint32_t)((p.dual ? 2 : 1) * p.M) * BM * 4u);
     }
     *cta_abort = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -323,9 +246,7 @@ k_gemm_dec(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CU
   if (cluster && !p.xstage_in_ring) asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
 
   bool acc_ok = false;
-  Prefetched pre[QUAD ? 4 : 1];
-#pragma unroll
-  for (int j = 0; j < (QUAD ? 4 : 1); ++j) pre[j] = Prefetched{false, 0.f, 0.f};
+  Prefetched pre{false, 0.f, 0.f};
   if (warp == 0) {
     if (lane == 0) {
       const int pre = min(nkb, STAGES);
@@ -395,19 +316,13 @@ k_gemm_dec(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CU
       // split-K: the element this thread will finish first is known now; fetch its residual (and
       // the next norm's gain) while the MMAs run instead of after the reduction
       const int lg = p.lg_rows_per;
-      if (et < (QUAD ? p.quads : p.M) << lg) {
-        const int col = (et >> lg) * (QUAD ? 4 : 1);
+      if (et < min(TN, p.M) << lg) {
+        const int col = et >> lg;
         const int n = n0 + (split << lg) + (et & ((1 << lg) - 1));
         if (n < p.N) {
-          float gain = 0.f;
-          if (p.xb_out) asm volatile("ld.global.f32 %0, [%1];" : "=f"(gain) : "l"(p.g_next + n) : "memory");
-#pragma unroll
-          for (int j = 0; j < (QUAD ? 4 : 1); ++j)
-            if (col + j < p.M) {
-              asm volatile("ld.global.f32 %0, [%1];" : "=f"(pre[j].res) : "l"(p.residual + (int64_t)(col + j) * p.ldo + n) : "memory");
-              pre[j].gain = gain;
-              pre[j].have = true;
-            }
+          asm volatile("ld.global.f32 %0, [%1];" : "=f"(pre.res) : "l"(p.residual + (int64_t)col * p.ldo + n) : "memory");
+          if (p.xb_out) asm volatile("ld.global.f32 %0, [%1];" : "=f"(pre.gain) : "l"(p.g_next + n) : "memory");
+          pre.have = true;
         }
       }
     }
@@ -475,8 +390,7 @@ k_gemm_dec(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CU
       const uint32_t owner = (uint32_t)(row >> lg);
       asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(xdst) : "r"(base + xoff), "r"(owner));
       asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(xbar) : "r"(bar_x), "r"(owner));
-      const int rl = row & ((1 << lg) - 1);
-      xdst += QUAD ? (uint32_t)(((split << lg) + rl) * stride4) * 16u : (uint32_t)(((split * xcols) << lg) + rl) * 4u;
+      xdst += (uint32_t)(((split * xcols) << lg) + (row & ((1 << lg) - 1))) * 4u;
     }
 #pragma unroll 1
     for (int c0 = 0; c0 < TN; c0 += 16) {
@@ -485,15 +399,7 @@ k_gemm_dec(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CU
       tmem_ld16(tmem_acc + ((uint32_t)(q * 32) << 16) + (uint32_t)c0, g);
       if (p.dual) tmem_ld16(tmem_acc + ((uint32_t)(q * 32) << 16) + (uint32_t)(TN + c0), u);
       asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-      if (cluster && QUAD) {
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          const int quad = (c0 >> 2) + j;
-          if (quad >= p.quads) break;
-          st_async4(xdst + (uint32_t)quad * 16u, g + 4 * j, xbar);
-          if (p.dual) st_async4(xdst + (uint32_t)(p.quads + quad) * 16u, u + 4 * j, xbar);
-        }
-      } else if (cluster) {
+      if (cluster) {
 #pragma unroll
         for (int j = 0; j < 16; ++j) {
           if (c0 + j >= p.M) break;
@@ -537,49 +443,40 @@ k_gemm_dec(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CU
     if (warp >= 2) {
       const bool got = mbar_wait_cluster(bar_x, 0, cta_abort, p.err) && !*cta_abort;
       const int S = p.splits, lg = p.lg_rows_per, et = tid - 64;
+      const int todo = min(TN, p.M) << lg;  // columns x rows this CTA finishes
+      const int xcols = (p.dual ? 2 : 1) * p.xstage_cols;
       const float* xs = (const float*)(gen + xoff);
-      if (QUAD) {
-        switch (S) {
-          case 2: finish_quads<2>(p, xs, sq, sc, got, et, split, n0, parity, pre); break;
-          case 4: finish_quads<4>(p, xs, sq, sc, got, et, split, n0, parity, pre); break;
-          case 8: finish_quads<8>(p, xs, sq, sc, got, et, split, n0, parity, pre); break;
-          default: finish_quads<16>(p, xs, sq, sc, got, et, split, n0, parity, pre); break;
+      for (int e = et; e < todo + et; e += 128) {  // (the same number of turns for every thread)
+        const int col = e >> lg, rl = e & ((1 << lg) - 1);
+        const bool in = got && e < todo;
+        float r2 = 0.f;
+        if (in) {
+          // the splits' partial sums in rank order (all loads first)
+          const float* x0 = xs + (col << lg) + rl;
+          const int step = xcols << lg, up = p.xstage_cols << lg;
+          float pg[16], pu[16];
+#pragma unroll
+          for (int s = 0; s < 16; ++s) {
+            pg[s] = s < S ? x0[s * step] : 0.f;
+            pu[s] = (p.dual && s < S) ? x0[s * step + up] : 0.f;
+          }
+          float g = 0.f, u = 0.f;
+#pragma unroll
+          for (int s = 0; s < 16; ++s) { g += pg[s]; u += pu[s]; }  // the zeros of absent ranks change nothing
+          const int n = n0 + (split << lg) + rl;
+          if (n < p.N) r2 = finish(p, col, n, g, u, parity, sc, e == et ? pre : Prefetched{false, 0.f, 0.f});
         }
-      } else {
-        const int todo = p.M << lg;  // columns x rows this CTA finishes
-        const int xcols = (p.dual ? 2 : 1) * p.xstage_cols;
-        for (int e = et; e < todo + et; e += 128) {  // (the same number of turns for every thread)
-          const int col = e >> lg, rl = e & ((1 << lg) - 1);
-          const bool in = got && e < todo;
-          float r2 = 0.f;
-          if (in) {
-            // the splits' partial sums in rank order (all loads first)
-            const float* x0 = xs + (col << lg) + rl;
-            const int step = xcols << lg, up = p.xstage_cols << lg;
-            float pg[16], pu[16];
-#pragma unroll
-            for (int s = 0; s < 16; ++s) {
-              pg[s] = s < S ? x0[s * step] : 0.f;
-              pu[s] = (p.dual && s < S) ? x0[s * step + up] : 0.f;
-            }
-            float g = 0.f, u = 0.f;
-#pragma unroll
-            for (int s = 0; s < 16; ++s) { g += pg[s]; u += pu[s]; }  // the zeros of absent ranks change nothing
-            const int n = n0 + (split << lg) + rl;
-            if (n < p.N) r2 = finish(p, col, n, g, u, parity, sc, e == et ? pre[0] : Prefetched{false, 0.f, 0.f});
-          }
-          if (p.ss_out && lg <= 5) {
-            // a token's rows are neighbouring lanes
-            for (int o = 1 << lg >> 1; o; o >>= 1) r2 += __shfl_xor_sync(0xffffffffu, r2, o);
-            if (in && rl == 0) p.ss_out[((int64_t)blockIdx.x * S + split) * 32 + col] = r2;
-          } else if (p.ss_out && in) {
-            sq[e] = r2;
-          }
+        if (p.ss_out && lg <= 5) {
+          // a token's rows are neighbouring lanes
+          for (int o = 1 << lg >> 1; o; o >>= 1) r2 += __shfl_xor_sync(0xffffffffu, r2, o);
+          if (in && rl == 0) p.ss_out[((int64_t)blockIdx.x * S + split) * 32 + col] = r2;
+        } else if (p.ss_out && in) {
+          sq[e] = r2;
         }
       }
       if (p.ss_out && lg > 5) {
         asm volatile("bar.sync 2, 128;" ::: "memory");
-        if (got && et < p.M) {
+        if (got && et < min(TN, p.M)) {
           float a = 0.f;
           for (int i = 0; i < 1 << lg; ++i) a += sq[(et << lg) + i];
           p.ss_out[((int64_t)blockIdx.x * S + split) * 32 + et] = a;
@@ -664,8 +561,7 @@ int gemm_dec(cg_ctx* c, const DecGemm& g) {
   // comes out of the same budget: three CTAs per SM may use 75 KB each, two 113 KB each.
   const int xstage_cols = splits > 1 ? (int)std::min<int64_t>(tn, g.M) : 0;
   const bool x_in_ring = tn == 32;  // above 16 tokens a separate area would cost the ring a stage (measured: 3 % per step)
-  const int quads = (int)((g.M + 3) / 4);
-  const size_t xarea = splits == 1 ? 0 : x_in_ring ? (size_t)((quads * (g.dual ? 2 : 1)) | 1) * 16 * BM : (size_t)(g.dual ? 2 : 1) * xstage_cols * BM * 4;
+  const size_t xarea = (size_t)(g.dual ? 2 : 1) * xstage_cols * BM * 4;
   const size_t xbytes = x_in_ring ? 0 : xarea;
   // (with the 8-row box the MMA of the last stage reads 1 KB past its activation slot: keep that inside the allocation)
   const size_t fixed = 1024 + 16 * 8 + 64 + 5 * 128 + (x_rows < tn ? 1024 : 0);
@@ -695,7 +591,7 @@ int gemm_dec(cg_ctx* c, const DecGemm& g) {
   while (BM >> (a.lg_rows_per + 1) >= splits) ++a.lg_rows_per;
   a.x_rows = x_rows;
   a.x = (const __nv_bfloat16*)g.x; a.ldx = g.ldx;
-  a.xstage_cols = xstage_cols; a.quads = quads;
+  a.xstage_cols = xstage_cols;
   a.xstage_in_ring = x_in_ring && splits > 1 ? 1 : 0;
   a.err = c->core->dev_err;
   a.trace = c->trace_on ? (int)(c->trace_next++ % TRACE_SLOTS) : -1;
