@@ -480,7 +480,7 @@ k_attn_fa(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUt
 // One layer, before (k_attn_fa; head size 256, soft-caps and rows of less than 64 tokens k_attn_prefill on mma.sync) -> now:
 // 1 x 8191 tokens, 32 heads of 128: 1188 -> 710 us (774 TFLOP/s); 32 x 509: 319 -> 183; 8 x 512, 32 heads of 64: 56 -> 44;
 // 13 x 389: 78 -> 63; 4 x 2048, 8 heads of 256, soft-cap: 768 -> 189 (364 TFLOP/s).  Over 456 shapes (17 to 2000 tokens, 8 to
-// 416 rows x heads, windows of 64 to 512, with and without soft-cap) it takes 0.14 to 0.95 of the time, 0.57 in the mean.
+// 416 rows x heads, windows of 64 to 512, with and without soft-cap) it takes 0.16 to 0.95 of the time, 0.57 in the mean.
 constexpr int FQ_BK = 64;  // keys per tile
 
 __device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t* v) {

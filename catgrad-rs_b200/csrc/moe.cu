@@ -481,7 +481,8 @@ __global__ void k_moe_combine(const float* y, const int32_t* pos, const float* w
 
 // out[t, :] = x[t, :] + the sum of k_moe_combine, and the norm the next block starts with, bf16(out / rms * gamma)
 // (k_rmsnorm's arithmetic): a block per token, its row in registers.  One dependent launch less per layer of a step
-// (with k_moe_topk_plan 703 -> 688 us for four layers); a prompt saves the norm's read of the residual stream.
+// (with k_moe_topk_plan 703 -> 688 us for four layers); a prompt saves the norm's read of the residual stream (8192 tokens
+// of 2048: 106 us and a norm of 19 -> 107; three layers of the Qwen3-30B-A3B shape, 1 x 24 to 32 x 300 tokens: 0.5 to 2 %).
 constexpr int CN_THREADS = 256, CN_VECS = 8;
 __global__ void __launch_bounds__(CN_THREADS)
 k_moe_combine_norm(const float* y, const int32_t* pos, const float* wts, int k, int H, const float* x, float* out, const float* gamma,

@@ -310,7 +310,8 @@ def test_fused_attention_tcgen05(cuda, b, nh, nkv, s, d, variant):
 def test_fused_attention_query_tiles(cuda, d, window, cap, s):
     """The prefill attention where its tiles (128 queries, 64 keys) end: one tile, one row of the second, whole
     tiles, windows that end inside a tile, growing scores (the outputs' rescaling), against float64.  Each probability and
-    the result are rounded to bf16, 2^-9 of itself: an output, a mean of values, is off by at most 2^-8 of the largest value."""
+    the result are rounded to bf16, by at most 2^-8 of itself.  The probabilities' errors all but cancel in a mean of values
+    (1e-3 is left for them), the result's is at most 2^-8 of the largest value."""
     b, nh, nkv = 2, 2, 1
     q, k, v = (synth.bf16_round(rnd((b, n, s, d))) for n in (nh, nkv, nkv))
     k = synth.bf16_round(k * np.linspace(0.2, 4.0, s, dtype=np.float32)[:, None])  # maxima that grow along the keys
