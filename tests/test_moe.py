@@ -65,7 +65,8 @@ def test_fused_moe_matches_op_stream(oracle, cuda_bf16, S, H, E, Fe, k, renorm):
 # threads, a hidden size that ends inside a block's walk; the last rows that fit the 48 KB a launch has without asking
 # (32 tokens, k = 2: 357 experts, beside 256 bytes of the kernel's own) and those that do not, with few and many choices
 @pytest.mark.gpu
-@pytest.mark.parametrize("S,H,E,Fe,k", [(31, 72, 16, 32, 3), (32, 72, 16, 32, 3), (33, 72, 16, 32, 3), (2, 64, 700, 8, 32), (1, 1032, 8, 32, 8),
+@pytest.mark.parametrize("S,H,E,Fe,k", [(31, 72, 16, 32, 3), (32, 72, 16, 32, 3), (33, 72, 16, 32, 3), (2, 64, 700, 8, 32), (32, 64, 340, 8, 2),
+                                        (32, 64, 372, 8, 2), (1, 1032, 8, 32, 8),
                                         (32, 64, 356, 8, 2), (32, 64, 357, 8, 2), (32, 64, 358, 8, 2), (32, 64, 359, 8, 2), (32, 64, 360, 8, 2),
                                         (32, 64, 352, 8, 10), (32, 64, 353, 8, 8)])
 def test_fused_moe_choice_and_plan(oracle, cuda_bf16, S, H, E, Fe, k):
