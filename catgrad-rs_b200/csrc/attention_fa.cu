@@ -26,6 +26,7 @@
 
 #include "act.cuh"
 #include "kernels.h"
+#include "mma.cuh"
 #include "tc_common.cuh"
 
 namespace cg {
@@ -72,12 +73,6 @@ __device__ __forceinline__ uint64_t umma_desc_mn(uint32_t saddr, uint32_t chunk_
 
 // the lowest n bits, n of any size
 __device__ __forceinline__ uint32_t bits_below(int n) { return n <= 0 ? 0u : n >= 32 ? 0xffffffffu : (1u << n) - 1u; }
-
-__device__ __forceinline__ float fast_exp2(float x) {
-  float y;
-  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-  return y;
-}
 
 // 32 consecutive TMEM columns of this thread's lane
 __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t* v) {
@@ -499,15 +494,6 @@ __device__ __forceinline__ void umma_bf16_ts(uint32_t tmem_d, uint32_t tmem_a, u
       ::"r"(tmem_d), "r"(tmem_a), "l"(db), "r"(idesc), "r"(accumulate)
       : "memory");
 }
-// 1 / x for x >= 1 (as good as 0 above 1e37): the approximation and one step of Newton's iteration, so that a soft-capped
-// score keeps its 24 bits.  (2048 tokens, 8 heads of 256: 183 us without the step, 189 with it, 455 with a division.)
-__device__ __forceinline__ float rcp_newton(float x) {
-  float y;
-  x = x > 1e37f ? 1e37f : x;  // (a NaN stays one)
-  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-  return fmaf(y, fmaf(-x, y, 1.f), y);
-}
-
 template <int D, bool CAP>
 __global__ void __launch_bounds__(256, D <= 128 ? 2 : 1)
 k_attn_fq(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,

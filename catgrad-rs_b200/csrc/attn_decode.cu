@@ -6,20 +6,18 @@
 // the masked softmax(q k^T / sqrt(d)) v of catgrad-llm/src/models/llama.rs:97-108 and the
 // cache append of catgrad-llm/src/legacy/models/utils.rs:210-228:
 //
-//   1. request this CTA's slice of cached keys and values (16-byte cp.async, coalesced)
+//   1. request this CTA's slice of cached keys and values (TMA, a tile of each per warp)
 //      before anything else, then, while they fly, split the f32 qkv row, normalise / rotate
 //      q and the new k, round them to bf16 (the cache precision) and append k, v to the cache;
 //   2. the query heads that share the kv head are the rows of one 16-row MMA tile, so
 //      q k^T and p v for 32 keys are a few mma.sync instructions per warp instead of
 //      thousands of scalar FMAs; online softmax per head;
-//   3. the slices of one (row, kv head) form a thread-block cluster: each leaves its partial
-//      (max, sum, weighted values) in shared memory and, after one cluster barrier, the
-//      partials are merged over distributed shared memory into the bf16 output that the
-//      output projection reads.  No scratch in HBM, no second kernel.
+//   3. the slices of one (row, kv head) form a thread-block cluster: each pushes its partials
+//      (max, sum, weighted values) to the CTA that finishes them, which merges them out of its own shared
+//      memory into the bf16 output that the output projection reads.  No scratch in HBM, no second kernel.
 //
 // The whole block is latency-bound (a few MB per layer), so the design minimises dependent
 // round trips and instruction count rather than bytes.
-#include <algorithm>
 
 #include "attn_decode.cuh"
 #include "kernels.h"
@@ -43,6 +41,7 @@ struct KernelEnv {
   // one item per CTA: partials are pushed into the finishing CTA's landing area
   static constexpr bool kPush = true;
   float* land;
+  const CUtensorMap *map_k, *map_v;
   __device__ __forceinline__ float* landing() const { return land; }
   // the projected row, and the position when it lives on the device, belong to the stream order
   const AttnDecArgs* args;
@@ -55,11 +54,16 @@ struct KernelEnv {
 };
 
 template <int D, bool ROWS>
-__global__ void __launch_bounds__(128) k_attn_dec(AttnDecArgs a, float scale) {
+__global__ void __launch_bounds__(128, 4) k_attn_dec(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v, const __grid_constant__ AttnDecArgs a,
+           float scale) {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-  extern __shared__ __align__(16) uint8_t smem[];
+  extern __shared__ uint8_t smem_raw[];
+  const uint32_t raw = (uint32_t)__cvta_generic_to_shared(smem_raw);
+  uint8_t* smem = smem_raw + (((raw + 1023u) & ~1023u) - raw);
   KernelEnv<ROWS> env;
   env.args = &a;
+  env.map_k = &map_k;
+  env.map_v = &map_v;
   env.land = (float*)(smem + attn_dec_smem_bytes<D>());
   // Before the dependency wait: the first tiles of cached keys and values can be on the way
   // while the projection GEMM still runs.  What makes that sound: every writer of the device-side
@@ -76,25 +80,17 @@ __global__ void __launch_bounds__(128) k_attn_dec(AttnDecArgs a, float scale) {
 
 template <int D, bool ROWS>
 int launch(cg_ctx* c, const AttnDecArgs& args) {
-  constexpr int LD = D + 8;
-  constexpr int KT = D > 128 ? 16 : 32;
   AttnDecArgs a = args;
-  // The push form of the slice merge needs a landing area nothing else uses; it is taken only
-  // where that does not cost a resident CTA per SM (head size 128 would drop from three to two,
-  // which measured 1 % slower per step on the mixture-of-experts shape).
-  const int rep = a.nh / a.nkv;
-  const int blocks = a.splits * ((rep * D + 128 * a.splits - 1) / (128 * a.splits));
-  const size_t land = (size_t)(8 * MAX_REP * 2 + blocks * 128) * 4;
-  auto per_sm = [](size_t bytes) { return (227 * 1024) / (bytes + 1024); };
-  a.push_merge = a.splits > 1 && a.splits <= 8 && land <= attn_dec_landing_bytes() &&
-                 per_sm(attn_dec_smem_bytes<D>() + land) == per_sm(attn_dec_smem_bytes<D>());
-  const size_t smem = attn_dec_smem_bytes<D>() + (a.push_merge ? land : 0);
-  static_assert(attn_dec_smem_bytes<D>() == (size_t)(16 * LD + 8 * KT * LD) * 2 + (size_t)(2 * D + 8 * MAX_REP + 16) * 4, "layout");
+  a.err = c->core->dev_err;
+  CUtensorMap mk, mv;
+  CG_TRY(tc::make_map(c, &mk, a.k_cache, a.cache_rows, D, D, attn_dec_keys(D)));
+  CG_TRY(tc::make_map(c, &mv, a.v_cache, a.cache_rows, D, D, attn_dec_keys(D)));
+  const size_t smem = 1024 + attn_dec_smem_bytes<D>() + (a.splits > 1 ? attn_dec_landing_bytes(a.nh / a.nkv, D, a.splits) : 0);
   static PerDeviceFlag configured_on;
   bool& configured = configured_on.at(c->core->device);
-  if (!configured && attn_dec_smem_bytes<D>() + attn_dec_landing_bytes() > 48 * 1024) {
+  if (!configured) {
     CG_CUDA(c, cudaFuncSetAttribute(k_attn_dec<D, ROWS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    (int)(attn_dec_smem_bytes<D>() + attn_dec_landing_bytes())));
+                                    (int)(1024 + attn_dec_smem_bytes<D>() + attn_dec_landing_bytes(MAX_REP, D, 16))));
     configured = true;
   }
   static PerDeviceFlag wide_on;
@@ -105,28 +101,27 @@ int launch(cg_ctx* c, const AttnDecArgs& args) {
   }
   dim3 grid((unsigned)a.nkv, (unsigned)a.B, (unsigned)a.splits);
   const float scale = a.scale > 0.f ? a.scale : 1.0f / sqrtf((float)D);
-  CG_CUDA(c, launch_kernel(c, k_attn_dec<D, ROWS>, grid, dim3(128), smem, a.splits, a, scale));
+  CG_CUDA(c, launch_kernel(c, k_attn_dec<D, ROWS>, grid, dim3(128), smem, a.splits, mk, mv, a, scale));
   CG_LAUNCHED(c);
   return CG_OK;
 }
 
 }  // namespace
 
-// context slices per (row, kv head): a power of two up to 8 (one portable cluster), about
-// 128 keys per slice at full context
-int attn_dec_splits(int64_t Tmax, int64_t pairs, int d) {
+// Context slices per (row, kv head): a power of two up to 16 (one cluster; above 8 is the non-portable size this GPU
+// supports).  A slice keeps at least 128 keys at full context, one chunk per warp, and all CTAs together
+// stay within two per SM: beyond that a CTA's fixed part (query preparation, merges) costs more than the
+// shorter loop gives, unless a slice would have more than 256 keys; then three to four per SM, as many as fit, will do.
+// Ms per pass with 1 / 2 / 4 / 8 / 16 slices (the rule's choice in brackets):
+//   8 rows x 8 kv heads, 640 keys, d 64 (128 steps of 16 layers)    106.2  102.0 [100.1] 101.9  119.0
+//   32 x 8, 558 keys, d 128 (48 steps of 4 layers)                   66.1 [64.3]   65.2   67.6   74.3
+//   1 x 8, 8200 keys, d 128 (8 steps of 4 layers)                    22.7   20.7   20.2   20.5  [20.1]
+//   4 x 4, 2113 keys, d 256 (64 steps of 4 layers)                   42.0   36.6   33.7   32.5  [32.4]
+//   8 x 4, 1073 keys, d 128, 8 heads each (48 steps of 4 layers)     38.6   37.9   37.5  [37.5]  38.4
+int attn_dec_splits(int64_t Tmax, int64_t pairs) {
+  constexpr int64_t SMS = 148;
   int s = 1;
-  while (s < 8 && (int64_t)s * 128 < Tmax) s *= 2;
-  // (head size 256 once had 32-key tiles: 143 KB per CTA, one CTA per SM, and clusters of 8 such
-  // CTAs did not all fit at once -- 128 CTAs took two waves; with 16-key tiles three CTAs share
-  // an SM)
-  (void)d;
-  // (16 slices -- a cluster size this GPU supports beyond the portable 8 -- were measured for
-  // few (row, kv head) pairs with long contexts and were slower: 2.92 -> 3.15 ms per step on
-  // the 256-wide heads of the Gemma shape.)
-  // many (row, kv head) pairs: fewer, longer slices, so that the fixed cost of a CTA (query
-  // preparation, merges) is spread over more keys; keep about four waves of CTAs
-  while (s > 1 && pairs * s > 4 * 3 * 148 && (int64_t)(s / 2) * 1024 >= Tmax / 4) s /= 2;
+  while (s < 16 && (int64_t)s * 128 < Tmax && (pairs * s * 2 <= 2 * SMS || ((int64_t)s * 256 < Tmax && pairs * s * 2 <= 4 * SMS))) s *= 2;
   return s;
 }
 
@@ -137,6 +132,7 @@ int k_launch_attn_dec(cg_ctx* c, const AttnDecArgs& a) {
   if (a.B > 65535) return fail(c, CG_ERR_UNSUPPORTED, "attention: too many rows");
   if (!a.rows.rows && !a.pos_dev && a.pos0 >= a.Tmax) return fail(c, CG_ERR_SHAPE, "attention: KV cache capacity exceeded");
   if (a.B == 0) return CG_OK;
+  if (a.cache_rows <= 0 || a.cache_rows > 2147483647ll) return fail(c, CG_ERR_UNSUPPORTED, "attention: more cache rows than a tile coordinate holds");
   if (a.rows.rows) {
     switch (a.d) {
       case 64: return launch<64, true>(c, a);

@@ -6,29 +6,43 @@
 // The caller supplies an environment:
 //   tid()            0..127, the thread's index among the 128 threads that run the item
 //   sync_cta()       barrier among those 128 threads
+//   kPush            keys and values come by TMA, and the slices' partial results are PUSHED (st.async, counted by an
+//                    mbarrier) into a landing area (landing(), attn_dec_landing_bytes() of shared memory that nothing
+//                    else uses) of the cluster CTA that finishes them: one way across the cluster, and nobody waits for
+//                    a reader.  The slice's number is the CTA's rank in its cluster, and a CTA runs one item.
+//   map_k, map_v     kPush: tensor maps of the caches as rows of d values, boxes of attn_dec_keys(d) rows of 64
+//                    Without kPush 16-byte copies bring the keys and values, and the finishing CTA reads the partials
+//                    where they lie, behind two barriers:
 //   sync_group()     barrier among the CTAs that hold the slices of one (row, kv head),
 //                    including a barrier among each CTA's own 128 threads
 //   cluster_rank(s)  cluster rank of the CTA that holds slice s
-//   kPush / landing()  kPush: the slices' partial results are PUSHED into a landing area (of
-//                    attn_dec_landing_bytes(), shared memory that nothing else uses) of the CTA that
-//                    finishes them, so one group barrier suffices and nobody waits before leaving;
-//                    otherwise the finishing CTA reads the partials where they lie (two barriers)
 //   kRows            the item is a row of AttnDecArgs::rows: its own slot and position, neighbouring pairs
 //                    rotated, norms over all heads at once, a sink
 //   settle(pos)      called once the first K/V tiles have been requested with a position that may
 //                    be one step old: waits for whatever the caller's inputs depend on and returns
 //                    the position to use (cached keys never change, so an early request is either
 //                    right or is repeated)
+//
+// What bounds an item is its chain of dependent steps and the instructions of its few warps, not its bytes (a few MB per
+// layer over all items).  So gains, angles and the first tiles are asked for before the projection is waited for; one
+// round of loads then brings every vector of the new token, a warp per vector, with its norm in shuffles and its
+// rotation pairs in one lane; the new token takes its place among the keys of a chunk instead of being a chunk of
+// its own; a tile is asked for by one lane; P V is taken as O^T = V^T P^T, whose 8 heads fill the MMA's 8
+// columns (half the instructions and registers of the other form, whose 16 rows they half fill); and nothing divides
+// where a reciprocal does.  From a per-warp timeline: a soft-capped chunk spent 2100 of its 5100 cycles in divisions, a
+// head norm 3000, the merge of 16 unrolled slices up to 2700.  Us that a launch keeps the stream, before / now: 32 rows
+// of 530 keys, 8 kv heads of 128: 40.5 / 26; 4 x 2080, 4 of 256, soft-cap: 21 / 13; 8 x 1050, 4 of 128, 8 heads each:
+// 16.7 / 9; 1 x 350, the same: 13.5 / 8.4; 8 x 576, 8 of 64: 7.0 / 5.4.
 #pragma once
 
 #include "kernels.h"
 #include "mma.cuh"
+#include "tc_common.cuh"
 
 namespace cg {
 
 constexpr int ATTN_MAX_REP = 8;  // query heads per kv head: rows 0..7 of the 16-row MMA tile
 
-__device__ __forceinline__ float attn_tanh_sig(float x) { return 2.f / (1.f + __expf(-2.f * x)) - 1.f; }
 __device__ __forceinline__ float attn_ld_dsmem(uint32_t local_addr, uint32_t rank) {
   uint32_t remote;
   float v;
@@ -36,116 +50,250 @@ __device__ __forceinline__ float attn_ld_dsmem(uint32_t local_addr, uint32_t ran
   asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(remote) : "memory");
   return v;
 }
-
-// shared memory one item needs
-template <int D>
-__host__ __device__ constexpr size_t attn_dec_smem_bytes() {
-  return (size_t)(16 * (D + 8) + 8 * (D > 128 ? 16 : 32) * (D + 8)) * 2 + (size_t)(2 * D + 8 * ATTN_MAX_REP + 16) * 4;
+// W = 1, 2 or 4 neighbouring floats through L2 (in the resident kernel another CTA wrote them in the same launch)
+template <int W>
+__device__ __forceinline__ void attn_ldcg(const float* p, float* v) {
+  if constexpr (W == 1) {
+    v[0] = __ldcg(p);
+  } else if constexpr (W == 2) {
+    const float2 x = __ldcg((const float2*)p);
+    v[0] = x.x; v[1] = x.y;
+  } else {
+    const float4 x = __ldcg((const float4*)p);
+    v[0] = x.x; v[1] = x.y; v[2] = x.z; v[3] = x.w;
+  }
 }
 
-// landing area of the push form: {max, sum} per source slice and head, then per source slice the
-// output values the CTA finishes (at most 8 slices; up to rep * D / 128 + 8 blocks of 128 values)
-__host__ __device__ constexpr size_t attn_dec_landing_bytes() { return (size_t)(8 * ATTN_MAX_REP * 2 + (16 + 8) * 128) * 4; }
+// Keys per warp tile: 32, or 16 for head size 256 so that a CTA's tiles fit a third of an SM's shared memory.
+__host__ __device__ constexpr int attn_dec_keys(int D) { return D > 128 ? 16 : 32; }
 
-// KT = keys per warp tile: 32, or 16 for head size 256 so that a CTA's tiles fit a third of an
-// SM's shared memory.
+// shared memory one item needs (from a multiple of 1024 bytes): 8 query rows, a key and a value tile per warp, the new
+// key and value, reductions and the tiles' barriers
+template <int D>
+__host__ __device__ constexpr size_t attn_dec_smem_bytes() {
+  return (size_t)(8 * attn_dec_keys(D) * D + 8 * (D + 8) + 2 * D) * 2 + (size_t)(8 * ATTN_MAX_REP + 4) * 4 + 64;
+}
+
+// landing area of the push form: a barrier, {max, sum} per source slice and head, and per source slice its share of
+// the output values that the CTA finishes
+__host__ __device__ constexpr size_t attn_dec_landing_bytes(int rep, int d, int splits) {
+  return 16 + (size_t)splits * ATTN_MAX_REP * 8 + (size_t)rep * d * 4;
+}
+
 template <int D, class Env>
 __device__ __forceinline__ void attn_dec_item(const AttnDecArgs& a, float scale, int kvh, int64_t b, int split, int64_t pos_early,
                                               uint8_t* smem, Env& env) {
-  constexpr int KT = D > 128 ? 16 : 32;
+  constexpr int KT = attn_dec_keys(D);
   constexpr int MAX_REP = ATTN_MAX_REP;
-  constexpr int LD = D + 8;     // padded rows: conflict-free ldmatrix
+  constexpr int LD = D + 8;     // padded rows of the queries: conflict-free ldmatrix
+  constexpr int BOX = KT * 128; // bytes of a box of a tile: KT rows of 64 values
   constexpr int CH = D / 8;     // 16-byte chunks per row
-  constexpr int NT = D / 8;     // output n-tiles
-  __nv_bfloat16* qt = (__nv_bfloat16*)smem;              // [16][LD] query heads (rows >= rep are zero)
-  __nv_bfloat16* kt = qt + 16 * LD;                      // [4 warps][KT][LD] key tiles
-  __nv_bfloat16* vt = kt + 4 * KT * LD;                  // [4 warps][KT][LD] value tiles
-  float* fl = (float*)(vt + 4 * KT * LD);
-  float* knew = fl;                                      // [D] the new key (bf16-rounded)
-  float* vnew = knew + D;                                // [D]
-  float* red_m = vnew + D;                               // [4][MAX_REP]
+  constexpr int W = D / 64;     // rotation pairs per lane
+  constexpr int NV = 3;         // vectors of the new token per warp: at most 8 query heads, a key and a value on 4 warps
+  constexpr int LDO = D + 4;    // row stride of the warps' outputs: conflict-free stores of O^T fragments
+  // Tiles are D / 64 boxes of KT rows of 64 values; 16-byte chunk c of row r of a box lies at place c ^ (r & 7), as TMA's
+  // 128-byte swizzle has it (the tiles begin on a multiple of 1024 bytes): conflict-free ldmatrix
+  uint8_t* kt = smem;                                    // [4 warps] key tiles
+  uint8_t* vt = kt + 4 * KT * D * 2;                     // [4 warps] value tiles
+  __nv_bfloat16* qt = (__nv_bfloat16*)(vt + 4 * KT * D * 2);  // [8][LD] query heads (rows >= rep are zero)
+  __nv_bfloat16* knew = qt + 8 * LD;                     // [D] the new key
+  __nv_bfloat16* vnew = knew + D;                        // [D]
+  float* red_m = (float*)(vnew + D);                     // [4][MAX_REP]
   float* red_l = red_m + 4 * MAX_REP;                    // [4][MAX_REP]
-  float* hsq = red_l + 4 * MAX_REP;                      // [MAX_REP + 1] per-head rms (norm), padded to 16
-  float* red_o = (float*)kt;                             // [4][MAX_REP][D] f32, reuses the tiles after the loop
+  volatile int* cta_abort = (volatile int*)(red_l + 4 * MAX_REP);
+  float* red_o = (float*)kt;                             // [4][MAX_REP][LDO] f32, over the tiles after the loop
 
   const int tid = env.tid(), warp = tid >> 5, lane = tid & 31;
+  // this warp's barriers: its keys have arrived, its values have arrived
+  const uint32_t bar_k = (uint32_t)__cvta_generic_to_shared(red_l + 4 * MAX_REP + 4) + (uint32_t)warp * 16u, bar_v = bar_k + 8;
+  if constexpr (Env::kPush) {
+    if (lane == 0) {
+      tc::mbar_init(bar_k, 1);
+      tc::mbar_init(bar_v, 1);
+      asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    }
+    if (tid == 0) *cta_abort = 0;
+  }
   const int rep = a.nh / a.nkv;
-  const int half = D / 2;
-  // pos: position of the new token = number of cached keys.  The projected row is read with
-  // L2 loads: in the resident kernel another CTA wrote it earlier in the same launch.
+  const int S = a.splits;
+  // A CTA finishes `wide` neighbouring columns of every head.  Landing area of the push form: slice s's {max, sum} of
+  // head r at land_ml[s][r], its values of those outputs at land_o[s][r].
+  const int lg = __ffs(S) - 1, wide = D >> lg;  // (the slices are a power of two in number)
+  const int per = rep * wide, lgw = 31 - __clz(wide);
+  uint32_t land_bar = 0, land_ml = 0, land_o = 0;
+  if constexpr (Env::kPush) {
+    land_bar = (uint32_t)__cvta_generic_to_shared(env.landing());
+    land_ml = land_bar + 16;
+    land_o = land_ml + (uint32_t)(S * MAX_REP * 8);
+    if (S > 1) {
+      if (tid == 0) {
+        tc::mbar_init(land_bar, 1);
+        tc::mbar_expect_tx(land_bar, (uint32_t)(rep * D * 4 + S * rep * 8));
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+      }
+      // the peers' barriers exist once they have arrived here; waited for just before the pushes
+      __syncwarp();
+      asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+    }
+  }
+  // pos: position of the new token = number of cached keys
   int64_t place = b;
   if constexpr (Env::kRows) place = a.rows.slot[b];
   __nv_bfloat16* kbase = a.k_cache + ((place * a.nkv + kvh) * a.Tmax) * (int64_t)D;
   __nv_bfloat16* vbase = a.v_cache + ((place * a.nkv + kvh) * a.Tmax) * (int64_t)D;
 
-  // The visible cached keys are the kf kept first ones and [lo, pos); [t0, t1) is this CTA's slice of
-  // their sequence.
-  int64_t pos = pos_early, t0 = 0, t1 = 0, lo = 0, kf = 0;
+  // The visible keys are the kf kept first ones, [lo, pos) and the new one.  They are numbered in that order, with the
+  // numbers from kf to the next multiple of KT left out; the new one is number `fresh`; [t0, t1) is this CTA's slice.
+  int64_t pos = pos_early;
+  int t0 = 0, t1 = 0, kf = 0, kfp = 0, fresh = 0;
+  int64_t skip = 0;  // from a key's number to its place in the cache, behind the kept ones
   auto plan = [&]() {
-    lo = a.window > 0 ? max((int64_t)0, pos - a.window + 1) : 0;
-    if constexpr (Env::kRows) kf = min(a.keep_first, lo);
-    const int64_t span = kf + pos - lo;
-    int64_t per = (span + a.splits - 1) / a.splits;
-    per = (per + KT - 1) / KT * KT;
-    t0 = split * per;
-    t1 = min(span, t0 + per);
+    const int64_t lo = a.window > 0 ? max((int64_t)0, pos - a.window + 1) : 0;
+    if constexpr (Env::kRows) {
+      kf = (int)min(a.keep_first, lo);
+      kfp = (kf + KT - 1) / KT * KT;
+    }
+    skip = lo - kfp;
+    fresh = (int)(pos - skip);
+    int n = (fresh + S) >> lg;
+    n = (n + KT - 1) / KT * KT;
+    t0 = split * n;
+    t1 = min(fresh + 1, t0 + n);
   };
   plan();
 
-  __nv_bfloat16* kw = kt + (size_t)warp * KT * LD;
-  __nv_bfloat16* vw = vt + (size_t)warp * KT * LD;
+  uint8_t* kw = kt + warp * (KT * D * 2);
+  uint8_t* vw = vt + warp * (KT * D * 2);
   const uint32_t kw_u = (uint32_t)__cvta_generic_to_shared(kw);
   const uint32_t vw_u = (uint32_t)__cvta_generic_to_shared(vw);
   const uint32_t qt_u = (uint32_t)__cvta_generic_to_shared(qt);
 
-  // Request the first chunk of this warp now: it does not depend on q.  Keys and values are groups of their own:
-  // the next keys are asked for as soon as the scores have been taken, the next values behind the
-  // product, so that of a warp's two tiles one is always on its way (with the new token's chunk moved off the warp
-  // that has most to do, a step of the Llama-3.2-1B shape, batch 8, 753 -> 747 us; of four layers of the
-  // Gemma-2-2B shape at 2048 keys 491 -> 482 us).
-  auto request = [&](int64_t c0, uint32_t tile, const __nv_bfloat16* from) {
-    // KT rows x CH chunks, 8 (or more) lanes per row: fully coalesced 16-byte copies
-    if (c0 < t1)
-      for (int i = lane; i < KT * CH; i += 32) {
-        const int r = i / CH, ch = i - r * CH;
-        const int64_t key = c0 + r;
-        const bool ok = key < t1;
-        int64_t kc = ok ? key : t0;
-        if (kc >= kf) kc += lo - kf;
-        cp_async16(tile + (uint32_t)(r * LD + ch * 8) * 2u, from + kc * (int64_t)D + ch * 8, ok ? 16 : 0);
+  // Request the first chunk of this warp now: it does not depend on q.  One lane asks for a tile by D / 64 TMA loads of
+  // whole boxes (16-byte copies cost a third of the kernel's instructions, which a warp has little to hide behind; bulk
+  // copies of single rows are slower than those where rows are 128 bytes).  Keys and values have barriers of their
+  // own: the next keys are asked for as soon as the scores have been taken, the next values behind the
+  // product, so that of a warp's two tiles one is always on its way.
+  auto request = [&](int c0, bool keys) {
+    if constexpr (Env::kPush) {
+      if (c0 < t1 && lane == 0) {
+        const uint32_t bar = keys ? bar_k : bar_v, tile = keys ? kw_u : vw_u;
+        const int at = (int)((place * a.nkv + kvh) * a.Tmax + (c0 < kfp ? c0 : c0 + skip));
+        tc::mbar_expect_tx(bar, KT * D * 2);
+#pragma unroll
+        for (int x = 0; x < D / 64; ++x) tc::tma_load_2d(tile + x * BOX, keys ? env.map_k : env.map_v, x * 64, at, bar);
       }
-    cp_async_commit();
+    } else {
+      if (c0 < t1) {
+        const uint32_t tile = keys ? kw_u : vw_u;
+        const __nv_bfloat16* from = keys ? kbase : vbase;
+#pragma unroll 4
+        for (int i = lane; i < KT * CH; i += 32) {
+          const int r = i / CH, ch = i % CH;
+          const int64_t key = c0 + r + skip;
+          const bool ok = key < pos;
+          cp_async16(tile + (uint32_t)((ch >> 3) * BOX + r * 128 + (((ch & 7) ^ (r & 7)) << 4)), from + (ok ? key : 0) * D + ch * 8, ok ? 16 : 0);
+        }
+      }
+      cp_async_commit();
+    }
   };
-  int64_t c0 = t0 + warp * KT;
-  request(c0, kw_u, kbase);
-  request(c0, vw_u, vbase);
+  uint32_t phase = 0;  // of both barriers
+  int c0 = t0 + warp * KT;
+  request(c0, true);
+  request(c0, false);
+
+  // Warp w has the new token's vectors w, w + 4, w + 8: the query heads, the key, the value.  A lane holds both
+  // components of W rotation pairs.  Pairs are (j, j + D / 2) with j = lane * W + i, or neighbours with j = lane + 32 i.
+  const int heads = a.nh + 2 * a.nkv;
+  auto pair = [&](int i) { return Env::kRows ? lane + 32 * i : lane * W + i; };
+  auto head_of = [&](int id) { return id < rep ? kvh * rep + id : id == rep ? a.nh + kvh : a.nh + a.nkv + kvh; };
+  auto is_new = [&](int v) { return warp + 4 * v < rep + 2; };
+  // what does not depend on the projection: gains and angles
+  float g1[NV][W], g2[NV][W], cs[W], sn[W], temp = 1.f;
+#pragma unroll
+  for (int v = 0; v < NV; ++v) {
+    const int id = warp + 4 * v;
+#pragma unroll
+    for (int i = 0; i < W; ++i) g1[v][i] = g2[v][i] = 1.f;
+    if (a.q_gamma && id <= rep) {
+      if constexpr (Env::kRows) {
+        const float* g = id < rep ? a.q_gamma + (int64_t)(kvh * rep + id) * D : a.k_gamma + (int64_t)kvh * D;
+#pragma unroll
+        for (int i = 0; i < W; ++i) {
+          const float2 x = *((const float2*)g + pair(i));
+          g1[v][i] = x.x; g2[v][i] = x.y;
+        }
+      } else {
+        const float* g = id < rep ? a.q_gamma : a.k_gamma;
+        const float plus = a.norm_plus_one ? 1.f : 0.f;
+#pragma unroll
+        for (int i = 0; i < W; ++i) {
+          g1[v][i] = plus + g[pair(i)];
+          g2[v][i] = plus + g[pair(i) + D / 2];
+        }
+      }
+    }
+  }
+  auto angles = [&]() {
+    const int n = Env::kRows ? a.rot_dims / 2 : D / 2;
+#pragma unroll
+    for (int i = 0; i < W; ++i) {
+      const int j = pair(i);
+      cs[i] = 1.f; sn[i] = 0.f;
+      if (j < n) { cs[i] = a.cos_t[pos * n + j]; sn[i] = a.sin_t[pos * n + j]; }
+    }
+    if constexpr (Env::kRows)
+      if (a.q_temp) temp = a.q_temp[pos];
+  };
+  angles();
+  for (int i = tid; i < (8 - rep) * CH; i += 128) *(uint4*)(qt + (rep + i / CH) * LD + i % CH * 8) = make_uint4(0u, 0u, 0u, 0u);
   {
     const int64_t pos_now = env.settle(pos);
     if (pos_now != pos) {  // the early position was stale: let the copies land, then ask again
-      cp_async_wait_group<0>();
+      if (c0 < t1) {
+        tc::mbar_drain(bar_k, phase, a.err);
+        tc::mbar_drain(bar_v, phase, a.err);
+        phase ^= 1u;
+      }
       __syncwarp();
       pos = pos_now;
       plan();
       c0 = t0 + warp * KT;
-      request(c0, kw_u, kbase);
-      request(c0, vw_u, vbase);
+      request(c0, true);
+      request(c0, false);
+      angles();
     }
   }
 
   // ---- 1. q, k, v of the new token ----
-  const int heads = a.nh + 2 * a.nkv;
   int64_t ld_row = (int64_t)heads * D, ld_out = (int64_t)a.nh * D;
   if constexpr (Env::kRows) {
     if (a.ld_qkv) ld_row = a.ld_qkv;
     if (a.ld_out) ld_out = a.ld_out;
   }
   const float* row = a.qkv + b * ld_row;
-  const float* qsrc = row + (int64_t)kvh * rep * D;
-  const float* ksrc = row + ((int64_t)a.nh + kvh) * D;
-  const float* vsrc = row + ((int64_t)a.nh + a.nkv + kvh) * D;
-  if constexpr (Env::kRows) {
-    if (a.q_gamma) {
-      // norms over all query heads and over all key heads: hsq[0], hsq[1] receive the factors
+  {
+    float x1[NV][W], x2[NV][W];
+#pragma unroll
+    for (int v = 0; v < NV; ++v) {
+#pragma unroll
+      for (int i = 0; i < W; ++i) x1[v][i] = x2[v][i] = 0.f;
+      if (!is_new(v)) continue;
+      const float* src = row + (int64_t)head_of(warp + 4 * v) * D;
+      if constexpr (Env::kRows) {
+#pragma unroll
+        for (int i = 0; i < W; ++i) {
+          const float2 x = __ldcg((const float2*)src + pair(i));
+          x1[v][i] = x.x; x2[v][i] = x.y;
+        }
+      } else {
+        attn_ldcg<W>(src + lane * W, x1[v]);
+        attn_ldcg<W>(src + lane * W + D / 2, x2[v]);
+      }
+    }
+    if (Env::kRows && a.q_gamma) {
+      // norms over all query heads and over all key heads
       float ss[2] = {0.f, 0.f};
 #pragma unroll
       for (int part = 0; part < 2; ++part) {
@@ -156,214 +304,164 @@ __device__ __forceinline__ void attn_dec_item(const AttnDecArgs& a, float scale,
           const float4 v = __ldcg(src + i);
           ss[part] += v.x * v.x + v.y * v.y + v.z * v.z + v.w * v.w;
         }
+      }
 #pragma unroll
-        for (int o = 16; o; o >>= 1) ss[part] += __shfl_xor_sync(0xffffffffu, ss[part], o);
-        if (lane == 0) red_m[part * 4 + warp] = ss[part];
+      for (int o = 16; o; o >>= 1) {
+        ss[0] += __shfl_xor_sync(0xffffffffu, ss[0], o);
+        ss[1] += __shfl_xor_sync(0xffffffffu, ss[1], o);
       }
+      if (lane == 0) { red_m[warp] = ss[0]; red_m[4 + warp] = ss[1]; }
       env.sync_cta();
-      if (tid < 2) {
-        const float* r = red_m + tid * 4;
-        hsq[tid] = 1.f / sqrtf(((r[0] + r[1]) + (r[2] + r[3])) / (float)((tid ? a.nkv : a.nh) * a.norm_dim) + a.norm_eps);
-      }
-      env.sync_cta();
-    } else if (a.head_norm) {
-      // norms per head: hsq[h] of the query heads, hsq[rep] of the key head
-      for (int h = warp; h <= rep; h += 4) {
-        const float* src = h < rep ? qsrc + h * D : ksrc;
-        float ss = 0.f;
-        for (int e = lane; e < D; e += 32) { const float v = __ldcg(src + e); ss += v * v; }
 #pragma unroll
-        for (int o = 16; o; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
-        if (lane == 0) hsq[h] = 1.f / sqrtf(ss / (float)a.norm_dim + a.norm_eps);
+      for (int v = 0; v < NV; ++v) {
+        const int id = warp + 4 * v;
+        if (id > rep) continue;
+        const float* r = red_m + (id < rep ? 0 : 4);
+        const float f = 1.f / sqrtf(((r[0] + r[1]) + (r[2] + r[3])) / (float)((id < rep ? a.nh : a.nkv) * a.norm_dim) + a.norm_eps);
+#pragma unroll
+        for (int i = 0; i < W; ++i) { x1[v][i] *= f * g1[v][i]; x2[v][i] *= f * g2[v][i]; }
       }
-      env.sync_cta();
-    }
-    // neighbouring components (2 j, 2 j + 1) of the first rot_dims turn together
-    const int rh = a.rot_dims / 2;
-    const float temp = a.q_temp ? a.q_temp[pos] : 1.f;
-    const float* ct = a.cos_t + pos * rh;
-    const float* st = a.sin_t + pos * rh;
-    for (int i = tid; i < 16 * half; i += 128) {
-      const int h = i / half, j = i - h * half;
-      float x1 = 0.f, x2 = 0.f;
-      if (h < rep) {
-        const float2 x = __ldcg((const float2*)(qsrc + h * D) + j);
-        x1 = x.x; x2 = x.y;
-        if (a.q_gamma) {
-          const float2 g = *((const float2*)(a.q_gamma + (kvh * rep + h) * D) + j);
-          x1 *= hsq[0] * g.x; x2 *= hsq[0] * g.y;
-        } else if (a.head_norm) {
-          x1 *= hsq[h]; x2 *= hsq[h];
+    } else if (Env::kRows ? a.head_norm != 0 : a.q_gamma != nullptr) {
+      // norms per head
+      float ss[NV];
+#pragma unroll
+      for (int v = 0; v < NV; ++v) {
+        ss[v] = 0.f;
+#pragma unroll
+        for (int i = 0; i < W; ++i) ss[v] += x1[v][i] * x1[v][i] + x2[v][i] * x2[v][i];
+      }
+#pragma unroll
+      for (int o = 16; o; o >>= 1)
+#pragma unroll
+        for (int v = 0; v < NV; ++v) ss[v] += __shfl_xor_sync(0xffffffffu, ss[v], o);
+#pragma unroll
+      for (int v = 0; v < NV; ++v) {
+        if (warp + 4 * v > rep) continue;
+        if constexpr (Env::kRows) {
+          const float f = 1.f / sqrtf(ss[v] / (float)a.norm_dim + a.norm_eps);
+#pragma unroll
+          for (int i = 0; i < W; ++i) { x1[v][i] *= f; x2[v][i] *= f; }
+        } else {
+          const float f = 1.f / sqrtf(ss[v] * (1.f / D) + a.norm_eps);
+#pragma unroll
+          for (int i = 0; i < W; ++i) { x1[v][i] *= f * g1[v][i]; x2[v][i] *= f * g2[v][i]; }
         }
-        if (j < rh) {
-          const float cs = ct[j], sn = st[j], t = x1;
-          x1 = cs * t - sn * x2;
-          x2 = cs * x2 + sn * t;
-        }
-        x1 *= temp; x2 *= temp;
-      }
-      *(__nv_bfloat162*)(qt + h * LD + 2 * j) = __floats2bfloat162_rn(x1, x2);
-    }
-    for (int j = tid; j < half; j += 128) {
-      const float2 x = __ldcg((const float2*)ksrc + j), v = __ldcg((const float2*)vsrc + j);
-      float x1 = x.x, x2 = x.y;
-      if (a.q_gamma) {
-        const float2 g = *((const float2*)(a.k_gamma + kvh * D) + j);
-        x1 *= hsq[1] * g.x; x2 *= hsq[1] * g.y;
-      } else if (a.head_norm) {
-        x1 *= hsq[rep]; x2 *= hsq[rep];
-      }
-      if (j < rh) {
-        const float cs = ct[j], sn = st[j], t = x1;
-        x1 = cs * t - sn * x2;
-        x2 = cs * x2 + sn * t;
-      }
-      const __nv_bfloat162 kk = __floats2bfloat162_rn(x1, x2), vv = __floats2bfloat162_rn(v.x, v.y);
-      knew[2 * j] = __low2float(kk); knew[2 * j + 1] = __high2float(kk);
-      vnew[2 * j] = __low2float(vv); vnew[2 * j + 1] = __high2float(vv);
-      if (split == 0) {  // append to the cache for the following steps
-        *(__nv_bfloat162*)(kbase + pos * D + 2 * j) = kk;
-        *(__nv_bfloat162*)(vbase + pos * D + 2 * j) = vv;
       }
     }
-    env.sync_cta();
-  } else {
-  if (a.q_gamma) {
-    // per-head RMSNorm over d for the rep query heads and the key head
-    for (int h = warp; h <= rep; h += 4) {
-      const float* src = h < rep ? qsrc + h * D : ksrc;
-      float ss = 0.f;
-      for (int e = lane; e < D; e += 32) { const float v = __ldcg(src + e); ss += v * v; }
 #pragma unroll
-      for (int o = 16; o; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
-      if (lane == 0) hsq[h] = sqrtf(ss / (float)D + a.norm_eps);
-    }
-    env.sync_cta();
-  }
-  for (int i = tid; i < 16 * half; i += 128) {
-    const int h = i / half, j = i - h * half;
-    if (h < rep) {
-      float x1 = __ldcg(qsrc + h * D + j), x2 = __ldcg(qsrc + h * D + j + half);
-      if (a.q_gamma) {
-        const float g1 = a.norm_plus_one ? 1.f + a.q_gamma[j] : a.q_gamma[j];
-        const float g2 = a.norm_plus_one ? 1.f + a.q_gamma[j + half] : a.q_gamma[j + half];
-        x1 = x1 / hsq[h] * g1;
-        x2 = x2 / hsq[h] * g2;
+    for (int v = 0; v < NV; ++v) {
+      if (!is_new(v)) continue;
+      const int id = warp + 4 * v;
+      if (id <= rep) {
+        const float t = id < rep ? temp : 1.f;
+#pragma unroll
+        for (int i = 0; i < W; ++i) {
+          const float u = x1[v][i], w = x2[v][i];
+          if (!Env::kRows || pair(i) < a.rot_dims / 2) {
+            x1[v][i] = cs[i] * u - sn[i] * w;
+            x2[v][i] = cs[i] * w + sn[i] * u;
+          }
+          x1[v][i] *= t; x2[v][i] *= t;
+        }
       }
-      const float cs = a.cos_t[pos * half + j], sn = a.sin_t[pos * half + j];
-      qt[h * LD + j] = __float2bfloat16_rn(cs * x1 - sn * x2);
-      qt[h * LD + j + half] = __float2bfloat16_rn(cs * x2 + sn * x1);
-    } else {
-      qt[h * LD + j] = __float2bfloat16_rn(0.f);
-      qt[h * LD + j + half] = __float2bfloat16_rn(0.f);
-    }
-  }
-  for (int j = tid; j < half; j += 128) {
-    float x1 = __ldcg(ksrc + j), x2 = __ldcg(ksrc + j + half);
-    if (a.q_gamma) {
-      const float g1 = a.norm_plus_one ? 1.f + a.k_gamma[j] : a.k_gamma[j];
-      const float g2 = a.norm_plus_one ? 1.f + a.k_gamma[j + half] : a.k_gamma[j + half];
-      x1 = x1 / hsq[rep] * g1;
-      x2 = x2 / hsq[rep] * g2;
-    }
-    const float cs = a.cos_t[pos * half + j], sn = a.sin_t[pos * half + j];
-    const __nv_bfloat16 k1 = __float2bfloat16_rn(cs * x1 - sn * x2), k2 = __float2bfloat16_rn(cs * x2 + sn * x1);
-    const __nv_bfloat16 v1 = __float2bfloat16_rn(__ldcg(vsrc + j)), v2 = __float2bfloat16_rn(__ldcg(vsrc + j + half));
-    knew[j] = __bfloat162float(k1);
-    knew[j + half] = __bfloat162float(k2);
-    vnew[j] = __bfloat162float(v1);
-    vnew[j + half] = __bfloat162float(v2);
-    if (split == 0) {  // append to the cache for the following steps
-      kbase[pos * D + j] = k1;
-      kbase[pos * D + j + half] = k2;
-      vbase[pos * D + j] = v1;
-      vbase[pos * D + j + half] = v2;
+      auto put = [&](__nv_bfloat16* to) {
+#pragma unroll
+        for (int i = 0; i < W; ++i) {
+          const int j = pair(i);
+          if constexpr (Env::kRows) {
+            *(__nv_bfloat162*)(to + 2 * j) = __floats2bfloat162_rn(x1[v][i], x2[v][i]);
+          } else {
+            to[j] = __float2bfloat16_rn(x1[v][i]);
+            to[j + D / 2] = __float2bfloat16_rn(x2[v][i]);
+          }
+        }
+      };
+      put(id < rep ? qt + id * LD : id == rep ? knew : vnew);
+      if (id >= rep && split == 0) put((id == rep ? kbase : vbase) + pos * D);  // append to the cache for the following steps
     }
   }
   env.sync_cta();
-  }
 
-  // ---- 2. this warp's chunks of 32 keys: S = Q K^T, online softmax, O += P V ----
-  // A thread owns head r = lane / 4 (rows 8..15 of the MMA tile are padding) and, per 8-key
-  // or 8-column tile, the two columns 2 * (lane % 4) + {0, 1}.
+  // ---- 2. this warp's chunks of KT keys: S = Q K^T, online softmax, O^T += V^T P^T ----
+  // In S a thread owns head hr = lane / 4 and, per 8-key tile, the two keys cq + {0, 1}; in O^T the two heads
+  // cq + {0, 1} and, per 16 output columns, columns lane / 4 and 8 + lane / 4.
   const int hr = lane >> 2, cq = (lane & 3) * 2;
   const float* bias = nullptr;
   if constexpr (Env::kRows)
     if (a.bias && hr < rep) bias = a.bias + (int64_t)(kvh * rep + hr) * a.ld_bias;
   float m = -INFINITY, l = 0.f;
-  float o[NT][4];
+  float o[D / 16][4];
 #pragma unroll
-  for (int j = 0; j < NT; ++j) o[j][0] = o[j][1] = o[j][2] = o[j][3] = 0.f;
-
-  // The last slice's last warp also owns the new token: one more chunk whose only live key is row 0.  Slices and
-  // warps are filled in order, so this is the warp that has the fewest cached keys, often none.
-  const bool owns_new = split == a.splits - 1 && warp == 3;
-  bool do_new = false;
-  while (true) {
-    int64_t limit;  // live keys of this chunk are [c0, limit)
-    if (c0 < t1) {
-      limit = t1;
-      cp_async_wait_group<1>();  // the keys
+  for (int j = 0; j < D / 16; ++j) o[j][0] = o[j][1] = o[j][2] = o[j][3] = 0.f;
+  // c tanh(x / c) = c (2 / (1 + 2^(x cap_unit / scale)) - 1)
+  const float cap_unit = a.softcap > 0.f ? -2.f * 1.44269504088896340736f * scale / a.softcap : 0.f;
+  auto chunk_of = [&](uint8_t* tile, int r, int ch) {
+    return (uint4*)(tile + (ch >> 3) * BOX + r * 128 + (((ch & 7) ^ (r & 7)) << 4));
+  };
+  // the new token's row of a tile, once the copies have landed
+  auto insert = [&](uint8_t* tile, const __nv_bfloat16* from) {
+    const int r = fresh - c0;
+    if (r >= 0 && r < KT) {
+      for (int i = lane; i < CH; i += 32) *chunk_of(tile, r, i) = *(const uint4*)(from + i * 8);
       __syncwarp();
-    } else if (owns_new && !do_new) {
-      do_new = true;
-      cp_async_wait_group<0>();
-      // build the one-row chunk in the tiles
-      for (int e = lane; e < D; e += 32) {
-        kw[e] = __float2bfloat16_rn(knew[e]);
-        vw[e] = __float2bfloat16_rn(vnew[e]);
-      }
-      for (int i = lane; i < (KT - 1) * CH; i += 32) {
-        const int r = 1 + i / CH, ch = i % CH;
-        *(uint4*)(vw + r * LD + ch * 8) = make_uint4(0u, 0u, 0u, 0u);  // p = 0 times NaN garbage must not happen
-        *(uint4*)(kw + r * LD + ch * 8) = make_uint4(0u, 0u, 0u, 0u);
-      }
-      __syncwarp();
-      limit = 1;  // in units relative to a chunk start of 0
-    } else {
+    }
+  };
+  // ldmatrix addresses of this lane: rows (lane & 7) + 8 (lane / 16) of a tile, chunks 2 x + (lane / 8) % 2 of a box
+  const uint32_t qa = qt_u + (uint32_t)((lane & 7) * LD + (lane >> 3) * 8) * 2u;
+  uint32_t xa[4];
+#pragma unroll
+  for (int x = 0; x < 4; ++x)
+    xa[x] = kw_u + (uint32_t)(((lane & 7) + 8 * (lane >> 4)) * 128 + (((2 * x + ((lane >> 3) & 1)) ^ (lane & 7)) << 4));
+  const uint32_t to_v = vw_u - kw_u;
+  // A warp leaves the loop as a whole where a wait gave up, behind the copies that are on their way to it.
+  auto landed = [&](uint32_t bar) {
+    if constexpr (Env::kPush) return __all_sync(0xffffffffu, tc::mbar_wait(bar, phase, cta_abort, a.err)) != 0;
+    cp_async_wait_group<1>();
+    __syncwarp();
+    return true;
+  };
+  for (; c0 < t1; c0 += 4 * KT) {
+    const int live = (c0 < kfp ? kf : t1) - c0;  // keys of this chunk, at least one
+    if (!landed(bar_k)) {
+      tc::mbar_drain(bar_k, phase, a.err);
+      tc::mbar_drain(bar_v, phase, a.err);
       break;
     }
-    const int64_t cbase = do_new ? 0 : c0;
-
-    float s[KT / 8][4];
+    insert(kw, knew);
+    // (two sums per key tile: a chain of half the length)
+    float s[KT / 8][4], s2[KT / 8][4];
 #pragma unroll
-    for (int j = 0; j < KT / 8; ++j) s[j][0] = s[j][1] = s[j][2] = s[j][3] = 0.f;
+    for (int j = 0; j < KT / 8; ++j) s[j][0] = s[j][1] = s[j][2] = s[j][3] = s2[j][0] = s2[j][1] = s2[j][2] = s2[j][3] = 0.f;
 #pragma unroll
-    for (int kk = 0; kk < D / 16; ++kk) {
-      uint32_t a0, a1, a2, a3;
-      {
-        const int r = (lane & 7) + 8 * ((lane >> 3) & 1);
-        const int col = kk * 16 + 8 * (lane >> 4);
-        ldsm_x4(qt_u + (uint32_t)(r * LD + col) * 2u, a0, a1, a2, a3);
-      }
+    for (int kk = 0; kk < D / 16; kk += 2) {
+      uint32_t q[4];
+      ldsm_x4(qa + (uint32_t)(kk * 32), q[0], q[1], q[2], q[3]);
 #pragma unroll
       for (int j = 0; j < KT / 8; j += 2) {
         uint32_t b0, b1, b2, b3;
-        const int key = j * 8 + (lane & 7) + 8 * (lane >> 4);
-        const int col = kk * 16 + 8 * ((lane >> 3) & 1);
-        ldsm_x4(kw_u + (uint32_t)(key * LD + col) * 2u, b0, b1, b2, b3);
-        mma_bf16(s[j], a0, a1, a2, a3, b0, b1);
-        mma_bf16(s[j + 1], a0, a1, a2, a3, b2, b3);
+        ldsm_x4(xa[kk & 3] + (uint32_t)(j * 8 * 128 + kk / 4 * BOX), b0, b1, b2, b3);
+        mma_bf16(s[j], q[0], 0u, q[1], 0u, b0, b1);
+        mma_bf16(s[j + 1], q[0], 0u, q[1], 0u, b2, b3);
+        ldsm_x4(xa[(kk + 1) & 3] + (uint32_t)(j * 8 * 128 + kk / 4 * BOX), b0, b1, b2, b3);
+        mma_bf16(s2[j], q[2], 0u, q[3], 0u, b0, b1);
+        mma_bf16(s2[j + 1], q[2], 0u, q[3], 0u, b2, b3);
       }
     }
-    if (!do_new) {
-      __syncwarp();
-      request(c0 + 4 * KT, kw_u, kbase);
-    }
+    __syncwarp();
+    request(c0 + 4 * KT, true);
     // scale, soft-cap, mask; this head's maximum over the chunk
     float mx = -INFINITY;
 #pragma unroll
     for (int j = 0; j < KT / 8; ++j) {
 #pragma unroll
       for (int e = 0; e < 2; ++e) {
-        float v = s[j][e] * scale;
-        if (a.softcap > 0.f) v = a.softcap * attn_tanh_sig(v / a.softcap);
-        const bool keep = cbase + j * 8 + cq + e < limit;
+        float v = s[j][e] + s2[j][e];
+        v = a.softcap > 0.f ? a.softcap * fmaf(2.f, rcp_newton(1.f + fast_exp2(v * cap_unit)), -1.f) : v * scale;
+        const int key = c0 + j * 8 + cq + e;
+        const bool keep = key - c0 < live;
         if constexpr (Env::kRows)
-          if (bias && keep && !do_new) {   // (at the new token itself the distance is 0, and so is what is taken off)
-            const int64_t i = cbase + j * 8 + cq + e;
-            v -= bias[pos - (i < kf ? i : i - kf + lo)];
-          }
+          if (bias && keep && key < fresh)   // (at the new token itself the distance is 0, and so is what is taken off)
+            v -= bias[pos - (key < kfp ? key : key + skip)];
         v = keep ? v : -INFINITY;
         s[j][e] = v;
         mx = fmaxf(mx, v);
@@ -386,52 +484,67 @@ __device__ __forceinline__ void attn_dec_item(const AttnDecArgs& a, float scale,
     sum += __shfl_xor_sync(0xffffffffu, sum, 1);
     sum += __shfl_xor_sync(0xffffffffu, sum, 2);
     l = l * corr + sum;
+    const float m_old = m;
     m = mnew;
+    if (__any_sync(0xffffffffu, corr != 1.f && m_old != -INFINITY)) {  // (a factor of one changes nothing, nor does one on zeros)
+      const float f0 = __shfl_sync(0xffffffffu, corr, cq * 4), f1 = __shfl_sync(0xffffffffu, corr, cq * 4 + 4);
 #pragma unroll
-    for (int j = 0; j < NT; ++j) {
-      o[j][0] *= corr;
-      o[j][1] *= corr;
+      for (int j = 0; j < D / 16; ++j) {
+        o[j][0] *= f0; o[j][1] *= f1;
+        o[j][2] *= f0; o[j][3] *= f1;
+      }
     }
-    if (!do_new) {
-      cp_async_wait_group<1>();  // the values
-      __syncwarp();
+    if (!landed(bar_v)) {
+      tc::mbar_drain(bar_v, phase, a.err);
+      if (c0 + 4 * KT < t1) tc::mbar_drain(bar_k, phase ^ 1u, a.err);
+      break;
     }
-    // O += P V; rows 8..15 of P are zero
+    insert(vw, vnew);
+    if (live < KT) {  // probability zero times whatever lies behind the live rows must not be NaN
+      for (int i = lane; i < (KT - live) * CH; i += 32) *chunk_of(vw, live + i / CH, i % CH) = make_uint4(0u, 0u, 0u, 0u);
+    }
+    __syncwarp();
+    // O^T += V^T P^T: the scores' fragments are those of P^T
 #pragma unroll
     for (int kk = 0; kk < KT / 16; ++kk) {
-      const uint32_t a0 = pack_bf16(s[2 * kk][0], s[2 * kk][1]);
-      const uint32_t a2 = pack_bf16(s[2 * kk + 1][0], s[2 * kk + 1][1]);
+      const uint32_t b0 = pack_bf16(s[2 * kk][0], s[2 * kk][1]);
+      const uint32_t b1 = pack_bf16(s[2 * kk + 1][0], s[2 * kk + 1][1]);
 #pragma unroll
-      for (int j = 0; j < NT; j += 2) {
-        uint32_t b0, b1, b2, b3;
-        const int key = kk * 16 + (lane & 7) + 8 * ((lane >> 3) & 1);
-        const int col = j * 8 + 8 * (lane >> 4);
-        ldsm_x4_t(vw_u + (uint32_t)(key * LD + col) * 2u, b0, b1, b2, b3);
-        mma_bf16(o[j], a0, 0u, a2, 0u, b0, b1);
-        mma_bf16(o[j + 1], a0, 0u, a2, 0u, b2, b3);
+      for (int j = 0; j < D / 16; ++j) {
+        uint32_t a0, a1, a2, a3;
+        ldsm_x4_t(xa[j & 3] + to_v + (uint32_t)(kk * 16 * 128 + j / 4 * BOX), a0, a1, a2, a3);
+        mma_bf16(o[j], a0, a1, a2, a3, b0, b1);
       }
     }
     __syncwarp();
-    if (do_new) break;
-    c0 += 4 * KT;
-    request(c0, vw_u, vbase);
+    request(c0 + 4 * KT, false);
+    phase ^= 1u;
   }
 
   // ---- 3. merge the four warps in this CTA, then the slices across the cluster ----
+  if ((lane & 3) == 0) red_m[warp * MAX_REP + hr] = m;
   env.sync_cta();  // all tiles are dead: reuse their space
-  if (hr < rep) {
-    if ((lane & 3) == 0) { red_m[warp * MAX_REP + hr] = m; red_l[warp * MAX_REP + hr] = l; }
+  // the maximum over the warps, to which each brings its sums and outputs
+  auto top_of = [&](int r) { return fmaxf(fmaxf(red_m[r], red_m[MAX_REP + r]), fmaxf(red_m[2 * MAX_REP + r], red_m[3 * MAX_REP + r])); };
+  auto factor = [&](int r) {
+    const float mw = red_m[warp * MAX_REP + r];
+    return mw == -INFINITY ? 0.f : __expf(mw - top_of(r));
+  };
+  auto sum_of = [&](int r) { return (red_l[r] + red_l[MAX_REP + r]) + (red_l[2 * MAX_REP + r] + red_l[3 * MAX_REP + r]); };
+  if ((lane & 3) == 0) red_l[warp * MAX_REP + hr] = l * factor(hr);
 #pragma unroll
-    for (int j = 0; j < NT; ++j) {
-      red_o[(warp * MAX_REP + hr) * D + j * 8 + cq] = o[j][0];
-      red_o[(warp * MAX_REP + hr) * D + j * 8 + cq + 1] = o[j][1];
+  for (int h = 0; h < 2; ++h) {
+    const int r = cq + h;
+    if (r < rep) {
+      const float f = factor(r);
+      float* to = red_o + (warp * MAX_REP + r) * LDO + hr;
+#pragma unroll
+      for (int j = 0; j < D / 16; ++j) {
+        to[j * 16] = o[j][h] * f;
+        to[j * 16 + 8] = o[j][2 + h] * f;
+      }
     }
   }
-  env.sync_cta();
-  // this slice's partial: part[r] = {max, sum}, part_o[r][e], left in shared memory for the cluster
-  float* part_ml = (float*)vt;                 // [MAX_REP][2]
-  float* part_o = part_ml + 2 * MAX_REP;       // [MAX_REP][D]
-  const int S = a.splits;
   // the merged output oo over the merged sum ll of exp(score - mm), which the sink joins, gated and scaled
   auto finished = [&](int r, int e, float mm, float ll, float oo) {
     if constexpr (Env::kRows) {
@@ -445,115 +558,114 @@ __device__ __forceinline__ void attn_dec_item(const AttnDecArgs& a, float scale,
     }
     return ll > 0.f ? oo / ll : 0.f;
   };
-  const bool push = Env::kPush && a.push_merge && S > 1;
-  // push form: output i is finished by slice (i / 128) % S, as its block number (i / 128) / S
-  const int kmax = (rep * D + 128 * S - 1) / (128 * S);
-  float* land_ml = nullptr;   // [8][MAX_REP][2]
-  float* land_o = nullptr;    // [S][kmax][128]
-  uint32_t land_u = 0;
-  if (push) {
-    land_ml = env.landing();
-    land_o = land_ml + 8 * MAX_REP * 2;
-    land_u = (uint32_t)__cvta_generic_to_shared(land_ml);
-  }
-  auto st_remote = [&](uint32_t local_addr, uint32_t rank, float v) {
-    uint32_t remote;
-    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(local_addr), "r"(rank));
-    asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(remote), "f"(v) : "memory");
+  auto store = [&](int r, int e, float v) { a.out[b * ld_out + (kvh * rep + r) * (int64_t)D + e] = __float2bfloat16_rn(v); };
+  // four neighbouring outputs, added over the warps in order
+  auto four = [&](int r, int e) {
+    float4 v = *(const float4*)(red_o + r * LDO + e);
+#pragma unroll
+    for (int w = 1; w < 4; ++w) {
+      const float4 x = *(const float4*)(red_o + (w * MAX_REP + r) * LDO + e);
+      v.x += x.x; v.y += x.y; v.z += x.z; v.w += x.w;
+    }
+    return v;
   };
-  for (int i = tid; i < rep * D; i += 128) {
-    const int r = i / D, e = i - r * D;
-    float mm = -INFINITY;
-    for (int w = 0; w < 4; ++w) mm = fmaxf(mm, red_m[w * MAX_REP + r]);
-    float ll = 0.f, oo = 0.f;
-    for (int w = 0; w < 4; ++w) {
-      const float mw = red_m[w * MAX_REP + r];
-      const float f = mw == -INFINITY ? 0.f : __expf(mw - mm);
-      ll += red_l[w * MAX_REP + r] * f;
-      oo += red_o[(w * MAX_REP + r) * D + e] * f;
-    }
-    if (push) {
-      const int blk = i >> 7;
-      st_remote(land_u + (uint32_t)(8 * MAX_REP * 2 + ((split * kmax + blk / S) << 7) + (i & 127)) * 4u, env.cluster_rank(blk % S), oo);
-      if (e == 0)
-        for (int s = 0; s < S; ++s) {
-          st_remote(land_u + (uint32_t)((split * MAX_REP + r) * 2) * 4u, env.cluster_rank(s), mm);
-          st_remote(land_u + (uint32_t)((split * MAX_REP + r) * 2 + 1) * 4u, env.cluster_rank(s), ll);
-        }
-      continue;
-    }
-    if (e == 0) { part_ml[2 * r] = mm; part_ml[2 * r + 1] = ll; }
-    part_o[r * D + e] = oo;
-  }
-  if (push) {
-    // one barrier: every slice's pushes are visible after it and nobody touches another CTA's
-    // shared memory again
-    env.sync_group();
-    int k = 0;
-    for (int i = tid + 128 * split; i < rep * D; i += 128 * S, ++k) {
-      const int r = i / D;
-      float ms[8], ls[8], os[8];
-#pragma unroll
-      for (int s = 0; s < 8; ++s) {
-        const bool in = s < S;
-        ms[s] = in ? land_ml[(s * MAX_REP + r) * 2] : -INFINITY;
-        ls[s] = in ? land_ml[(s * MAX_REP + r) * 2 + 1] : 0.f;
-        os[s] = in ? land_o[((s * kmax + k) << 7) + tid] : 0.f;
-      }
-      float mm = -INFINITY;
-#pragma unroll
-      for (int s = 0; s < 8; ++s) mm = fmaxf(mm, ms[s]);
-      float ll = 0.f, oo = 0.f;
-#pragma unroll
-      for (int s = 0; s < 8; ++s) {
-        const float f = ms[s] == -INFINITY ? 0.f : __expf(ms[s] - mm);
-        ll += ls[s] * f;
-        oo += os[s] * f;
-      }
-      a.out[b * ld_out + (kvh * rep + r) * (int64_t)D + (i - r * D)] = __float2bfloat16_rn(finished(r, i - r * D, mm, ll, oo));
-    }
-    return;
-  }
+  env.sync_cta();
   if (S == 1) {
-    env.sync_cta();
-    for (int i = tid; i < rep * D; i += 128) {
-      const int r = i / D, e = i - r * D;
-      const float ll = part_ml[2 * r + 1];
-      a.out[b * ld_out + (kvh * rep + r) * (int64_t)D + e] = __float2bfloat16_rn(finished(r, e, part_ml[2 * r], ll, part_o[i]));
+    for (int i = tid * 4; i < rep * D; i += 512) {
+      const int r = i / D, e = i % D;
+      const float4 v = four(r, e);
+      const float mm = top_of(r), ll = sum_of(r);
+      store(r, e, finished(r, e, mm, ll, v.x));
+      store(r, e + 1, finished(r, e + 1, mm, ll, v.y));
+      store(r, e + 2, finished(r, e + 2, mm, ll, v.z));
+      store(r, e + 3, finished(r, e + 3, mm, ll, v.w));
     }
     env.sync_cta();  // the partials are read: the next item of a resident CTA may reuse the space
     return;
   }
-  // the slices of one (row, kv head) are one thread-block cluster: merge over distributed
-  // shared memory, each CTA finishing an interleaved share of the outputs
-  env.sync_group();
-  const uint32_t ml_u = (uint32_t)__cvta_generic_to_shared(part_ml);
-  const uint32_t po_u = (uint32_t)__cvta_generic_to_shared(part_o);
-  for (int i = tid + 128 * split; i < rep * D; i += 128 * S) {
-    const int r = i / D;
-    // all remote loads first (their latencies overlap), then the arithmetic; S <= 8
-    float ms[8], ls[8], os[8];
-#pragma unroll
-    for (int s = 0; s < 8; ++s) {
-      const bool in = s < S;
-      ms[s] = in ? attn_ld_dsmem(ml_u + (uint32_t)(2 * r) * 4u, env.cluster_rank(s)) : -INFINITY;
-      ls[s] = in ? attn_ld_dsmem(ml_u + (uint32_t)(2 * r + 1) * 4u, env.cluster_rank(s)) : 0.f;
-      os[s] = in ? attn_ld_dsmem(po_u + (uint32_t)i * 4u, env.cluster_rank(s)) : 0.f;
-    }
+  // The slices of one (row, kv head) lie in one thread-block cluster.  (Kept as loops: every instruction of a step's
+  // kernel is fetched anew, and 16 slices unrolled took 1000 to 2500 cycles here.)
+  auto merge = [&](int r, int e, auto ml, auto ol) {
     float mm = -INFINITY;
-#pragma unroll
-    for (int s = 0; s < 8; ++s) mm = fmaxf(mm, ms[s]);
+#pragma unroll 4
+    for (int s = 0; s < S; ++s) mm = fmaxf(mm, ml(s).x);
     float ll = 0.f, oo = 0.f;
-#pragma unroll
-    for (int s = 0; s < 8; ++s) {
-      const float f = ms[s] == -INFINITY ? 0.f : __expf(ms[s] - mm);
-      ll += ls[s] * f;
-      oo += os[s] * f;
+#pragma unroll 4
+    for (int s = 0; s < S; ++s) {
+      const float2 x = ml(s);
+      const float f = x.x == -INFINITY ? 0.f : __expf(x.x - mm);
+      ll += x.y * f;
+      oo += ol(s) * f;
     }
-    a.out[b * ld_out + (kvh * rep + r) * (int64_t)D + (i - r * D)] = __float2bfloat16_rn(finished(r, i - r * D, mm, ll, oo));
+    store(r, e, finished(r, e, mm, ll, oo));
+  };
+  if constexpr (Env::kPush) {
+    auto remote = [&](uint32_t addr, int rank) {
+      uint32_t to;
+      asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(to) : "r"(addr), "r"(rank));
+      return to;
+    };
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+    if (tid < MAX_REP * S && (tid & (MAX_REP - 1)) < rep) {
+      const int s = tid / MAX_REP, r = tid & (MAX_REP - 1);
+      const float mm = top_of(r), ll = sum_of(r);
+      asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.v2.b32 [%0], {%1, %2}, [%3];" ::"r"(
+                       remote(land_ml + (uint32_t)((split * MAX_REP + r) * 8), s)),
+                   "r"(__float_as_uint(mm)), "r"(__float_as_uint(ll)), "r"(remote(land_bar, s))
+                   : "memory");
+    }
+    for (int i = tid * 4; i < rep * D; i += 512) {
+      const int r = i / D, e = i % D, owner = e >> lgw;
+      const float4 v = four(r, e);
+      asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.v4.b32 [%0], {%1, %2, %3, %4}, [%5];" ::"r"(
+                       remote(land_o + (uint32_t)((split * per + r * wide + (e & (wide - 1))) * 4), owner)),
+                   "r"(__float_as_uint(v.x)), "r"(__float_as_uint(v.y)), "r"(__float_as_uint(v.z)), "r"(__float_as_uint(v.w)),
+                   "r"(remote(land_bar, owner))
+                   : "memory");
+    }
+    // Arrived when every CTA of the cluster has issued its pushes; waited for before this CTA leaves, so that no
+    // push can find its target gone even where a wait has given up.
+    __syncwarp();
+    asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
+    if (tc::mbar_wait_cluster(land_bar, 0, cta_abort, a.err)) {
+      const float* ml = env.landing() + 4;
+      const float* ol = ml + S * MAX_REP * 2;
+      for (int t = tid; t < per; t += 128) {
+        const int r = t >> lgw;
+        merge(r, split * wide + (t & (wide - 1)), [&](int s) { return *(const float2*)(ml + (s * MAX_REP + r) * 2); },
+              [&](int s) { return ol[s * per + t]; });
+      }
+    }
+    __syncwarp();
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+    if (*cta_abort) tc::mbar_drain(land_bar, 0, a.err);  // (issued is not arrived: what is still on its way, after a wait gave up)
+  } else {
+    // this slice's partial: {max, sum} and the values of every head, left in shared memory for the group
+    float* part_ml = red_o + 4 * MAX_REP * LDO;  // [MAX_REP][2]
+    float* part_o = part_ml + 2 * MAX_REP;       // [MAX_REP][D]
+    for (int i = tid * 4; i < rep * D; i += 512) {
+      const int r = i / D, e = i % D;
+      if (e == 0) {
+        part_ml[2 * r] = top_of(r);
+        part_ml[2 * r + 1] = sum_of(r);
+      }
+      *(float4*)(part_o + i) = four(r, e);
+    }
+    env.sync_group();
+    const uint32_t ml_u = (uint32_t)__cvta_generic_to_shared(part_ml);
+    const uint32_t po_u = (uint32_t)__cvta_generic_to_shared(part_o);
+    for (int t = tid; t < per; t += 128) {
+      const int r = t >> lgw, e = split * wide + (t & (wide - 1));
+      merge(r, e,
+            [&](int s) {
+              return make_float2(attn_ld_dsmem(ml_u + (uint32_t)(2 * r) * 4u, env.cluster_rank(s)),
+                                 attn_ld_dsmem(ml_u + (uint32_t)(2 * r + 1) * 4u, env.cluster_rank(s)));
+            },
+            [&](int s) { return attn_ld_dsmem(po_u + (uint32_t)(r * D + e) * 4u, env.cluster_rank(s)); });
+    }
+    // nobody leaves while a peer may still read its shared memory
+    env.sync_group();
   }
-  // nobody leaves while a peer may still read its shared memory
-  env.sync_group();
 }
 
 }  // namespace cg

@@ -503,7 +503,7 @@ __global__ void __launch_bounds__(R_THREADS, 1) k_decode_resident(const __grid_c
         a.qkv = p.qkv; a.cos_t = L.cos_t; a.sin_t = L.sin_t; a.q_gamma = L.q_gamma; a.k_gamma = L.k_gamma;
         a.norm_eps = p.eps; a.norm_plus_one = p.plus_one; a.k_cache = L.k_cache; a.v_cache = L.v_cache; a.out = p.att;
         a.pos_dev = nullptr; a.pos0 = pos0 + step; a.Tmax = p.Tmax; a.B = p.M; a.nh = p.nh; a.nkv = p.nkv; a.d = D;
-        a.window = L.window; a.softcap = p.attn_softcap; a.splits = p.attn_group; a.push_merge = 0;
+        a.window = L.window; a.softcap = p.attn_softcap; a.splits = p.attn_group; a.err = p.err;
         const int groups_per_cluster = R_CS / p.attn_group;
         const int n_groups = p.n_clusters * groups_per_cluster;
         const int pairs = p.M * p.nkv;

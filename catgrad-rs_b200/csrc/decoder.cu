@@ -398,7 +398,6 @@ int run_layers(cg_decoder* D, int64_t B, int64_t S, int64_t pos0, bool from_dev_
     const bool windowed = cfg.sliding_window > 0 && (cfg.window_every <= 1 || (li % cfg.window_every) != cfg.window_every - 1);
     if (S == 1) {
       AttnDecArgs f;
-      f.push_merge = 0;  // (chosen by the launcher)
       f.qkv = (const float*)D->qkvb->data();
       f.cos_t = cos_t;
       f.sin_t = sin_t;
@@ -409,12 +408,13 @@ int run_layers(cg_decoder* D, int64_t B, int64_t S, int64_t pos0, bool from_dev_
       f.k_cache = (__nv_bfloat16*)L.k_cache->data();
       f.v_cache = (__nv_bfloat16*)L.v_cache->data();
       f.out = (__nv_bfloat16*)D->att->data();
+      f.cache_rows = L.k_cache->numel() / D->d;
       f.pos_dev = from_dev_pos ? D->pos_dev() : nullptr;
       f.pos0 = pos0; f.Tmax = cfg.max_seq; f.B = B;
       f.nh = D->nh; f.nkv = D->nkv; f.d = D->d;
       f.window = windowed ? cfg.sliding_window : 0;
       f.softcap = cfg.attn_softcap;
-      f.splits = attn_dec_splits(cfg.max_seq, B * D->nkv, D->d);
+      f.splits = attn_dec_splits(windowed ? std::min<int64_t>(cfg.sliding_window, cfg.max_seq) : cfg.max_seq, B * D->nkv);
       CG_TRY(k_launch_attn_dec(c, f));
     } else {
     RopeStoreArgs r;

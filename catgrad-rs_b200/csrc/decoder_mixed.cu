@@ -914,6 +914,7 @@ int attention_layer(cg_decoder* D, const MixedLayer& L, MixedRun& run, const Row
     f.cos_t = (const float*)L.cos_t->data(); f.sin_t = (const float*)L.sin_t->data();
     f.q_gamma = q_gain; f.k_gamma = k_gain; f.norm_eps = D->cfg.rms_eps;
     f.k_cache = (__nv_bfloat16*)run.cache->data(); f.v_cache = (__nv_bfloat16*)run.cache_v->data();
+    f.cache_rows = run.cache->numel() / L.Dk;
     f.out = (__nv_bfloat16*)out.p; f.ld_out = out.ld;
     f.head_norm = k.qk_norm == 2; f.keep_first = k.keep_first;
     f.gate = gate; f.ld_gate = in.ld; f.out_scale = L.out_scale();
@@ -923,7 +924,7 @@ int attention_layer(cg_decoder* D, const MixedLayer& L, MixedRun& run, const Row
     f.scale = (float)k.scale; f.sink = sink;
     f.wide_gate = k.gate == 2; f.q_temp = q_temp; f.bias = bias; f.ld_bias = ld_bias;
     const int64_t reach = k.window > 0 ? std::min<int64_t>((int64_t)k.window + k.keep_first, f.Tmax) : f.Tmax;
-    f.splits = attn_dec_splits(reach, f.B * f.nkv, f.d);
+    f.splits = attn_dec_splits(reach, f.B * f.nkv);
     return k_launch_attn_dec(c, f);
   }
   RowsAttnArgs a;

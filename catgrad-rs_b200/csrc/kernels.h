@@ -161,11 +161,12 @@ struct AttnDecArgs {
   const float* bias = nullptr;   // rows: [nh], ld_bias apart: bias[distance] is taken off the scores
   int64_t ld_bias = 0;
   const float* q_temp = nullptr; // rows: [Tmax], factor on the query at a position
-  int push_merge;                // set by the launcher: the slices' partials are pushed to the finishing CTA
+  int64_t cache_rows = 0;        // rows of d values in each cache: all slots' [nkv, Tmax]
+  int32_t* err = nullptr;        // error block of the bounded waits (set by the launcher)
 };
 // Rope + cache append + attention + merge of one new token per row, in one launch.
 int k_launch_attn_dec(cg_ctx* c, const AttnDecArgs& a);
-int attn_dec_splits(int64_t Tmax, int64_t pairs, int d);
+int attn_dec_splits(int64_t Tmax, int64_t pairs);
 
 // tokens[b] = argmax over the vocabulary with the reference's tie rule (last index); optional
 // soft-cap applied to the logits in place first.  The logits are `parts` vocabulary slices of

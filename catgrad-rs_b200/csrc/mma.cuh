@@ -1,5 +1,5 @@
-// mma.cuh — warp-level tensor-core helpers for the attention kernels: ldmatrix fragment loads
-// and the bf16 m16n8k16 MMA with f32 accumulation.
+// mma.cuh — helpers of the attention kernels: ldmatrix fragment loads, the bf16 m16n8k16 MMA with f32
+// accumulation, exponentials and reciprocals.
 #pragma once
 
 #include <cuda_bf16.h>
@@ -28,6 +28,19 @@ __device__ __forceinline__ void mma_bf16(float* c, uint32_t a0, uint32_t a1, uin
 __device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
   __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
   return *(uint32_t*)&v;
+}
+__device__ __forceinline__ float fast_exp2(float x) {
+  float y;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+// 1 / x for x >= 1 (as good as 0 above 1e37): the approximation and one step of Newton's iteration, so that a soft-capped
+// score keeps its 24 bits.  (Prompt attention, 2048 tokens, 8 heads of 256: 183 us without the step, 189 with it, 455 with a division.)
+__device__ __forceinline__ float rcp_newton(float x) {
+  float y;
+  x = x > 1e37f ? 1e37f : x;  // (a NaN stays one)
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return fmaf(y, fmaf(-x, y, 1.f), y);
 }
 // 16-byte asynchronous copy global -> shared; src_bytes = 0 writes zeros
 __device__ __forceinline__ void cp_async16(uint32_t dst, const void* src, int src_bytes) {
