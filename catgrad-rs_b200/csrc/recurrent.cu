@@ -191,6 +191,11 @@ __global__ void __launch_bounds__(128) k_recur_steps(RecurArgs a) {
 // ------------------------------------------------------------------ one token per row ----
 // One block per (head, row).  A thread keeps four columns of up to RD_ROWS rows of the state in
 // registers from the load to the store; sums over the key dimension go through shared memory.
+// What bounds it is the chain from the projection to the output, beside 5 us of state bytes at batch 8: so all that does not
+// depend on the projection (state, earlier inputs of the convolutions, weights, gains) is read before it is waited
+// for, its values come in one round of loads, and four barriers are left.  Four blocks per SM where a thread has
+// eight rows, which lets 512 blocks start at once.  Us that a launch keeps the stream, 8 rows, before / now: 64 heads of
+// 128 x 64: 17.4 / 11.6; 32 heads of 128 x 128 with the delta rule: 12.9 / 12.0.
 // KD: a decay per key channel; the second factors of the low-rank projections are applied here, a row of them
 // per thread, from shared memory where they fit (rows R + 8 apart: no bank conflicts).
 __device__ __forceinline__ float low_rank_staged(const float* x, const __nv_bfloat16* w, int R) {
@@ -207,10 +212,11 @@ __device__ __forceinline__ float low_rank_staged(const float* x, const __nv_bflo
   return v[0] + v[1];
 }
 template <int RD_ROWS, bool KD>
-__global__ void __launch_bounds__(256, RD_ROWS <= 8 ? 3 : 2) k_recur_decode(RecurArgs a, GatedNorm n) {
+__global__ void __launch_bounds__(256, RD_ROWS <= 8 ? 4 : 2) k_recur_decode(RecurArgs a, GatedNorm n) {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-  __shared__ float sq[128], sk[128], sv[128], so[128], sg[4];
-  __shared__ float sd[KD ? 128 : 1], sgate[KD ? 128 : 1];  // decays, gates before their activation
+  __shared__ __align__(16) float sq[128], sk[128], sv[128];
+  __shared__ float sg[4];
+  __shared__ float sd[KD ? 128 : 1], sgate[128], sgain[128];  // decays, gates before their activation, the norm's gains
   // KD: [a_rank], [g_rank]; with w_staged then this head's rows of the second factors
   extern __shared__ __align__(16) float low[];
   __nv_bfloat16* const staged = (__nv_bfloat16*)(low + (a.a_rank + a.g_rank));  // (ranks are multiples of 8)
@@ -227,7 +233,7 @@ __global__ void __launch_bounds__(256, RD_ROWS <= 8 ? 3 : 2) k_recur_decode(Recu
                  (decay ? wa : wg) + x * 8, 16);
     }
   }
-  __shared__ __align__(16) float red[1024];
+  __shared__ __align__(16) float red[KD ? 1 : 2][1024];  // (KD: staged weights want the room)
   const int h = blockIdx.x, row = blockIdx.y, rep = a.H / a.KH, kh = h / rep;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int lpr = a.dvs / 4, rpp = 256 / lpr;         // threads per state row, rows per pass
@@ -252,31 +258,72 @@ __global__ void __launch_bounds__(256, RD_ROWS <= 8 ? 3 : 2) k_recur_decode(Recu
   asm volatile("ld.acquire.gpu.global.s64 %0, [%1];" : "=l"(step_early) : "l"(a.rows.step) : "memory");
   const int64_t pos_early = a.rows.pos0[row] + step_early;
   load_state(pos_early > 0);
+  // The short convolutions of this head's channels, two a thread at most: bias and earlier inputs now (their last
+  // writer is the state's), the projection's new input behind the wait.
+  float* tail = a.tail + (int64_t)slot * a.taps * a.C;
+  const int n_conv = 2 * a.dk + a.dvs;
+  int ring = 0;
+  float past[2], w_now[2];
+  auto part_of = [&](int x) { return x < a.dk ? 0 : x < 2 * a.dk ? 1 : 2; };
+  auto channel = [&](int x) {
+    const int seg = part_of(x);
+    return seg == 0 ? a.q_off + kh * a.qs + x : seg == 1 ? a.k_off + kh * a.qs + x - a.dk : a.v_off + h * a.vs + x - 2 * a.dk;
+  };
+  auto has = [&](int x) { return x < 2 * a.dk + a.dv; };  // (values past dv are padding)
+  auto load_past = [&](int64_t pos) {
+    ring = a.taps ? (int)((uint32_t)pos % (uint32_t)a.taps) : 0;  // this position's place among the last inputs
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      const int x = tid + 256 * i;
+      past[i] = 0.f; w_now[i] = 1.f;
+      if (!a.taps || !has(x)) continue;
+      const int c = channel(x);
+      const float* w = a.conv_w + (int64_t)c * a.taps + a.taps - 1;
+      float v = a.conv_b ? a.conv_b[c] : 0.f;
+      w_now[i] = w[0];
+      for (int j = 1; j < a.taps; ++j)
+        if (pos >= j) v += w[-j] * __ldcg(tail + (int64_t)(ring >= j ? ring - j : ring - j + a.taps) * a.C + c);
+      past[i] = v;
+    }
+  };
+  load_past(pos_early);
+  // one thread with little else to do takes the decay and the step size
+  const bool gates = tid == 255;
+  float dt_bias = 0.f, a_exp = 0.f;
+  if (!KD && gates && !a.log_decay) { dt_bias = a.dt_bias[h]; a_exp = expf(a.a_log[h]); }
+  const bool normed = a.delta || KD;
+  if (normed && tid < a.dv) sgain[tid] = n.norm[tid];
   asm volatile("griddepcontrol.wait;" ::: "memory");
   int64_t step_now;
   asm volatile("ld.acquire.gpu.global.s64 %0, [%1];" : "=l"(step_now) : "l"(a.rows.step) : "memory");
   const int64_t m = row, pos = a.rows.pos0[row] + step_now;
-  if (pos != pos_early) load_state(pos > 0);
-  // short convolutions of this head's channels
   const float* p = a.proj + m * a.ldp;
-  float* tail = a.tail + (int64_t)slot * a.taps * a.C;
-  const int ring = a.taps ? (int)((uint32_t)pos % (uint32_t)a.taps) : 0;  // this position's place among the last inputs
-  for (int x = tid; x < 2 * a.dk + a.dvs; x += 256) {
-    const int seg = x < a.dk ? 0 : x < 2 * a.dk ? 1 : 2;
-    const int e = seg == 0 ? x : seg == 1 ? x - a.dk : x - 2 * a.dk;
-    if (seg == 2 && e >= a.dv) { sv[e] = 0.f; continue; }
-    const int c = seg == 0 ? a.q_off + kh * a.qs + e : seg == 1 ? a.k_off + kh * a.qs + e : a.v_off + h * a.vs + e;
-    const float now = p[c];
-    float v = now;
-    if (a.taps) {
-      v = (a.conv_b ? a.conv_b[c] : 0.f) + a.conv_w[(int64_t)c * a.taps + a.taps - 1] * now;
-      for (int j = 1; j < a.taps; ++j)
-        if (pos >= j) v += a.conv_w[(int64_t)c * a.taps + a.taps - 1 - j] * tail[(int64_t)(ring >= j ? ring - j : ring - j + a.taps) * a.C + c];
-      if (seg == 2 || h % rep == 0) tail[(int64_t)ring * a.C + c] = now;  // read by no block of this step
+  const float* sp = p + a.small_off;
+  float now[2], g_in = 0.f, b_in = 0.f;
+#pragma unroll
+  for (int i = 0; i < 2; ++i) now[i] = has(tid + 256 * i) ? p[channel(tid + 256 * i)] : 0.f;
+  if (gates) {
+    if (a.delta) b_in = sp[h];
+    if (!KD && !a.log_decay) g_in = sp[a.delta ? a.H + h : h];
+  }
+  if (a.delta && !KD && tid < a.dv) sgate[tid] = ((const float*)n.gate)[m * n.ldg + (int64_t)h * a.dv + tid];
+  if (pos != pos_early) {
+    load_state(pos > 0);
+    load_past(pos);
+  }
+#pragma unroll
+  for (int i = 0; i < 2; ++i) {
+    const int x = tid + 256 * i;
+    if (x >= n_conv) break;
+    const int seg = part_of(x);
+    float v = 0.f;
+    if (has(x)) {
+      v = a.taps ? past[i] + w_now[i] * now[i] : now[i];
+      if (a.taps && (seg == 2 || h % rep == 0)) tail[(int64_t)ring * a.C + channel(x)] = now[i];  // read by no block of this step
+      if (a.linear) v *= seg == 0 ? a.q_scale : 1.f;
+      else v = silu(v);
     }
-    if (a.linear) v *= seg == 0 ? a.q_scale : 1.f;
-    else v = silu(v);
-    (seg == 0 ? sq : seg == 1 ? sk : sv)[e] = v;
+    (seg == 0 ? sq : seg == 1 ? sk : sv)[x - seg * a.dk] = v;
   }
   if (KD) {
     for (int j = tid; j < a.a_rank; j += 256) low[j] = p[a.a1_off + j];
@@ -304,34 +351,35 @@ __global__ void __launch_bounds__(256, RD_ROWS <= 8 ? 3 : 2) k_recur_decode(Recu
       else sgate[e - a.dk] = v;
     }
   }
-  const float* sp = p + a.small_off;
-  if (tid == 64) {
+  if (gates) {
     if (KD) {
-      sg[1] = a.delta ? 1.f / (1.f + expf(-sp[h])) : 1.f;
+      sg[1] = a.delta ? 1.f / (1.f + expf(-b_in)) : 1.f;
     } else if (a.log_decay) {
       sg[0] = expf(a.log_decay[h]);
       sg[1] = 1.f;
     } else {
-      const float dt = softplus(sp[a.delta ? a.H + h : h] + a.dt_bias[h]);
-      sg[0] = expf(-expf(a.a_log[h]) * dt);
-      sg[1] = a.delta ? 1.f / (1.f + expf(-sp[h])) : dt;
+      const float dt = softplus(g_in + dt_bias);
+      sg[0] = expf(-a_exp * dt);
+      sg[1] = a.delta ? 1.f / (1.f + expf(-b_in)) : dt;
     }
   }
   __syncthreads();
+  // delta: queries and keys of unit length (every warp for itself, which saves a barrier)
+  float fq = 1.f, fk = 1.f;
   if (a.delta) {
-    if (warp < 2) {
-      float* x = warp ? sk : sq;
-      float ss = 0.f;
-      for (int e = lane; e < a.dk; e += 32) ss += x[e] * x[e];
-      ss = warp_sum(ss);
-      const float f = (warp ? 1.f : 1.f / sqrtf((float)a.dk)) / sqrtf(ss + 1e-6f);
-      for (int e = lane; e < a.dk; e += 32) x[e] *= f;
+    float qq = 0.f, kk = 0.f;
+    for (int e = lane; e < a.dk; e += 32) { qq += sq[e] * sq[e]; kk += sk[e] * sk[e]; }
+#pragma unroll
+    for (int o = 16; o; o >>= 1) {
+      qq += __shfl_xor_sync(0xffffffffu, qq, o);
+      kk += __shfl_xor_sync(0xffffffffu, kk, o);
     }
-    __syncthreads();
+    fq = 1.f / sqrtf((float)a.dk) / sqrtf(qq + 1e-6f);
+    fk = 1.f / sqrtf(kk + 1e-6f);
   }
   const float g0 = sg[0], co = sg[1];
   auto decay = [&](int r) { return KD ? sd[r < a.dk ? r : 0] : g0; };
-  auto sum_rows = [&](float4 v) {   // over all rows of the state, for this thread's columns
+  auto sum_rows = [&](float4 v, float* red) {   // over all rows of the state, for this thread's columns
     if (act) *(float4*)(red + rg * a.dvs + 4 * cg) = v;
     __syncthreads();
     float4 t = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -350,13 +398,13 @@ __global__ void __launch_bounds__(256, RD_ROWS <= 8 ? 3 : 2) k_recur_decode(Recu
 #pragma unroll
     for (int i = 0; i < RD_ROWS; ++i) {
       const int r = rg + i * rpp;
-      const float k = act && r < a.dk ? sk[r] : 0.f, g = decay(r);
+      const float k = act && r < a.dk ? sk[r] * fk : 0.f, g = decay(r);
       S[i].x *= g; S[i].y *= g; S[i].z *= g; S[i].w *= g;
       s.x += S[i].x * k; s.y += S[i].y * k; s.z += S[i].z * k; s.w += S[i].w * k;
     }
-    s = sum_rows(s);
+    s = sum_rows(s, red[0]);
+    if (KD) __syncthreads();
     u.x -= s.x; u.y -= s.y; u.z -= s.z; u.w -= s.w;
-    __syncthreads();
   }
   u.x *= co; u.y *= co; u.z *= co; u.w *= co;
   float4 o = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -364,7 +412,7 @@ __global__ void __launch_bounds__(256, RD_ROWS <= 8 ? 3 : 2) k_recur_decode(Recu
   for (int i = 0; i < RD_ROWS; ++i) {
     const int r = rg + i * rpp;
     if (act && r < a.dk) {
-      const float k = sk[r], q = sq[r], g = decay(r);
+      const float k = sk[r] * fk, q = sq[r] * fq, g = decay(r);
       if (a.delta) {
         S[i].x += k * u.x; S[i].y += k * u.y; S[i].z += k * u.z; S[i].w += k * u.w;
       } else {
@@ -375,8 +423,9 @@ __global__ void __launch_bounds__(256, RD_ROWS <= 8 ? 3 : 2) k_recur_decode(Recu
       *(float4*)(Sg + (int64_t)r * a.dvs + 4 * cg) = S[i];
     }
   }
-  o = sum_rows(o);
-  if (!a.delta && !KD) {
+  o = sum_rows(o, red[KD ? 0 : 1]);
+  if (warp) return;
+  if (!normed) {
     if (rg == 0) {
       const float d = a.dskip ? a.dskip[h] : 0.f;
       *(float4*)(a.o + m * (int64_t)a.H * a.dvs + (int64_t)h * a.dvs + 4 * cg) =
@@ -384,15 +433,20 @@ __global__ void __launch_bounds__(256, RD_ROWS <= 8 ? 3 : 2) k_recur_decode(Recu
     }
     return;
   }
-  if (rg == 0) *(float4*)(so + 4 * cg) = o;
-  __syncthreads();
-  const float* gate = (const float*)n.gate + m * n.ldg + (int64_t)h * a.dv;
-  const float x = tid < a.dv ? so[tid] : 0.f;
-  const float ss = block_sum(x * x, red);
-  if (tid < a.dv) {
-    const float z = KD ? sgate[tid] : gate[tid];
-    const float y = x / sqrtf(ss / (float)a.dv + n.eps) * n.norm[tid] * (n.sigmoid ? 1.f / (1.f + expf(-z)) : silu(z));
-    const int64_t at = m * n.ld_att + (int64_t)h * a.dv + tid;
+  // the lanes of the first row (of which there are at most 32) hold the head's outputs
+  const float out[4] = {o.x, o.y, o.z, o.w};
+  float ss = 0.f;
+#pragma unroll
+  for (int j = 0; j < 4; ++j)
+    if (4 * lane + j < a.dv) ss += out[j] * out[j];
+  const float len = sqrtf(warp_sum(ss) / (float)a.dv + n.eps);
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    const int e = 4 * lane + j;
+    if (e >= a.dv) break;
+    const float g = sgate[e];
+    const float y = out[j] / len * sgain[e] * (n.sigmoid ? 1.f / (1.f + expf(-g)) : silu(g));
+    const int64_t at = m * n.ld_att + (int64_t)h * a.dv + e;
     if (n.att_bf16) ((__nv_bfloat16*)n.att)[at] = __float2bfloat16_rn(y);
     else ((float*)n.att)[at] = y;
   }

@@ -57,3 +57,15 @@ def test_attention_windows_and_soft_caps(cuda_bf16, D, cap, window):
 @pytest.mark.parametrize("D,nh,nkv", [(64, 4, 4), (128, 8, 1), (128, 6, 2)])
 def test_attention_head_norms(cuda_bf16, D, nh, nkv):
     check(cuda_bf16, shape(D, nh, nkv, arch="qwen3"), 2, [1, 31, 32, 128, 200], 310, spread=1.0)
+
+
+@pytest.mark.parametrize("kind,dk,dv,taps", [("mamba2", 128, 64, 4), ("mamba2", 24, 32, 2), ("mamba2", 128, 128, 3), ("delta", 128, 128, 4),
+                                             ("delta", 128, 64, 4), ("delta", 16, 40, 3), ("delta", 40, 24, 2)])
+def test_recurrences(cuda_bf16, kind, dk, dv, taps):
+    """A block's convolutions: fewer channels than threads and more, values with and without padding."""
+    if kind == "mamba2":
+        sizes = {"heads": 4, "groups": 2, "state": dk, "vdim": dv, "norm_groups": 2, "conv": taps}
+    else:
+        sizes = {"heads": 4, "kv_heads": 2, "dim": dk, "vdim": dv, "conv": taps}
+    cfg = cg.LayeredConfig("step-recurrent", 128, 512, [cg.LayerSpec(kind, sizes, 256 if kind == "delta" else 0)], None)
+    check(cuda_bf16, cfg, 3, [1, 2, 3, 5, 70], 80)
