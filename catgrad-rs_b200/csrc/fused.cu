@@ -247,40 +247,46 @@ __global__ void k_rmsnorm_add_norm(const float* y, const float* g1, const float*
 // gains (weights: nothing in the stream writes them) before the dependency.  Each of the scalar form's three walks
 // over the row waits for its loads: in a step of four rows of 2304 it kept the stream 9.5 us, this one 6.8 us (seven
 // of them in a step of four layers: 482 -> 463 us).
+// Many rows (STEP false) are bound by bytes, 14 per value: there a thread has two vectors (four of rows above 4096),
+// blocks are as wide as the row needs and the gains come when they are used, so that several rows share an SM.  8192
+// rows of 2304: 140 us in the scalar form, 60 in this one (40 at the copy rate).
 constexpr int AN_THREADS = 512, AN_VECS = 4;
-__global__ void __launch_bounds__(AN_THREADS)
+template <int VECS, bool STEP>
+__global__ void __launch_bounds__(AN_THREADS, STEP ? 1 : 2)
 k_rmsnorm_add_norm_vec(const float* y, const float* g1, const float* g2, float eps, int plus_one, int H, float* x, __nv_bfloat16* out) {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   __shared__ float sh[32];
   const int64_t m = blockIdx.x;
-  const int n4 = H / 4, tid = threadIdx.x;
+  const int n4 = H / 4, tid = threadIdx.x, threads = STEP ? AN_THREADS : blockDim.x;
   const float one = plus_one ? 1.f : 0.f;
-  float4 a[AN_VECS], b[AN_VECS], v[AN_VECS], u[AN_VECS];
+  float4 a[VECS], b[VECS], v[VECS], u[VECS];
+  auto gain = [&](const float* g, int j) {
+    const int i = tid + j * threads;
+    return i < n4 ? __ldg((const float4*)g + i) : make_float4(0.f, 0.f, 0.f, 0.f);
+  };
+  if (STEP)
 #pragma unroll
-  for (int j = 0; j < AN_VECS; ++j) {
-    const int i = tid + j * AN_THREADS;
-    a[j] = i < n4 ? __ldg((const float4*)g1 + i) : make_float4(0.f, 0.f, 0.f, 0.f);
-    b[j] = i < n4 ? __ldg((const float4*)g2 + i) : make_float4(0.f, 0.f, 0.f, 0.f);
-  }
+    for (int j = 0; j < VECS; ++j) { a[j] = gain(g1, j); b[j] = gain(g2, j); }
   asm volatile("griddepcontrol.wait;" ::: "memory");
   float ss = 0.f;
 #pragma unroll
-  for (int j = 0; j < AN_VECS; ++j) {
-    const int i = tid + j * AN_THREADS;
+  for (int j = 0; j < VECS; ++j) {
+    const int i = tid + j * threads;
     v[j] = i < n4 ? ((const float4*)(y + m * H))[i] : make_float4(0.f, 0.f, 0.f, 0.f);
     u[j] = i < n4 ? ((const float4*)(x + m * H))[i] : make_float4(0.f, 0.f, 0.f, 0.f);
   }
 #pragma unroll
-  for (int j = 0; j < AN_VECS; ++j) ss += v[j].x * v[j].x + v[j].y * v[j].y + v[j].z * v[j].z + v[j].w * v[j].w;
+  for (int j = 0; j < VECS; ++j) ss += v[j].x * v[j].x + v[j].y * v[j].y + v[j].z * v[j].z + v[j].w * v[j].w;
   const float rms1 = sqrtf(block_sum(ss, sh) / (float)H + eps);
   float s2 = 0.f;
 #pragma unroll
-  for (int j = 0; j < AN_VECS; ++j) {
+  for (int j = 0; j < VECS; ++j) {
+    if (!STEP) a[j] = gain(g1, j);
     u[j].x += v[j].x / rms1 * (one + a[j].x);
     u[j].y += v[j].y / rms1 * (one + a[j].y);
     u[j].z += v[j].z / rms1 * (one + a[j].z);
     u[j].w += v[j].w / rms1 * (one + a[j].w);
-    const int i = tid + j * AN_THREADS;
+    const int i = tid + j * threads;
     if (i < n4) {
       ((float4*)(x + m * H))[i] = u[j];
       s2 += u[j].x * u[j].x + u[j].y * u[j].y + u[j].z * u[j].z + u[j].w * u[j].w;
@@ -288,9 +294,10 @@ k_rmsnorm_add_norm_vec(const float* y, const float* g1, const float* g2, float e
   }
   const float rms2 = sqrtf(block_sum(s2, sh) / (float)H + eps);
 #pragma unroll
-  for (int j = 0; j < AN_VECS; ++j) {
-    const int i = tid + j * AN_THREADS;
+  for (int j = 0; j < VECS; ++j) {
+    const int i = tid + j * threads;
     if (i >= n4) break;
+    if (!STEP) b[j] = gain(g2, j);
     const __nv_bfloat162 p = __floats2bfloat162_rn(u[j].x / rms2 * (one + b[j].x), u[j].y / rms2 * (one + b[j].y)),
                          q = __floats2bfloat162_rn(u[j].z / rms2 * (one + b[j].z), u[j].w / rms2 * (one + b[j].w));
     ((uint2*)(out + m * H))[i] = make_uint2(*(const uint32_t*)&p, *(const uint32_t*)&q);
@@ -887,9 +894,16 @@ int k_launch_rmsnorm_add_norm(cg_ctx* c, const float* y, const float* g1, const 
                               int64_t H, float* x, __nv_bfloat16* out) {
   if (M == 0) return CG_OK;
   const bool aligned = (((uintptr_t)y | (uintptr_t)g1 | (uintptr_t)g2 | (uintptr_t)x | (uintptr_t)out) & 15) == 0;
-  // (its registers leave one block to an SM: 8192 rows take 109 us longer than in the scalar form)
-  if (aligned && M <= 2 * 148 && H % 4 == 0 && H <= AN_THREADS * AN_VECS * 4) {
-    CG_CUDA(c, launch_kernel(c, k_rmsnorm_add_norm_vec, dim3((unsigned)M), dim3(AN_THREADS), 0, 1, y, g1, g2, eps, plus_one, (int)H, x, out));
+  if (aligned && H % 4 == 0 && H <= AN_THREADS * AN_VECS * 4) {
+    // (the form of a step leaves one block to an SM: 8192 rows take 109 us longer in it than in the scalar form)
+    const int n4 = (int)(H / 4);
+    auto threads = [&](int vecs) { return dim3((unsigned)((n4 + vecs * 32 - 1) / (vecs * 32) * 32)); };
+    if (M <= 2 * 148)
+      CG_CUDA(c, launch_kernel(c, k_rmsnorm_add_norm_vec<AN_VECS, true>, dim3((unsigned)M), dim3(AN_THREADS), 0, 1, y, g1, g2, eps, plus_one, (int)H, x, out));
+    else if (n4 <= 2 * AN_THREADS)
+      CG_CUDA(c, launch_kernel(c, k_rmsnorm_add_norm_vec<2, false>, dim3((unsigned)M), threads(2), 0, 1, y, g1, g2, eps, plus_one, (int)H, x, out));
+    else
+      CG_CUDA(c, launch_kernel(c, k_rmsnorm_add_norm_vec<4, false>, dim3((unsigned)M), threads(4), 0, 1, y, g1, g2, eps, plus_one, (int)H, x, out));
     CG_LAUNCHED(c);
     return CG_OK;
   }

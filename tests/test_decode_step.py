@@ -69,3 +69,9 @@ def test_recurrences(cuda_bf16, kind, dk, dv, taps):
         sizes = {"heads": 4, "kv_heads": 2, "dim": dk, "vdim": dv, "conv": taps}
     cfg = cg.LayeredConfig("step-recurrent", 128, 512, [cg.LayerSpec(kind, sizes, 256 if kind == "delta" else 0)], None)
     check(cuda_bf16, cfg, 3, [1, 2, 3, 5, 70], 80)
+
+
+@pytest.mark.parametrize("hidden", [256, 2304, 4096, 4104, 8192])
+def test_post_norms_of_many_rows(cuda_bf16, hidden):
+    """297 rows and more take the residual norms' form for prompts, the step the one for few rows."""
+    check(cuda_bf16, shape(64, 2, 1, hidden, 256, 1, arch="gemma"), 3, [99, 120], 130, spread=1.0)
