@@ -54,8 +54,8 @@ struct KernelEnv {
 };
 
 template <int D, bool ROWS>
-__global__ void __launch_bounds__(128, 4) k_attn_dec(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v, const __grid_constant__ AttnDecArgs a,
-           float scale) {
+__global__ void __launch_bounds__(128, 4)
+k_attn_dec(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v, AttnDecArgs a, float scale) {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw = (uint32_t)__cvta_generic_to_shared(smem_raw);
