@@ -29,6 +29,13 @@
 //     A step of the Llama-3.2-1B shape, batch 1 / batch 8: 733 / 835 us -> 645 / 754 us; four layers of
 //     the Gemma-2-2B shape 514 -> 491 us, the Ralapel design 792 -> 740 us.  Of that the early requests and
 //     the cheaper epilogue indices give 7 %.
+//     The epilogue is bound by instructions of a few warps, not by bytes.  It has one form per kind of output,
+//     a thread finishes one row and steps through the tokens by constants, only the splits there are get added,
+//     sigmoids have no division, and the sums of squares of a handed-over norm are asked for together with the
+//     activations instead of behind them.  From a per-CTA timeline (Llama-3.2-1B shape, batch 8): the norm's factors
+//     3200 -> 900 cycles behind the activations, ahead of the accumulators now; a value's way from the last addend to
+//     memory 1900 to 5800 -> 800 to 2200.  Ms per pass: Llama-3.2-1B shape, batch 8 101.2 -> 98.9, four layers
+//     of the Llama-3-8B shape, batch 32 66.0 -> 61.8, Ralapel, batch 8 52.5 -> 50.6.
 //
 //   * two optional hand-overs ride on the epilogue.  Norm hand-over: a residual GEMM also
 //     leaves bf16(out * gain) and per-CTA sums of out^2, and the GEMM behind the norm applies
@@ -40,6 +47,7 @@
 // All waits are bounded; on expiry the context's error word is raised and the kernel still
 // passes its cluster barriers, frees its TMEM and returns.
 #include <algorithm>
+#include <type_traits>
 
 #include "act.cuh"
 #include "kernels.h"
@@ -82,6 +90,7 @@ struct DecArgs {
   float ss_inv_h, ss_eps;
 };
 
+constexpr int SS_FIRST = 4;      // partial sums of squares a thread asks for together with its activations
 constexpr int SQ_FLOATS = 2048;  // per-CTA staging of squared outputs (cluster epilogue)
 
 // Timeline of the decode GEMM launches (diagnostics): per slot {first CTA start, predecessor
@@ -96,40 +105,69 @@ __device__ __forceinline__ void trace_max(int slot, int f) {
   if (slot >= 0) atomicMax(&g_trace[slot * 4 + f], (unsigned long long)globaltimer());
 }
 
-// `pre` (optional): the residual and next-norm gain of this element, fetched before the accumulator was ready
-struct Prefetched {
-  bool have;
-  float res, gain;
-};
-__device__ __forceinline__ float finish(const DecArgs& p, int m, int n, float g, float u, uint32_t parity, const float* sc,
-                                        const Prefetched pre = Prefetched{false, 0.f, 0.f}) {
+// What the epilogue does with a finished sum.  One form per kind of output, chosen once per CTA.
+enum Form : int { FORM_F32, FORM_BF16, FORM_RESIDUAL, FORM_NORM, FORM_DUAL, FORM_PUSH };
+template <class F>
+__device__ __forceinline__ void with_form(const DecArgs& p, F f) {
+  if (p.dual) f(std::integral_constant<int, FORM_DUAL>{});
+  else if (p.xb_out) f(std::integral_constant<int, FORM_NORM>{});
+  else if (p.out_mode == 2) f(std::integral_constant<int, FORM_RESIDUAL>{});
+  else if (p.out_mode == 0) f(std::integral_constant<int, FORM_F32>{});
+  else if (p.out_mode == 3) f(std::integral_constant<int, FORM_PUSH>{});
+  else f(std::integral_constant<int, FORM_BF16>{});
+}
+// silu or tanh-gelu of g: 1 / (1 + e^-x) by an approximation and one step of Newton's iteration, which keeps its 24 bits
+// where a division is a call; 0 where e^-x is infinite, NaN where x is NaN, as the division has it
+__device__ __forceinline__ float act_of(int act, float g) {
+  const float x = act == 0 ? g : 1.5957691216f * (g + 0.044715f * g * g * g);
+  const float d = 1.f + __expf(-x);
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(d));
+  return g * (d < 1e37f ? fmaf(r, fmaf(-d, r, 1.f), r) : r);
+}
+// Output (m, n), o = m * ldo + n; `res`: the residual there; `gain`: the next norm's at n.  Returns what the row's sum of
+// squares gets.
+template <int FORM>
+__device__ __forceinline__ float finish(const DecArgs& p, int m, int n, int64_t o, float g, float u, uint32_t parity, const float* sc,
+                                        float res, float gain) {
   if (p.ss_in) {  // the activations were handed over un-normalised: the row's 1 / rms goes here
     g *= sc[m];
     u *= sc[m];
   }
-  float v = g;
-  if (p.dual) v = (p.act == 0 ? silu_f(g) : gelu_f(g)) * u;
-  const int64_t o = (int64_t)m * p.ldo + n;
-  if (p.xb_out) {
+  if constexpr (FORM == FORM_NORM) {
     // residual epilogue that also prepares the next norm: the new residual in f32, its
     // gain-scaled bf16 copy for the next GEMM, and its square for the row's sum of squares
-    const float r = v + (pre.have ? pre.res : p.residual[o]);
+    const float r = g + res;
     ((float*)p.out)[o] = r;
-    const float gw = pre.have ? pre.gain : p.g_next[n];
-    const float gn = p.g_plus_one ? 1.f + gw : gw;
-    p.xb_out[o] = __float2bfloat16_rn(r * gn);
+    p.xb_out[o] = __float2bfloat16_rn(r * gain);
     return r * r;
-  }
-  if (p.out_mode == 3) {
+  } else if constexpr (FORM == FORM_PUSH) {
     // this rank's addend goes into slot [parity][rank] of every rank's exchange area
     const int64_t slot = ((int64_t)parity * p.push.world + p.push.rank) * p.push.max_elems + o;
-    for (int r = 0; r < p.push.world; ++r) p.push.data[r][slot] = v;
-    return 0.f;
+    for (int r = 0; r < p.push.world; ++r) p.push.data[r][slot] = g;
+  } else if constexpr (FORM == FORM_DUAL) {
+    g = act_of(p.act, g) * u;
+    if (p.out_mode == 0) ((float*)p.out)[o] = g;
+    else ((__nv_bfloat16*)p.out)[o] = __float2bfloat16_rn(g);
+  } else if constexpr (FORM == FORM_F32) {
+    ((float*)p.out)[o] = g;
+  } else if constexpr (FORM == FORM_BF16) {
+    ((__nv_bfloat16*)p.out)[o] = __float2bfloat16_rn(bf16_out(p.out_mode, g, p.residual, n));
+  } else {
+    ((float*)p.out)[o] = g + res;
   }
-  if (p.out_mode == 0) ((float*)p.out)[o] = v;
-  else if (p.out_mode != 2) ((__nv_bfloat16*)p.out)[o] = __float2bfloat16_rn(bf16_out(p.out_mode, v, p.residual, n));
-  else ((float*)p.out)[o] = v + (pre.have ? pre.res : p.residual[o]);
   return 0.f;
+}
+// the splits' partial sums in rank order, all loads first
+template <int S>
+__device__ __forceinline__ float add_ranks(const float* x, int step) {
+  float v[S];
+#pragma unroll
+  for (int s = 0; s < S; ++s, x += step) v[s] = *x;
+  float sum = 0.f;
+#pragma unroll
+  for (int s = 0; s < S; ++s) sum += v[s];
+  return sum;
 }
 
 __device__ __forceinline__ void st_async(uint32_t addr, uint32_t v, uint32_t bar) {
@@ -246,7 +284,7 @@ k_gemm_dec(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CU
   if (cluster && !p.xstage_in_ring) asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
 
   bool acc_ok = false;
-  Prefetched pre{false, 0.f, 0.f};
+  float res0 = 0.f, res1 = 0.f, gain = 0.f;  // split-K: residuals of the first two elements this thread will finish, their gain
   if (warp == 0) {
     if (lane == 0) {
       const int pre = min(nkb, STAGES);
@@ -312,18 +350,28 @@ k_gemm_dec(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CU
     const int chunks = npre << (lg_rows + 3);
     uint4 xv[XCH];
     load_x_chunks(p, kb0, et, chunks, lg_rows, xv);
-    if (p.splits > 1 && (p.out_mode == 2 || p.xb_out)) {
-      // split-K: the element this thread will finish first is known now; fetch its residual (and
+    // The sums of squares of the norm that is handed over are asked for together with them: per token the producer's
+    // per-CTA partials, 128 / G threads over the parts for each group of four tokens.
+    const int lg_q = p.M <= 4 ? 0 : p.M <= 8 ? 1 : p.M <= 16 ? 2 : 3;
+    const float* src = p.ss_in + ((et & ((1 << lg_q) - 1)) << 2) + (int64_t)(et >> lg_q) * 32;
+    float4 ssv[SS_FIRST];
+    if (p.ss_in) {
+#pragma unroll
+      for (int i = 0; i < SS_FIRST; ++i) {
+        ssv[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+        if ((et >> lg_q) + i * (128 >> lg_q) < p.ss_parts) ssv[i] = __ldcg((const float4*)(src + (int64_t)i * (128 >> lg_q) * 32));
+      }
+    }
+    if (p.splits > 1 && p.out_mode == 2) {
+      // split-K: the elements this thread will finish first are known now; fetch their residuals (and
       // the next norm's gain) while the MMAs run instead of after the reduction
-      const int lg = p.lg_rows_per;
-      if (et < min(TN, p.M) << lg) {
-        const int col = et >> lg;
-        const int n = n0 + (split << lg) + (et & ((1 << lg) - 1));
-        if (n < p.N) {
-          asm volatile("ld.global.f32 %0, [%1];" : "=f"(pre.res) : "l"(p.residual + (int64_t)col * p.ldo + n) : "memory");
-          if (p.xb_out) asm volatile("ld.global.f32 %0, [%1];" : "=f"(pre.gain) : "l"(p.g_next + n) : "memory");
-          pre.have = true;
-        }
+      const int lg = p.lg_rows_per, col = et >> lg;
+      const int n = n0 + (split << lg) + (et & ((1 << lg) - 1));
+      if (n < p.N) {
+        if (col < p.M) asm volatile("ld.global.f32 %0, [%1];" : "=f"(res0) : "l"(p.residual + (int64_t)col * p.ldo + n) : "memory");
+        if (col + (128 >> lg) < p.M)
+          asm volatile("ld.global.f32 %0, [%1];" : "=f"(res1) : "l"(p.residual + (int64_t)(col + (128 >> lg)) * p.ldo + n) : "memory");
+        if (p.xb_out) asm volatile("ld.global.f32 %0, [%1];" : "=f"(gain) : "l"(p.g_next + n) : "memory");
       }
     }
     store_x_chunks(base + wbytes, stage_bytes, et, chunks, lg_rows, xv);
@@ -335,14 +383,14 @@ k_gemm_dec(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CU
     asm volatile("bar.sync 1, 128;" ::: "memory");
     if (et < npre) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bars + 8 * et) : "memory");
     if (p.ss_in) {
-      // per-token sum of squares = the producer's per-CTA partials, in a fixed order: 128 / G threads
-      // over the parts for each group of four tokens, then a shuffle tree, then the four warps in order
-      const int lg = p.M <= 4 ? 0 : p.M <= 8 ? 1 : p.M <= 16 ? 2 : 3;
-      const float* src = p.ss_in + ((et & ((1 << lg) - 1)) << 2);
+      // in a fixed order: a thread's parts, then a shuffle tree, then the four warps in order
+      const int lg = lg_q;
       float4 a = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+      for (int i = 0; i < SS_FIRST; ++i) { a.x += ssv[i].x; a.y += ssv[i].y; a.z += ssv[i].z; a.w += ssv[i].w; }
 #pragma unroll 4
-      for (int i = et >> lg; i < p.ss_parts; i += 128 >> lg) {
-        const float4 v = __ldcg((const float4*)(src + (int64_t)i * 32));
+      for (int i = (et >> lg) + SS_FIRST * (128 >> lg); i < p.ss_parts; i += 128 >> lg) {
+        const float4 v = __ldcg((const float4*)(src + (int64_t)(i - (et >> lg)) * 32));
         a.x += v.x; a.y += v.y; a.z += v.z; a.w += v.w;
       }
       for (int o = 16; o >= (1 << lg); o >>= 1) {
@@ -357,6 +405,8 @@ k_gemm_dec(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CU
         sc[et] = 1.0f / sqrtf((((sc[32 + et] + sc[64 + et]) + sc[96 + et]) + sc[128 + et]) * p.ss_inv_h + p.ss_eps);
       asm volatile("bar.sync 1, 128;" ::: "memory");
     }
+    // (the peers' barriers: waited for here, where there is time)
+    if (cluster && !p.xstage_in_ring) asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
     if (nkb > 0) {
       acc_ok = mbar_wait(bar_accum, 0, cta_abort, p.err);
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -373,7 +423,7 @@ k_gemm_dec(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CU
     // loads have landed and its MMAs have read them; after this the rings may be written by the peers)
     __syncwarp();
     if (p.xstage_in_ring) asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+    if (p.xstage_in_ring || warp < 2) asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
   }
   // with split-K a CTA whose accumulator never came pushes all the same: its peers count on the bytes
   // (the error word is set: what a peer makes of them is not a result)
@@ -392,33 +442,50 @@ k_gemm_dec(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CU
       asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(xbar) : "r"(bar_x), "r"(owner));
       xdst += (uint32_t)(((split * xcols) << lg) + (row & ((1 << lg) - 1))) * 4u;
     }
+    if (cluster) {
 #pragma unroll 1
-    for (int c0 = 0; c0 < TN; c0 += 16) {
-      if (c0 >= p.M) break;
-      uint32_t g[16], u[16];
-      tmem_ld16(tmem_acc + ((uint32_t)(q * 32) << 16) + (uint32_t)c0, g);
-      if (p.dual) tmem_ld16(tmem_acc + ((uint32_t)(q * 32) << 16) + (uint32_t)(TN + c0), u);
-      asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-      if (cluster) {
+      for (int c0 = 0; c0 < TN; c0 += 16) {
+        if (c0 >= p.M) break;
+        uint32_t g[16], u[16];
+        tmem_ld16(tmem_acc + ((uint32_t)(q * 32) << 16) + (uint32_t)c0, g);
+        if (p.dual) tmem_ld16(tmem_acc + ((uint32_t)(q * 32) << 16) + (uint32_t)(TN + c0), u);
+        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
         for (int j = 0; j < 16; ++j) {
           if (c0 + j >= p.M) break;
           st_async(xdst + ((uint32_t)(c0 + j) << (lg + 2)), g[j], xbar);
           if (p.dual) st_async(xdst + ((uint32_t)(p.xstage_cols + c0 + j) << (lg + 2)), u[j], xbar);
         }
-      } else {
+      }
+    } else {
+      with_form(p, [&](auto form) {
+        constexpr int FORM = decltype(form)::value;
+        const bool in = n < p.N;
+        float gn = 0.f;
+        if (FORM == FORM_NORM && in) gn = p.g_plus_one ? 1.f + p.g_next[n] : p.g_next[n];
+#pragma unroll 1
+        for (int c0 = 0; c0 < TN; c0 += 16) {
+          if (c0 >= p.M) break;
+          uint32_t g[16], u[16];
+          tmem_ld16(tmem_acc + ((uint32_t)(q * 32) << 16) + (uint32_t)c0, g);
+          if (FORM == FORM_DUAL) tmem_ld16(tmem_acc + ((uint32_t)(q * 32) << 16) + (uint32_t)(TN + c0), u);
+          asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+          int64_t o = (int64_t)c0 * p.ldo + n;
 #pragma unroll
-        for (int j = 0; j < 16; ++j) {
-          if (c0 + j >= p.M) break;
-          float r2 = 0.f;
-          if (n < p.N) r2 = finish(p, c0 + j, n, __uint_as_float(g[j]), p.dual ? __uint_as_float(u[j]) : 0.f, parity, sc);
-          if (p.ss_out) {
-            // one CTA per tile here: the tile's 128 rows are summed per token, warp tree then warps in order
-            for (int o = 16; o; o >>= 1) r2 += __shfl_xor_sync(0xffffffffu, r2, o);
-            if (lane == 0) sq[q * 32 + c0 + j] = r2;
+          for (int j = 0; j < 16; ++j, o += p.ldo) {
+            if (c0 + j >= p.M) break;
+            float r2 = 0.f;
+            if (in)
+              r2 = finish<FORM>(p, c0 + j, n, o, __uint_as_float(g[j]), FORM == FORM_DUAL ? __uint_as_float(u[j]) : 0.f, parity, sc,
+                                FORM == FORM_NORM || FORM == FORM_RESIDUAL ? p.residual[o] : 0.f, gn);
+            if (FORM == FORM_NORM) {
+              // one CTA per tile here: the tile's 128 rows are summed per token, warp tree then warps in order
+              for (int i = 16; i; i >>= 1) r2 += __shfl_xor_sync(0xffffffffu, r2, i);
+              if (lane == 0) sq[q * 32 + c0 + j] = r2;
+            }
           }
         }
-      }
+      });
     }
   }
   if (warp >= 2 && p.ss_out && !cluster) {
@@ -442,38 +509,51 @@ k_gemm_dec(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CU
     // cluster where a barrier over all threads costs a return trip
     if (warp >= 2) {
       const bool got = mbar_wait_cluster(bar_x, 0, cta_abort, p.err) && !*cta_abort;
+      // A thread finishes one row n and every (128 >> lg)-th token: what depends on n is done once, the rest
+      // moves on by constants.
       const int S = p.splits, lg = p.lg_rows_per, et = tid - 64;
-      const int todo = min(TN, p.M) << lg;  // columns x rows this CTA finishes
-      const int xcols = (p.dual ? 2 : 1) * p.xstage_cols;
-      const float* xs = (const float*)(gen + xoff);
-      for (int e = et; e < todo + et; e += 128) {  // (the same number of turns for every thread)
-        const int col = e >> lg, rl = e & ((1 << lg) - 1);
-        const bool in = got && e < todo;
-        float r2 = 0.f;
-        if (in) {
-          // the splits' partial sums in rank order (all loads first)
-          const float* x0 = xs + (col << lg) + rl;
-          const int step = xcols << lg, up = p.xstage_cols << lg;
-          float pg[16], pu[16];
-#pragma unroll
-          for (int s = 0; s < 16; ++s) {
-            pg[s] = s < S ? x0[s * step] : 0.f;
-            pu[s] = (p.dual && s < S) ? x0[s * step + up] : 0.f;
+      const int rl = et & ((1 << lg) - 1), dc = 128 >> lg, n = n0 + (split << lg) + rl;
+      const int cols = min(TN, p.M), turns = (cols + dc - 1) / dc;  // (the same number of turns for every thread)
+      const float* x0 = (const float*)(gen + xoff) + et;
+      const int step = ((p.dual ? 2 : 1) * p.xstage_cols) << lg, up = p.xstage_cols << lg;
+      if (p.g_plus_one) gain += 1.f;
+      with_form(p, [&](auto form) {
+        constexpr int FORM = decltype(form)::value;
+        auto all = [&](auto ranks) {
+          constexpr int R = decltype(ranks)::value;
+          const float* x = x0;
+          int col = et >> lg;
+          int64_t o = (int64_t)col * p.ldo + n;
+          const int64_t dn = (int64_t)dc * p.ldo;
+          float res = res0, next = res1;
+#pragma unroll 1
+          for (int t = 0; t < turns; ++t, col += dc, o += dn, x += 128) {
+            const bool in = got && col < cols && n < p.N;
+            float r2 = 0.f, third = 0.f;
+            if (in) {
+              if ((FORM == FORM_NORM || FORM == FORM_RESIDUAL) && col + 2 * dc < cols) third = p.residual[o + 2 * dn];  // two turns ahead
+              const float g = add_ranks<R>(x, step);
+              const float u = FORM == FORM_DUAL ? add_ranks<R>(x + up, step) : 0.f;
+              r2 = finish<FORM>(p, col, n, o, g, u, parity, sc, res, gain);
+            }
+            res = next;
+            next = third;
+            if (FORM == FORM_NORM) {
+              if (lg <= 5) {
+                // a token's rows are neighbouring lanes
+                for (int i = 1 << lg >> 1; i; i >>= 1) r2 += __shfl_xor_sync(0xffffffffu, r2, i);
+                if (got && col < cols && rl == 0) p.ss_out[((int64_t)blockIdx.x * S + split) * 32 + col] = r2;
+              } else if (got && col < cols) {
+                sq[et + 128 * t] = r2;
+              }
+            }
           }
-          float g = 0.f, u = 0.f;
-#pragma unroll
-          for (int s = 0; s < 16; ++s) { g += pg[s]; u += pu[s]; }  // the zeros of absent ranks change nothing
-          const int n = n0 + (split << lg) + rl;
-          if (n < p.N) r2 = finish(p, col, n, g, u, parity, sc, e == et ? pre : Prefetched{false, 0.f, 0.f});
-        }
-        if (p.ss_out && lg <= 5) {
-          // a token's rows are neighbouring lanes
-          for (int o = 1 << lg >> 1; o; o >>= 1) r2 += __shfl_xor_sync(0xffffffffu, r2, o);
-          if (in && rl == 0) p.ss_out[((int64_t)blockIdx.x * S + split) * 32 + col] = r2;
-        } else if (p.ss_out && in) {
-          sq[e] = r2;
-        }
-      }
+        };
+        if (S == 16) all(std::integral_constant<int, 16>{});
+        else if (S == 8) all(std::integral_constant<int, 8>{});
+        else if (S == 4) all(std::integral_constant<int, 4>{});
+        else all(std::integral_constant<int, 2>{});
+      });
       if (p.ss_out && lg > 5) {
         asm volatile("bar.sync 2, 128;" ::: "memory");
         if (got && et < min(TN, p.M)) {

@@ -75,3 +75,10 @@ def test_recurrences(cuda_bf16, kind, dk, dv, taps):
 def test_post_norms_of_many_rows(cuda_bf16, hidden):
     """297 rows and more take the residual norms' form for prompts, the step the one for few rows."""
     check(cuda_bf16, shape(64, 2, 1, hidden, 256, 1, arch="gemma"), 3, [99, 120], 130, spread=1.0)
+
+
+@pytest.mark.parametrize("hidden,ffn", [(128, 256), (256, 640), (512, 1024), (1024, 2048), (2048, 1152)])
+@pytest.mark.parametrize("batch", [1, 4, 5, 8, 9, 16, 17, 31, 32])
+def test_projections_by_slices_and_tokens(cuda_bf16, hidden, ffn, batch):
+    """Clusters of 1 to 16 slices along k; 1 to 32 tokens, so a thread finishes 1 to 16 values of a row."""
+    check(cuda_bf16, shape(64, hidden // 64, max(1, hidden // 256), hidden, ffn, 2), batch, [3], 8, spread=1.0)
