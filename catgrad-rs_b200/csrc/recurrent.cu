@@ -498,7 +498,6 @@ __global__ void k_gated_norm(GatedNorm a) {
 template <class TG, class T, int V>
 __global__ void k_gated_norm_vec(GatedNorm a, int n, int units, int threads) {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-  asm volatile("griddepcontrol.wait;" ::: "memory");
   __shared__ float sh[32];
   const int per = blockDim.x / threads, sub = threadIdx.x / threads, t = threadIdx.x - sub * threads;
   const int64_t unit = blockIdx.x * (int64_t)per + sub;
@@ -508,7 +507,13 @@ __global__ void k_gated_norm_vec(GatedNorm a, int n, int units, int threads) {
   const float* o = a.o + m * (int64_t)a.H * a.dv + c0;
   const TG* gate = (const TG*)a.gate + m * a.ldg + c0;
   T* out = (T*)a.att + m * a.ld_att + c0;
-  float4 x[V], g[V];
+  float4 x[V], g[V], w[V];
+#pragma unroll
+  for (int j = 0; j < V; ++j) {  // the gains are weights: asked for before the dependency
+    const int i = 4 * (t + j * threads);
+    w[j] = live && i < n ? __ldg((const float4*)(a.norm + (a.shared_gain ? 0 : c0) + i)) : make_float4(0.f, 0.f, 0.f, 0.f);
+  }
+  asm volatile("griddepcontrol.wait;" ::: "memory");
   float ss = 0.f;
 #pragma unroll
   for (int j = 0; j < V; ++j) {
@@ -536,8 +541,7 @@ __global__ void k_gated_norm_vec(GatedNorm a, int n, int units, int threads) {
   for (int j = 0; j < V; ++j) {
     const int i = 4 * (t + j * threads);
     if (!live || i >= n) continue;
-    const float4 w = *(const float4*)(a.norm + (a.shared_gain ? 0 : c0) + i);
-    float4 r = make_float4(x[j].x * inv * w.x, x[j].y * inv * w.y, x[j].z * inv * w.z, x[j].w * inv * w.w);
+    float4 r = make_float4(x[j].x * inv * w[j].x, x[j].y * inv * w[j].y, x[j].z * inv * w[j].z, x[j].w * inv * w[j].w);
     if (!a.gate_first) { r.x *= g[j].x; r.y *= g[j].y; r.z *= g[j].z; r.w *= g[j].w; }
     st4(out + i, r);
   }
