@@ -281,6 +281,7 @@ k_rmsnorm_add_norm_vec(const float* y, const float* g1, const float* g2, float e
   float s2 = 0.f;
 #pragma unroll
   for (int j = 0; j < VECS; ++j) {
+    if (j * threads >= n4) break;  // (for every thread: dividing for vectors that no thread has cost 1.7 % of a Gemma-2-2B pass)
     if (!STEP) a[j] = gain(g1, j);
     u[j].x += v[j].x / rms1 * (one + a[j].x);
     u[j].y += v[j].y / rms1 * (one + a[j].y);
