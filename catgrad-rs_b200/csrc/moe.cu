@@ -243,9 +243,70 @@ k_moe_norm_split_vec(const float* x, const float* gamma, float eps, int plus_one
 // and weighted by probability.  Dynamic shared memory: E floats per warp, 2 E with correction.
 constexpr uint32_t TAKEN = 0xFFFFFFFFu;  // a chosen expert's mark (a NaN no sum here produces)
 // Lane r < k receives the expert of slot r and its weight; pr: the warp's shared memory.
-__device__ __forceinline__ void topk_of_row(const float* lg, int E, int k, int norm_topk, int sigmoid, const float* correction, float scale,
-                                            float* pr, uint32_t* id, float* weight) {
+// `corr`: the corrections of experts lane + 32 i (load_corrections).
+// Up to ONE_PASS experts a lane keeps its four candidates in registers, and a round is two warp reductions (the largest
+// key, then the lowest expert that has it) instead of ten shuffles of 64-bit pairs between reads of shared memory.  Us per launch of k_moe_topk_plan,
+// 128 experts, 8 choices: 8 corrected rows 7.8 -> 4.2, one row 5.8 -> 4.2.
+constexpr int ONE_PASS = 128;
+__device__ __forceinline__ void load_corrections(const float* correction, int E, float* corr) {
   const int lane = threadIdx.x & 31;
+#pragma unroll
+  for (int i = 0; i < ONE_PASS / 32; ++i) corr[i] = correction && lane + 32 * i < E ? __ldg(correction + lane + 32 * i) : 0.f;
+}
+// unsigned order = float order, whatever the signs; never 0 (that would take the bits of TAKEN)
+__device__ __forceinline__ uint32_t order_key(float v) {
+  const uint32_t u = __float_as_uint(v);
+  return u & 0x80000000u ? ~u : u | 0x80000000u;
+}
+__device__ __forceinline__ void topk_of_row(const float* lg, int E, int k, int norm_topk, int sigmoid, const float* correction, float scale,
+                                            float* pr, uint32_t* id, float* weight, const float* corr) {
+  const int lane = threadIdx.x & 31;
+  if (E <= ONE_PASS) {
+    float v[ONE_PASS / 32], mx = -3.4028234663852886e38f, sum = 0.f;
+#pragma unroll
+    for (int i = 0; i < ONE_PASS / 32; ++i) {
+      v[i] = lane + 32 * i < E ? lg[lane + 32 * i] : -INFINITY;
+      mx = fmaxf(mx, v[i]);
+    }
+    for (int o = 16; o; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+#pragma unroll
+    for (int i = 0; i < ONE_PASS / 32; ++i)
+      if (lane + 32 * i < E) {
+        v[i] = sigmoid ? 1.f / (1.f + expf(-v[i])) : expf(v[i] - mx);
+        sum += v[i];
+      }
+    for (int o = 16; o; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+    uint32_t key[ONE_PASS / 32];
+#pragma unroll
+    for (int i = 0; i < ONE_PASS / 32; ++i) {
+      key[i] = 0u;
+      if (lane + 32 * i < E) {
+        if (!sigmoid) v[i] = v[i] / sum;
+        pr[lane + 32 * i] = v[i];
+        key[i] = order_key(correction ? v[i] + corr[i] : v[i]);
+      }
+    }
+    __syncwarp();
+    float chosen = 0.f;
+    uint32_t chosen_id = 0;
+    for (int r = 0; r < k; ++r) {
+      uint32_t best = 0u;
+      int at = 0;
+#pragma unroll
+      for (int i = 0; i < ONE_PASS / 32; ++i)
+        if (key[i] > best) { best = key[i]; at = i; }
+      const uint32_t top = __reduce_max_sync(0xffffffffu, best);
+      const uint32_t e = min(__reduce_min_sync(0xffffffffu, best == top ? (uint32_t)(lane + 32 * at) : 0xFFFFFFFFu), (uint32_t)E - 1u);
+      if (lane == r) { chosen = pr[e]; chosen_id = e; }
+#pragma unroll
+      for (int i = 0; i < ONE_PASS / 32; ++i)
+        if (e == (uint32_t)(lane + 32 * i)) key[i] = 0u;
+    }
+    const float total = sum_in_reference_order(chosen, k);  // bit-identical to the reference's sum over the k values
+    *id = chosen_id;
+    *weight = (norm_topk ? chosen / total : chosen) * scale;
+    return;
+  }
   float* ch = correction ? pr + E : pr;  // what the choice goes by
   float mx = -3.4028234663852886e38f;
   for (int e = lane; e < E; e += 32) {
@@ -272,10 +333,8 @@ __device__ __forceinline__ void topk_of_row(const float* lg, int E, int k, int n
   for (int r = 0; r < k; ++r) {
     unsigned long long best = 0;
     for (int e = lane; e < E; e += 32) {
-      const uint32_t u = __float_as_uint(ch[e]);
-      if (u == TAKEN) continue;
-      // unsigned order = float order, whatever the signs
-      const uint32_t key = u & 0x80000000u ? ~u : u | 0x80000000u;
+      if (__float_as_uint(ch[e]) == TAKEN) continue;
+      const uint32_t key = order_key(ch[e]);
       const unsigned long long q = ((unsigned long long)key << 32) | (uint32_t)(0xFFFFFFFFu - (uint32_t)e);
       best = q > best ? q : best;
     }
@@ -296,6 +355,8 @@ __device__ __forceinline__ void topk_of_row(const float* lg, int E, int k, int n
 __global__ void k_moe_topk(const float* logits, int64_t M, int E, int k, int norm_topk, int sigmoid, const float* correction,
                            float scale, uint32_t* ids, float* wts) {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  float corr[ONE_PASS / 32];
+  load_corrections(correction, E, corr);
   asm volatile("griddepcontrol.wait;" ::: "memory");
   extern __shared__ float sm[];
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
@@ -303,7 +364,7 @@ __global__ void k_moe_topk(const float* logits, int64_t M, int E, int k, int nor
   if (m >= M) return;
   uint32_t id;
   float w;
-  topk_of_row(logits + m * E, E, k, norm_topk, sigmoid, correction, scale, sm + (size_t)wid * E * (correction ? 2 : 1), &id, &w);
+  topk_of_row(logits + m * E, E, k, norm_topk, sigmoid, correction, scale, sm + (size_t)wid * E * (correction ? 2 : 1), &id, &w, corr);
   if (lane < k) {
     ids[m * k + lane] = id;
     wts[m * k + lane] = w;
@@ -382,6 +443,8 @@ k_moe_topk_plan(const float* logits, int M, int E, int k, int norm_topk, int sig
                 uint32_t* ids, float* wts, int e_lo, int El, int tn, int32_t* pos, int32_t* tile_expert, int32_t* tile_row0,
                 int32_t* tile_rows, int32_t* n_tiles) {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  float corr[ONE_PASS / 32];
+  load_corrections(correction, E, corr);  // (weights: before the dependency)
   asm volatile("griddepcontrol.wait;" ::: "memory");
   extern __shared__ float sm[];
   int* sh_i = (int*)sm;                          // [2 El] the plan's
@@ -391,7 +454,7 @@ k_moe_topk_plan(const float* logits, int M, int E, int k, int norm_topk, int sig
   if (m < M) {
     uint32_t id;
     float w;
-    topk_of_row(logits + (int64_t)m * E, E, k, norm_topk, sigmoid, correction, scale, pr + (size_t)m * E * (correction ? 2 : 1), &id, &w);
+    topk_of_row(logits + (int64_t)m * E, E, k, norm_topk, sigmoid, correction, scale, pr + (size_t)m * E * (correction ? 2 : 1), &id, &w, corr);
     if (lane < k) {
       ids[m * k + lane] = chosen[m * k + lane] = id;
       wts[m * k + lane] = w;

@@ -73,6 +73,14 @@ def test_fused_moe_choice_and_plan(oracle, cuda_bf16, S, H, E, Fe, k):
     test_fused_moe_matches_op_stream(oracle, cuda_bf16, S, H, E, Fe, k, True)
 
 
+# candidates in a lane's registers up to 128 experts, in shared memory above; few and all of them chosen
+@pytest.mark.gpu
+@pytest.mark.parametrize("E,k", [(1, 1), (2, 2), (31, 31), (32, 8), (33, 32), (96, 3), (127, 8), (128, 8), (128, 32), (129, 8)])
+@pytest.mark.parametrize("S", [3, 40])
+def test_fused_moe_choice_of_experts(oracle, cuda_bf16, S, E, k):
+    test_fused_moe_matches_op_stream(oracle, cuda_bf16, S, 64, E, 8, k, True)
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("S,H,E,Fe,k,renorm", [CASES[1], CASES[5]])
 def test_fused_moe_f32_router(oracle, cuda, S, H, E, Fe, k, renorm):
