@@ -247,6 +247,21 @@ k_gemm_tcp2(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ C
     for (int t = pair; t < total_tiles && ok; t += pairs, ++ti) {
       const uint32_t buf = (uint32_t)ti & 1u;
       const int m0 = (t % p.m_tiles) * P2_TOK, m_end = p.M;
+      // The residual of 32 tokens is asked for a round ahead, that of the first while the tile is still multiplied: with
+      // K = 2048 a tile's residuals, read where they are added, take as long as the tile.
+      // 5057 tokens, 2048 x 2048: 77 -> 64 us; 2048 x 8192: 184 -> 178; a prompt batch of 13 x 389 tokens 16.6 -> 16.2 ms.  (Tiles
+      // of 192 and 128 tokens, which fill the last round of 74 pairs better, are slower: 83 and 97 us for 77 and 64.)
+      float ra[GLU ? 1 : 32], rb[GLU ? 1 : 32];
+      auto ask = [&](float* r, int c0) {
+        if constexpr (!GLU) {
+          const int n = (t / p.m_tiles) * P2_ROWS + (int)rank * 128 + row;
+          const float* from = p.residual + (int64_t)(m0 + c0) * p.ldo + n;
+#pragma unroll
+          for (int j = 0; j < 32; ++j)
+            if (n < p.N && m0 + c0 + j < m_end) asm volatile("ld.global.f32 %0, [%1];" : "=f"(r[j]) : "l"(from + (int64_t)j * p.ldo) : "memory");
+        }
+      };
+      if (!GLU && p.out_mode == 2) ask(ra, col0);
       ok = mbar_wait(bar_acc_full + 8 * buf, ((uint32_t)ti >> 1) & 1u, cta_abort, p.err);
       if (!ok) break;
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -289,18 +304,12 @@ k_gemm_tcp2(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ C
       } else {
         const int n = (t / p.m_tiles) * P2_ROWS + (int)rank * 128 + row;
         const bool live = n < p.N;
-        auto round = [&](const uint32_t* cur, uint32_t* nxt, int c0) {
+        auto round = [&](const uint32_t* cur, uint32_t* nxt, const float* res, float* res_nxt, int c0) {
           if (c0 + 32 < col0 + P2_TOK / 2) tmem_ld32(acc + (uint32_t)(c0 + 32), nxt);
+          // (out may alias residual: an element is read a round before it is written, by the thread that writes it)
+          if (p.out_mode == 2 && c0 + 32 < col0 + P2_TOK / 2) ask(res_nxt, c0 + 32);
           if (live) {
             if (p.out_mode == 2) {
-              // out may alias residual: all loads of the round before its stores (and all 32 in
-              // flight together)
-              float res[32];
-#pragma unroll
-              for (int j = 0; j < 32; ++j) {
-                const int m = m0 + c0 + j;
-                res[j] = m < m_end ? p.residual[(int64_t)m * p.ldo + n] : 0.f;
-              }
 #pragma unroll
               for (int j = 0; j < 32; ++j) {
                 const int m = m0 + c0 + j;
@@ -333,8 +342,8 @@ k_gemm_tcp2(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ C
 #pragma unroll 1
         for (int c0 = col0; c0 < col0 + P2_TOK / 2; c0 += 64) {
           if (m0 + c0 >= m_end) break;
-          round(va, vb, c0);
-          round(vb, va, c0 + 32);
+          round(va, vb, ra, rb, c0);
+          round(vb, va, rb, ra, c0 + 32);
         }
       }
       // this buffer may be overwritten once the four warps of both CTAs have read it

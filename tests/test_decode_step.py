@@ -42,10 +42,10 @@ EDGES = [1, 15, 16, 31, 32, 33, 63, 64, 127, 128, 129, 255, 256, 300]
 
 
 @pytest.mark.parametrize("D,nh,nkv", [(64, 1, 1), (64, 6, 2), (64, 8, 1), (128, 2, 2), (128, 8, 1), (256, 2, 1), (256, 8, 1)])
-@pytest.mark.parametrize("batch,max_seq", [(1, 310), (1, 4200), (2, 600), (40, 310)])
+@pytest.mark.parametrize("batch,max_seq", [(1, 310), (1, 4200), (2, 600), (40, 310), (230, 310)])
 def test_attention_edges(cuda_bf16, D, nh, nkv, batch, max_seq):
-    """1 to 16 slices of the context, most of them empty where the context is short."""
-    check(cuda_bf16, shape(D, nh, nkv), batch, EDGES if batch < 40 else [1, 33, 129, 300], max_seq)
+    """1 to 16 slices of the context, most of them empty where the context is short; few CTAs and more than fit at once."""
+    check(cuda_bf16, shape(D, nh, nkv), batch, EDGES if batch < 40 else [1, 15, 16, 33, 65, 129, 300], max_seq)
 
 
 @pytest.mark.parametrize("D,cap,window", [(64, 0.0, 40), (128, 0.0, 129), (256, 30.0, 0), (256, 50.0, 100)])
