@@ -47,25 +47,38 @@ class TaggedTensor:
     """A backend tensor with its dtype tag (interpreter/types.rs:15-98).  Owns one
     reference to the library handle; copying the Python object shares it."""
 
-    __slots__ = ("_b", "_h", "dtype")
+    __slots__ = ("_b", "_h", "_dtype", "_shape")
 
-    def __init__(self, backend: "TraitBackend", handle, dtype: int):
+    # dtype and shape are the library's, and never change.  Most results of an op stream are only passed on, so they are
+    # asked for when they are read, and then once (a prompt of 61 tokens through the trait methods: 2.24 -> 2.00 ms).
+    def __init__(self, backend: "TraitBackend", handle, dtype: int | None = None):
         self._b = backend
         self._h = handle
-        self.dtype = dtype
+        self._dtype = dtype
+        self._shape = None
+
+    @property
+    def dtype(self) -> int:
+        if self._dtype is None:
+            d = C.c_int32()
+            self._b._f("dtype_of")(self._h, C.byref(d))
+            self._dtype = d.value
+        return self._dtype
 
     @property
     def shape(self) -> tuple[int, ...]:
         """BackendTensorOps::shape (backend/mod.rs:84-86): host metadata, no sync."""
-        rank = C.c_int32()
-        dims = (C.c_int64 * 8)()
-        self._b._f("shape")(self._h, C.byref(rank), dims)
-        return tuple(dims[i] for i in range(rank.value))
+        if self._shape is None:
+            rank = C.c_int32()
+            dims = (C.c_int64 * 8)()
+            self._b._f("shape")(self._h, C.byref(rank), dims)
+            self._shape = tuple(dims[:rank.value])
+        return self._shape
 
     def __del__(self):
         try:
             if self._h is not None:
-                self._b._f("tensor_release")(self._h)
+                self._b._release(self._h)
                 self._h = None
         except Exception:
             pass
@@ -134,6 +147,7 @@ class TraitBackend:
             fn = self._f(name)
             fn.argtypes = args
             fn.restype = res
+        self._release = self._f("tensor_release")
 
     def _err(self) -> str:
         msg = self._f("last_error")(self._ctx)
@@ -144,16 +158,14 @@ class TraitBackend:
             raise BackendPanic(status, self._err())
 
     def _wrap(self, handle, dtype: int | None = None) -> TaggedTensor:
-        if dtype is None:
-            d = C.c_int32()
-            self._f("dtype_of")(handle, C.byref(d))
-            dtype = d.value
         return TaggedTensor(self, handle, dtype)
 
     def _out1(self, name: str, *args) -> TaggedTensor:
         h = _c_vp()
-        self._check(self._f(name)(self._ctx, *args, C.byref(h)))
-        return self._wrap(h)
+        status = self._f(name)(self._ctx, *args, C.byref(h))
+        if status != 0:
+            self._check(status)
+        return TaggedTensor(self, h)
 
     # -- trait methods (backend/mod.rs line in the comment) -----------------------
     def zeros(self, shape, target_dtype) -> TaggedTensor:  # :26
