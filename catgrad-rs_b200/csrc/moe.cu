@@ -593,6 +593,7 @@ k_moe_combine_norm(const float* y, const int32_t* pos, const float* wts, int k, 
   }
 }
 
+constexpr uint32_t MOE_BAR_BYTES = 256;  // barriers, TMEM address and abort flag of the split form
 struct MoeGemmArgs {
   const int32_t* tile_expert;
   const int32_t* tile_row0;
@@ -613,7 +614,13 @@ struct MoeGemmArgs {
 // tensor-core GEMM: warp 0 lane 0 loads with TMA, warp 1 lane 0 issues the MMAs, warps 2-5
 // read the accumulators back.  DUAL keeps two accumulators (gate in TMEM columns [0, TN), up
 // in [TN, 2 TN)) fed by the same activation tile.
-template <int TN, int DUAL, int STAGES, int MINB>
+//
+// SPLIT (DUAL, TN 16): where a step has so few tiles that they leave most SMs idle, the CTAs of a cluster (grid z, 2 or 4) take
+// a part of k each, push their accumulators (st.async, counted by an mbarrier) to the CTA that finishes the row and
+// add them in rank order, as the decode GEMM does.  An SM takes in some 44 GB/s however deep its ring, so 48 CTAs
+// stream at 2.1 TB/s.  One row, 8 experts of 768 x 2048: 18.4 -> 12.9 us, four layers of the Qwen3-30B-A3B shape 357 -> 336 us a
+// step.  (Three ring stages leave one CTA per SM, and 192 CTAs take two waves: 16.4 us.)
+template <int TN, int DUAL, int STAGES, int MINB, int SPLIT = 0>
 __global__ void __launch_bounds__(192, MINB)
 k_moe_gemm(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_u,
            const __grid_constant__ CUtensorMap map_x, MoeGemmArgs p) {
@@ -644,7 +651,10 @@ k_moe_gemm(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CU
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int n0 = blockIdx.x * BM;
   const int wrow = expert * p.w_rows + n0;
-  const int nkb = p.kb_total;
+  const int splits = SPLIT ? gridDim.z : 1, split = SPLIT ? blockIdx.z : 0;
+  const int kb0 = split * p.kb_total / splits, nkb = (split + 1) * p.kb_total / splits - kb0;
+  const uint32_t bar_x = bars + 64 + 16 * STAGES;  // SPLIT: every addend of this CTA's rows has arrived
+  constexpr uint32_t XOFF = STAGES * STAGE_BYTES + MOE_BAR_BYTES;  // [splits][2][TN][128 / splits] f32
 
   if (tid == 0) {
     for (int s = 0; s < STAGES; ++s) {
@@ -652,6 +662,10 @@ k_moe_gemm(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CU
       mbar_init(bars + 8 * (STAGES + s), 1);  // empty[s]: one tcgen05.commit
     }
     mbar_init(bar_accum, 1);
+    if (SPLIT) {
+      mbar_init(bar_x, 1);
+      mbar_expect_tx(bar_x, (uint32_t)(2 * min(rows, TN)) * BM * 4u);
+    }
     *cta_abort = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -660,8 +674,8 @@ k_moe_gemm(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CU
       const uint32_t full = bars + 8 * i;
       const uint32_t a = base + i * STAGE_BYTES;
       mbar_expect_tx(full, W_BYTES);
-      tma_load_2d(a, &map_w, i * BK, wrow, full);
-      if (DUAL) tma_load_2d(a + A_BYTES, &map_u, i * BK, wrow, full);
+      tma_load_2d(a, &map_w, (kb0 + i) * BK, wrow, full);
+      if (DUAL) tma_load_2d(a + A_BYTES, &map_u, (kb0 + i) * BK, wrow, full);
     }
   }
   if (warp == 1) {
@@ -674,6 +688,8 @@ k_moe_gemm(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CU
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem_acc = *tmem_slot;
+  // the peers' barriers exist once they have arrived here; waited for just before the pushes
+  if (SPLIT) asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
 
   bool acc_ok = false;
   if (warp == 0) {
@@ -684,7 +700,7 @@ k_moe_gemm(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CU
         const int s = i % STAGES;
         const uint32_t full = bars + 8 * s;
         const uint32_t a = base + s * STAGE_BYTES;
-        const int k = i * BK;
+        const int k = (kb0 + i) * BK;
         if (i >= pre) {
           const uint32_t ph = (uint32_t)(i / STAGES) & 1u;
           if (!mbar_wait(bars + 8 * (STAGES + s), ph ^ 1u, cta_abort, p.err)) break;
@@ -731,7 +747,49 @@ k_moe_gemm(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CU
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   }
 
-  if (warp >= 2 && acc_ok) {
+  if constexpr (SPLIT != 0) {
+    __syncwarp();
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+    const int lg = splits == 4 ? 5 : 6, cols = min(rows, TN);  // log2 of the rows that a CTA finishes; tokens
+    if (warp >= 2) {
+      // (a CTA whose accumulator never came pushes all the same: its peers count on the bytes, and the error word is set)
+      const int q = warp & 3, row = q * 32 + lane;
+      uint32_t g[16], u[16], xdst, xbar;
+      asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(xdst) : "r"(base + XOFF), "r"(row >> lg));
+      asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(xbar) : "r"(bar_x), "r"(row >> lg));
+      xdst += (uint32_t)(((split * 2 * TN) << lg) + (row & ((1 << lg) - 1))) * 4u;
+      tmem_ld16(tmem_acc + ((uint32_t)(q * 32) << 16), g);
+      tmem_ld16(tmem_acc + ((uint32_t)(q * 32) << 16) + (uint32_t)TN, u);
+      asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+      auto push = [&](uint32_t to, uint32_t v) {
+        asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.b32 [%0], %1, [%2];" ::"r"(to), "r"(v), "r"(xbar) : "memory");
+      };
+#pragma unroll
+      for (int j = 0; j < 16; ++j) {
+        if (j >= cols) break;
+        push(xdst + ((uint32_t)j << (lg + 2)), g[j]);
+        push(xdst + ((uint32_t)(TN + j) << (lg + 2)), u[j]);
+      }
+    }
+    // Arrived when every CTA has issued its pushes; waited for before this CTA leaves, so that no push can find its
+    // target gone even where a wait has given up.
+    __syncwarp();
+    asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
+    if (warp >= 2 && mbar_wait_cluster(bar_x, 0, cta_abort, p.err) && !*cta_abort) {
+      const int et = tid - 64, n = n0 + (split << lg) + (et & ((1 << lg) - 1));
+      const int step = (2 * TN) << lg, up = TN << lg;
+      const float* xs = (const float*)(gen + XOFF) + et;  // token et >> lg, this row
+      if (n < p.N)
+        for (int c = et >> lg; c < cols; c += 128 >> lg, xs += 128) {
+          float a = 0.f, b = 0.f;
+          for (int s = 0; s < splits; ++s) { a += xs[s * step]; b += xs[s * step + up]; }
+          ((__nv_bfloat16*)p.out)[(int64_t)(row0 + c) * p.ldo + n] = __float2bfloat16_rn(glu_f(p.act, p.limit, a, b));
+        }
+    }
+    __syncwarp();
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+    if (*cta_abort) mbar_drain(bar_x, 0, p.err);  // (issued is not arrived)
+  } else if (warp >= 2 && acc_ok) {
     const int q = warp & 3;
     const int n = n0 + q * 32 + lane;
     const uint32_t lane_addr = tmem_acc + ((uint32_t)(q * 32) << 16);
@@ -855,17 +913,18 @@ __global__ void __launch_bounds__(256) k_moe_gemm_f32(MoeF32Args p) {
     }
 }
 
-template <int TN, int DUAL, int STAGES, int MINB>
+template <int TN, int DUAL, int STAGES, int MINB, int SPLIT = 0>
 int launch_moe_gemm(cg_ctx* c, const CUtensorMap& mw, const CUtensorMap& mu, const CUtensorMap& mx, const MoeGemmArgs& a,
                     dim3 grid) {
-  constexpr size_t smem = (size_t)STAGES * (A_BYTES * (DUAL ? 2 : 1) + TN * BK * 2) + 1024 + 16 * STAGES + 64;
+  constexpr size_t smem = (size_t)STAGES * (A_BYTES * (DUAL ? 2 : 1) + TN * BK * 2) + 1024 +
+                          (SPLIT ? MOE_BAR_BYTES + 2 * TN * BM * 4 : 16 * STAGES + 64);
   static PerDeviceFlag configured_on;
   bool& configured = configured_on.at(c->core->device);
   if (!configured) {
-    CG_CUDA(c, cudaFuncSetAttribute(k_moe_gemm<TN, DUAL, STAGES, MINB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    CG_CUDA(c, cudaFuncSetAttribute(k_moe_gemm<TN, DUAL, STAGES, MINB, SPLIT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     configured = true;
   }
-  CG_CUDA(c, launch_kernel(c, k_moe_gemm<TN, DUAL, STAGES, MINB>, grid, dim3(192), smem, 1, mw, mu, mx, a));
+  CG_CUDA(c, launch_kernel(c, k_moe_gemm<TN, DUAL, STAGES, MINB, SPLIT>, grid, dim3(192), smem, (int)grid.z, mw, mu, mx, a));
   CG_LAUNCHED(c);
   return CG_OK;
 }
@@ -1053,7 +1112,15 @@ int moe_experts(cg_ctx* c, const MoeArgs& a) {
   };
   if (!gated) CG_TRY(single());
   else switch (tn) {
-    case 16: CG_TRY((launch_moe_gemm<16, 1, 3, 2>(c, mw, mu, mx, g, grid))); break;
+    case 16: {
+      // few tiles: k in 2 or 4 parts, up to two CTAs for every SM, four k blocks or more for each
+      unsigned splits = 1;
+      while (splits < 4 && (int64_t)grid.x * grid.y * splits * 2 <= 2 * 148 && g.kb_total / (int)(splits * 2) >= 4) splits *= 2;
+      grid.z = splits;
+      if (splits > 1) CG_TRY((launch_moe_gemm<16, 1, 2, 2, 1>(c, mw, mu, mx, g, grid)));
+      else CG_TRY((launch_moe_gemm<16, 1, 3, 2>(c, mw, mu, mx, g, grid)));
+      break;
+    }
     case 32: CG_TRY((launch_moe_gemm<32, 1, 3, 1>(c, mw, mu, mx, g, grid))); break;
     case 64: CG_TRY((launch_moe_gemm<64, 1, 4, 1>(c, mw, mu, mx, g, grid))); break;
     default: CG_TRY((launch_moe_gemm<128, 1, 4, 1>(c, mw, mu, mx, g, grid))); break;

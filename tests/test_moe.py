@@ -81,6 +81,14 @@ def test_fused_moe_choice_of_experts(oracle, cuda_bf16, S, E, k):
     test_fused_moe_matches_op_stream(oracle, cuda_bf16, S, 64, E, 8, k, True)
 
 
+# few tiles: k in two and four parts, k blocks that do not divide evenly, ragged features, several rows of one expert
+@pytest.mark.gpu
+@pytest.mark.parametrize("S,H,E,Fe,k", [(1, 512, 8, 96, 2), (1, 1024, 16, 200, 4), (2, 1088, 8, 328, 8), (1, 1160, 4, 8, 4), (5, 1024, 1, 136, 1),
+                                        (16, 1024, 1, 264, 1), (3, 2048, 128, 768, 8), (7, 576, 2, 1000, 1)])
+def test_fused_moe_parts_of_k(oracle, cuda_bf16, S, H, E, Fe, k):
+    test_fused_moe_matches_op_stream(oracle, cuda_bf16, S, H, E, Fe, k, True)
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("S,H,E,Fe,k,renorm", [CASES[1], CASES[5]])
 def test_fused_moe_f32_router(oracle, cuda, S, H, E, Fe, k, renorm):
