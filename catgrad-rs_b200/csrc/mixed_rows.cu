@@ -47,24 +47,26 @@ __device__ __forceinline__ float4 gains_of(const float* g, int i, int W) {
     return make_float4(t[0], t[1], t[2], t[3]);
   }
 }
-// v += the sum, in order, over a token's slots of weight * expert's row; absent experts (-1) are left out.  Eight slots
+// v += the sum, in order, over a token's slots of weight * expert's row; absent experts (-1) are left out.  SLOTS of them
 // at a time: their places and weights in one trip, their rows in the next, where one slot after the other took two
-// trips each.  (With the choice of experts in moe.cu: Segedra rows 49.0 -> 47.8 ms per pass.)
+// trips each.  (Eight, with the choice of experts in moe.cu: Segedra rows 49.0 -> 47.8 ms per pass.  They hold 48 registers,
+// which a block of 1024 threads does not have.)
+template <int SLOTS>
 __device__ __forceinline__ void add_experts(const float* y, int64_t ldy, const int32_t* pos, const float* wts, int top, int col, float* v) {
-  for (int q0 = 0; q0 < top; q0 += 8) {
-    int r[8];
-    float w[8];
-    float4 x[8];
+  for (int q0 = 0; q0 < top; q0 += SLOTS) {
+    int r[SLOTS];
+    float w[SLOTS];
+    float4 x[SLOTS];
 #pragma unroll
-    for (int q = 0; q < 8; ++q) {
+    for (int q = 0; q < SLOTS; ++q) {
       r[q] = q0 + q < top ? pos[q0 + q] : -1;
       w[q] = wts && q0 + q < top ? wts[q0 + q] : 1.f;
     }
 #pragma unroll
-    for (int q = 0; q < 8; ++q)
+    for (int q = 0; q < SLOTS; ++q)
       if (r[q] >= 0) x[q] = *(const float4*)(y + (int64_t)r[q] * ldy + col);
 #pragma unroll
-    for (int q = 0; q < 8; ++q)
+    for (int q = 0; q < SLOTS; ++q)
       if (r[q] >= 0) { v[0] += w[q] * x[q].x; v[1] += w[q] * x[q].y; v[2] += w[q] * x[q].z; v[3] += w[q] * x[q].w; }
   }
 }
@@ -119,7 +121,7 @@ __device__ __forceinline__ void norm_row(float (*v)[4], int centred, float eps, 
 
 // One block per row; the row lives in registers (RU_VEC 128-bit vectors per thread).
 // EXACT: W is a multiple of 8, so no column is padding and gains and table rows are read as vectors.
-template <class T, int RU_VEC, bool EXACT>
+template <class T, int RU_VEC, bool EXACT, int SLOTS = 8>
 __global__ void k_row_update(RowUpdate u, int32_t* err) {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   __shared__ float sh[32];
@@ -172,7 +174,7 @@ __global__ void k_row_update(RowUpdate u, int32_t* err) {
             const float4 t = *(const float4*)(u.y + m * u.ldy + 4 * i);
             v[j][0] = t.x; v[j][1] = t.y; v[j][2] = t.z; v[j][3] = t.w;
           }
-          if (RU_VEC == 1 && u.top) add_experts(u.ye, u.ldye, u.pos + m * u.top, u.wts ? u.wts + m * u.top : nullptr, u.top, 4 * i, v[j]);
+          if (RU_VEC == 1 && u.top) add_experts<SLOTS>(u.ye, u.ldye, u.pos + m * u.top, u.wts ? u.wts + m * u.top : nullptr, u.top, 4 * i, v[j]);
           for (int q = 0; RU_VEC > 1 && q < u.top; ++q) {
             const int r = u.pos[m * u.top + q];
             if (r < 0) continue;
@@ -216,7 +218,7 @@ __global__ void k_row_update(RowUpdate u, int32_t* err) {
 
 // One block per token.  Vector i of all streams is read, mixed and written by one thread, which keeps
 // its part of the next sublayer's input (VEC 128-bit vectors) for the norm.  NS bounds the streams.
-template <class T, int NS, int VEC, bool EXACT>
+template <class T, int NS, int VEC, bool EXACT, int SLOTS = 8>
 __global__ void k_stream_update(StreamUpdate u, int32_t* err) {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   __shared__ float sh[32];
@@ -283,7 +285,7 @@ __global__ void k_stream_update(StreamUpdate u, int32_t* err) {
           for (int e = 0; e < 4; ++e) x[t][e] = old[t][e];
       } else {
         if (u.top && VEC == 1) {
-          add_experts(u.y, u.ldy, u.pos + m * u.top, u.wts + m * u.top, u.top, 4 * i, y);
+          add_experts<SLOTS>(u.y, u.ldy, u.pos + m * u.top, u.wts + m * u.top, u.top, 4 * i, y);
         } else if (u.top) {
           for (int q = 0; q < u.top; ++q) {
             const int r = u.pos[m * u.top + q];
@@ -388,49 +390,69 @@ __global__ void k_pair_rope_tables(PairRope f, int64_t T, int r, float* cos_t, f
 
 }  // namespace
 
+// Threads a block of a kernel may have: its registers have to fit an SM.
+template <auto KERNEL>
+static int largest_block(cg_ctx* c) {
+  static PerDeviceSize known;
+  size_t& threads = known.at(c->core->device);
+  cudaFuncAttributes a;
+  if (!threads && cudaFuncGetAttributes(&a, KERNEL) == cudaSuccess) threads = (size_t)a.maxThreadsPerBlock;
+  return (int)threads;
+}
+
+// One block per row.  Few rows take the form with most threads, one vector each, if its registers fit so wide a block: with
+// eight experts' slots at a time they do up to 640 threads (plain rows, up to 2 streams), 512 (up to 8) and 256 (16), with
+// four slots (V1_WIDE) up to 1024, 896 (4 streams) and 640 (8).  Us of a decode step with the four-slot form, and with the
+// two-vector form in its place: Ralapel shape, 4096 wide, one row 1208, 1272, eight 1388, 1435; Segedra, 2880 wide, 4 streams, one row 1097,
+// 1189; Regupel, 2880 wide, one row 1100, 1124; Kivorax, 3072 wide, one row 939, 945.  Many rows share an SM: two vectors each, four
+// above 8192 values or where two do not fit.
+template <auto V1, auto V1_WIDE, auto V2, auto V4, class U>
+static int launch_rows(cg_ctx* c, const U& u, int64_t M) {
+  const int n4 = (u.W + 7) / 8 * 2;
+  auto launch = [&](auto kernel, int block) -> int {
+    CG_CUDA(c, launch_kernel(c, kernel, dim3((unsigned)M), dim3(block), 0, 1, u, c->core->dev_err));
+    CG_LAUNCHED(c);
+    return CG_OK;
+  };
+  auto block = [&](int vec) { return ((n4 + vec - 1) / vec + 31) / 32 * 32; };
+  if (M <= 296 && block(1) <= largest_block<V1>(c)) return launch(V1, block(1));
+  if (M <= 296 && block(1) <= largest_block<V1_WIDE>(c)) return launch(V1_WIDE, block(1));
+  if (n4 <= (M <= 296 ? 1024 : 2048) && block(2) <= largest_block<V2>(c)) return launch(V2, block(2));
+  if (block(4) <= largest_block<V4>(c)) return launch(V4, block(4));
+  return fail(c, CG_ERR_UNSUPPORTED, block(4) > 1024 ? "decoder: rows wider than 16384 are not supported"
+                                                     : "decoder: rows this wide are not supported with so many streams");
+}
+
 int k_launch_row_update(cg_ctx* c, const RowUpdate& u, int64_t M, int out_bf16) {
   if (M == 0) return CG_OK;
-  const int n4 = (u.W + 7) / 8 * 2;
-  const bool exact = u.W % 8 == 0;
-  const int vec = M <= 296 ? (n4 <= 1024 ? 1 : 4) : n4 <= 2048 ? 2 : 4;
-  const int block = ((n4 + vec - 1) / vec + 31) / 32 * 32;
-  if (block > 1024) return fail(c, CG_ERR_UNSUPPORTED, "decoder: rows wider than 16384 are not supported");
-  auto pick = [&](auto t) {
+  auto pick = [&](auto t, auto exact) {
     using T = decltype(t);
-    if (exact) return vec == 1 ? k_row_update<T, 1, true> : vec == 2 ? k_row_update<T, 2, true> : k_row_update<T, 4, true>;
-    return vec == 1 ? k_row_update<T, 1, false> : vec == 2 ? k_row_update<T, 2, false> : k_row_update<T, 4, false>;
+    constexpr bool E = decltype(exact)::value;
+    return launch_rows<k_row_update<T, 1, E>, k_row_update<T, 1, E, 4>, k_row_update<T, 2, E>, k_row_update<T, 4, E>>(c, u, M);
   };
-  auto kernel = out_bf16 ? pick(__nv_bfloat16()) : pick(float());
-  CG_CUDA(c, launch_kernel(c, kernel, dim3((unsigned)M), dim3(block), 0, 1, u, c->core->dev_err));
-  CG_LAUNCHED(c);
-  return CG_OK;
+  if (u.W % 8 == 0) return out_bf16 ? pick(__nv_bfloat16(), std::true_type()) : pick(float(), std::true_type());
+  return out_bf16 ? pick(__nv_bfloat16(), std::false_type()) : pick(float(), std::false_type());
 }
 
 int k_launch_stream_update(cg_ctx* c, const StreamUpdate& u, int64_t M, int out_bf16) {
   if (M == 0) return CG_OK;
-  const int n4 = (u.W + 7) / 8 * 2;
-  const bool exact = u.W % 8 == 0;
-  const int vec = M <= 296 ? (n4 <= 1024 ? 1 : 4) : n4 <= 2048 ? 2 : 4;
-  const int block = ((n4 + vec - 1) / vec + 31) / 32 * 32;
-  if (block > 1024) return fail(c, CG_ERR_UNSUPPORTED, "decoder: rows wider than 16384 are not supported");
   if (u.ns < 1 || u.ns > MAX_STREAMS) return fail(c, CG_ERR_UNSUPPORTED, "decoder: 1 to 16 streams");
-  auto run = [&](auto t, auto ns) {
+  auto run = [&](auto t, auto exact, auto ns) {
     using T = decltype(t);
+    constexpr bool E = decltype(exact)::value;
     constexpr int NS = decltype(ns)::value;
-    auto kernel = exact ? (vec == 1 ? k_stream_update<T, NS, 1, true> : vec == 2 ? k_stream_update<T, NS, 2, true> : k_stream_update<T, NS, 4, true>)
-                        : (vec == 1 ? k_stream_update<T, NS, 1, false> : vec == 2 ? k_stream_update<T, NS, 2, false> : k_stream_update<T, NS, 4, false>);
-    return launch_kernel(c, kernel, dim3((unsigned)M), dim3(block), 0, 1, u, c->core->dev_err);
+    return launch_rows<k_stream_update<T, NS, 1, E>, k_stream_update<T, NS, 1, E, 4>,
+                       k_stream_update<T, NS, 2, E>, k_stream_update<T, NS, 4, E>>(c, u, M);
   };
-  auto pick = [&](auto t) {
-    if (u.ns == 1) return run(t, std::integral_constant<int, 1>());
-    if (u.ns == 2) return run(t, std::integral_constant<int, 2>());
-    if (u.ns <= 4) return run(t, std::integral_constant<int, 4>());
-    if (u.ns <= 8) return run(t, std::integral_constant<int, 8>());
-    return run(t, std::integral_constant<int, 16>());
+  auto pick = [&](auto t, auto exact) {
+    if (u.ns == 1) return run(t, exact, std::integral_constant<int, 1>());
+    if (u.ns == 2) return run(t, exact, std::integral_constant<int, 2>());
+    if (u.ns <= 4) return run(t, exact, std::integral_constant<int, 4>());
+    if (u.ns <= 8) return run(t, exact, std::integral_constant<int, 8>());
+    return run(t, exact, std::integral_constant<int, 16>());
   };
-  CG_CUDA(c, out_bf16 ? pick(__nv_bfloat16()) : pick(float()));
-  CG_LAUNCHED(c);
-  return CG_OK;
+  if (u.W % 8 == 0) return out_bf16 ? pick(__nv_bfloat16(), std::true_type()) : pick(float(), std::true_type());
+  return out_bf16 ? pick(__nv_bfloat16(), std::false_type()) : pick(float(), std::false_type());
 }
 
 int k_launch_affine(cg_ctx* c, float* x, int64_t n, float f, float v) {

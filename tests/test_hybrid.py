@@ -360,6 +360,21 @@ def test_long_memory_of_the_recurrences(backends, prec):
 
 
 @gpu
+@pytest.mark.parametrize("prec", ["f32", "bf16"])
+@pytest.mark.parametrize("width", [2560, 2568, 2949, 4096, 4104, 16384])
+def test_wide_rows(backends, width, prec):
+    """Every block of the row update can be launched: steps, a short prompt and one of more than 296 tokens."""
+    cfg = model([with_ff(latent(heads=1), 16)], width=width, vocab=24)
+    W, seq = weights(cfg, 21), toks(300, width, 24)
+    want = oracle.forward(cfg, W, seq[:5])
+    dec = decoder(backends[prec], cfg, W, max_seq=300, max_batch=1)
+    assert close(everything(dec, seq[:5], [3, 1, 1]), want, prec)
+    s = dec.open_sequence()
+    assert close(dec.B.to_numpy(dec.run([(s, seq)], [(0, k) for k in range(5)])), want, prec)
+    dec.close()
+
+
+@gpu
 def test_residual_stream_is_f32_in_a_bf16_context(backends):
     """A residual stream far larger than what the layers add: rounded to bf16 the additions would be lost."""
     cfg = model([delta(), ssd(), with_ff(latent())])

@@ -296,6 +296,21 @@ def test_wide_rows_take_the_persistent_kernels(backends):
 
 @gpu
 @pytest.mark.parametrize("prec", ["f32", "bf16"])
+@pytest.mark.parametrize("width", [2560, 2568, 2949, 4096, 4104])
+def test_wide_rows(backends, width, prec):
+    """Rows of plain residuals with nine experts' slots, wider than a block of the narrow form."""
+    cfg = model([moe(att(heads=1, kv_heads=1), 11, 9, 8, 0)], width=width, vocab=24)
+    W, seq = weights(cfg, 21), toks(300, width, 24)
+    want, ok = expected(cfg, W, seq[:5])
+    dec = decoder(backends[prec], cfg, W, max_seq=300, max_batch=1)
+    assert agrees(everything(dec, seq[:5], [3, 1, 1]), want, ok, prec)
+    s = dec.open_sequence()
+    assert agrees(dec.B.to_numpy(dec.run([(s, seq)], [(0, k) for k in range(5)])), want, ok, prec)
+    dec.close()
+
+
+@gpu
+@pytest.mark.parametrize("prec", ["f32", "bf16"])
 def test_strong_and_weak_sinks(backends, prec):
     """Sinks from nothing to nearly everything, and beyond what an exponential can hold."""
     cfg = model([att(heads=4, kv_heads=1, dim=64, vdim=64, window=50)])

@@ -387,6 +387,27 @@ def test_window_passes_over_decoded_tokens(backends, prec):
     dec.close()
 
 
+# widths at which a form's widest block ends, one past it, and the widest rows
+@gpu
+@pytest.mark.parametrize("prec", ["f32", "bf16"])
+@pytest.mark.parametrize("width,streams", [(w, s) for w in (2944, 3072, 4096) for s in (1, 4, 8, 16)] +
+                         [(2560, 1), (2568, 2), (2048, 4), (2056, 3), (2949, 4), (3584, 4), (3592, 3), (4104, 2), (14336, 4), (16384, 2),
+                          (2048, 8), (2056, 5), (2568, 7), (5120, 8), (5128, 8), (8192, 8), (1024, 16), (1032, 9), (3080, 16), (6144, 16)])
+def test_wide_streams(backends, width, streams, prec):
+    """Every block of the stream update can be launched: steps, a short prompt and one of more than 296 tokens; nine experts'
+    slots are three rounds of four and two of eight."""
+    cfg = model([dense(att(heads=1, kv_heads=1), 16), moe(att(heads=1, kv_heads=1), 11, 9, 8)], width=width, streams=streams, vocab=24)
+    W = weights(cfg, 21)
+    seq = toks(300, width + streams, 24)
+    want, ok = expected(cfg, W, seq[:5])
+    dec = decoder(backends[prec], cfg, W, max_seq=300, max_batch=1)
+    assert agrees(everything(dec, seq[:5], [3, 1, 1]), want, ok, prec)
+    s = dec.open_sequence()
+    got = dec.B.to_numpy(dec.run([(s, seq)], [(0, k) for k in range(5)]))
+    assert agrees(got, want, ok, prec)
+    dec.close()
+
+
 @gpu
 def test_residual_streams_are_f32_in_a_bf16_context(backends):
     """Streams far larger than what the layers add: rounded to bf16 the additions would be lost."""
