@@ -494,9 +494,11 @@ __global__ void k_gated_norm(GatedNorm a) {
   }
 }
 
-// Groups of whole 128-bit vectors, kept in registers: G threads per group (a warp, or a block).
-template <class TG, class T, int V>
-__global__ void k_gated_norm_vec(GatedNorm a, int n, int units, int threads) {
+// Groups of whole 128-bit vectors, kept in registers: G threads per group (a warp, or a block of up to THREADS).
+// Gains that wait for the dependency in registers make 73 or 74 a thread, which 1024 threads do not have: there they are read
+// when they are used.
+template <class TG, class T, int V, int THREADS>
+__global__ void __launch_bounds__(THREADS) k_gated_norm_vec(GatedNorm a, int n, int units, int threads) {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   __shared__ float sh[32];
   const int per = blockDim.x / threads, sub = threadIdx.x / threads, t = threadIdx.x - sub * threads;
@@ -507,11 +509,16 @@ __global__ void k_gated_norm_vec(GatedNorm a, int n, int units, int threads) {
   const float* o = a.o + m * (int64_t)a.H * a.dv + c0;
   const TG* gate = (const TG*)a.gate + m * a.ldg + c0;
   T* out = (T*)a.att + m * a.ld_att + c0;
-  float4 x[V], g[V], w[V];
+  float4 x[V], g[V];
+  constexpr bool EARLY = THREADS <= 512;
+  float4 w[EARLY ? V : 1];
+  auto gains = [&](int i) { return __ldg((const float4*)(a.norm + (a.shared_gain ? 0 : c0) + i)); };
+  if constexpr (EARLY) {
 #pragma unroll
-  for (int j = 0; j < V; ++j) {  // the gains are weights: asked for before the dependency
-    const int i = 4 * (t + j * threads);
-    w[j] = live && i < n ? __ldg((const float4*)(a.norm + (a.shared_gain ? 0 : c0) + i)) : make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int j = 0; j < V; ++j) {  // the gains are weights: asked for before the dependency
+      const int i = 4 * (t + j * threads);
+      w[j] = live && i < n ? gains(i) : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
   }
   asm volatile("griddepcontrol.wait;" ::: "memory");
   float ss = 0.f;
@@ -541,7 +548,8 @@ __global__ void k_gated_norm_vec(GatedNorm a, int n, int units, int threads) {
   for (int j = 0; j < V; ++j) {
     const int i = 4 * (t + j * threads);
     if (!live || i >= n) continue;
-    float4 r = make_float4(x[j].x * inv * w[j].x, x[j].y * inv * w[j].y, x[j].z * inv * w[j].z, x[j].w * inv * w[j].w);
+    const float4 f = EARLY ? w[EARLY ? j : 0] : gains(i);
+    float4 r = make_float4(x[j].x * inv * f.x, x[j].y * inv * f.y, x[j].z * inv * f.z, x[j].w * inv * f.w);
     if (!a.gate_first) { r.x *= g[j].x; r.y *= g[j].y; r.z *= g[j].z; r.w *= g[j].w; }
     st4(out + i, r);
   }
@@ -554,11 +562,12 @@ int launch_gated_norm(cg_ctx* c, const GatedNorm& a) {
   const bool vec = a.dv == a.dvs && n % 4 == 0 && a.ldg % 4 == 0 && a.ld_att % 4 == 0 && (((uintptr_t)a.gate | (uintptr_t)a.norm) & 15) == 0 && n <= 16384;
   if (vec && n <= 512) {
     const int64_t blocks = (a.M * units + 7) / 8;
-    if (n <= 128) CG_CUDA(c, launch_kernel(c, k_gated_norm_vec<TG, T, 1>, dim3((unsigned)blocks), dim3(256), 0, 1, a, n, units, 32));
-    else CG_CUDA(c, launch_kernel(c, k_gated_norm_vec<TG, T, 4>, dim3((unsigned)blocks), dim3(256), 0, 1, a, n, units, 32));
+    if (n <= 128) CG_CUDA(c, launch_kernel(c, k_gated_norm_vec<TG, T, 1, 256>, dim3((unsigned)blocks), dim3(256), 0, 1, a, n, units, 32));
+    else CG_CUDA(c, launch_kernel(c, k_gated_norm_vec<TG, T, 4, 512>, dim3((unsigned)blocks), dim3(256), 0, 1, a, n, units, 32));
   } else if (vec) {
     const int threads = n <= 4096 ? 256 : n <= 8192 ? 512 : 1024;
-    CG_CUDA(c, launch_kernel(c, k_gated_norm_vec<TG, T, 4>, dim3((unsigned)(a.M * units)), dim3(threads), 0, 1, a, n, units, threads));
+    auto kernel = threads <= 512 ? k_gated_norm_vec<TG, T, 4, 512> : k_gated_norm_vec<TG, T, 4, 1024>;
+    CG_CUDA(c, launch_kernel(c, kernel, dim3((unsigned)(a.M * units)), dim3(threads), 0, 1, a, n, units, threads));
   } else {
     dim3 grid((unsigned)units, (unsigned)a.M);
     if (grid.y > 65535) return fail(c, CG_ERR_UNSUPPORTED, "recurrence: too many tokens in one portion");

@@ -375,6 +375,20 @@ def test_wide_rows(backends, width, prec):
 
 
 @gpu
+@pytest.mark.parametrize("prec", ["f32", "bf16"])
+@pytest.mark.parametrize("heads,vdim,norm_groups", [(32, 128, 1), (64, 128, 1), (205, 40, 1), (130, 128, 2), (128, 128, 1)])
+def test_wide_norm_groups(backends, heads, vdim, norm_groups, prec):
+    """Groups of the gated norm of 4096 to 16384 values: 256, 512 and 1024 threads, behind a prompt and behind steps."""
+    cfg = model([ssd(heads=heads, groups=1, vdim=vdim, norm_groups=norm_groups)])
+    W, seq = weights(cfg, 22), toks(9, heads)
+    want = oracle.forward(cfg, W, seq)
+    dec = decoder(backends[prec], cfg, W, max_seq=16, max_batch=1)
+    assert close(everything(dec, seq), want, prec)
+    assert close(everything(dec, seq, [5, 1, 1, 1, 1]), want, prec)
+    dec.close()
+
+
+@gpu
 def test_residual_stream_is_f32_in_a_bf16_context(backends):
     """A residual stream far larger than what the layers add: rounded to bf16 the additions would be lost."""
     cfg = model([delta(), ssd(), with_ff(latent())])
