@@ -113,7 +113,8 @@ __device__ __forceinline__ void attn_dec_item(const AttnDecArgs& a, float scale,
       asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
       asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     }
-    if (tid == 0) *cta_abort = 0;
+    __syncwarp();
+    if (tid == 0) *cta_abort = 0;  // (for the other warps behind the first CTA barrier)
   }
   const int rep = a.nh / a.nkv;
   const int S = a.splits;
@@ -248,20 +249,32 @@ __device__ __forceinline__ void attn_dec_item(const AttnDecArgs& a, float scale,
   };
   angles();
   for (int i = tid; i < (8 - rep) * CH; i += 128) *(uint4*)(qt + (rep + i / CH) * LD + i % CH * 8) = make_uint4(0u, 0u, 0u, 0u);
+  bool ok = true;
   {
     const int64_t pos_now = env.settle(pos);
     if (pos_now != pos) {  // the early position was stale: let the copies land, then ask again
-      if (c0 < t1) {
-        tc::mbar_drain(bar_k, phase, a.err);
-        tc::mbar_drain(bar_v, phase, a.err);
-        phase ^= 1u;
+      if constexpr (Env::kPush) {
+        if (c0 < t1) {
+          int gave_up = 0;
+          ok = tc::mbar_wait(bar_k, phase, &gave_up, a.err) && tc::mbar_wait(bar_v, phase, &gave_up, a.err);
+          ok = __all_sync(0xffffffffu, ok) != 0;
+          if (!ok) {
+            tc::mbar_drain(bar_k, phase, a.err);
+            tc::mbar_drain(bar_v, phase, a.err);
+          }
+          phase ^= 1u;
+        }
+      } else {
+        cp_async_wait_group<0>();
       }
       __syncwarp();
       pos = pos_now;
       plan();
       c0 = t0 + warp * KT;
-      request(c0, true);
-      request(c0, false);
+      if (ok) {
+        request(c0, true);
+        request(c0, false);
+      }
       angles();
     }
   }
@@ -381,6 +394,10 @@ __device__ __forceinline__ void attn_dec_item(const AttnDecArgs& a, float scale,
     }
   }
   env.sync_cta();
+  if (!ok) {  // without keys from here on, but past every barrier
+    *cta_abort = 1;
+    c0 = t1;
+  }
 
   // ---- 2. this warp's chunks of KT keys: S = Q K^T, online softmax, O^T += V^T P^T ----
   // In S a thread owns head hr = lane / 4 and, per 8-key tile, the two keys cq + {0, 1}; in O^T the two heads

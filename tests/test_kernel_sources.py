@@ -54,3 +54,19 @@ def test_the_step_counter_is_released_to_early_readers():
         body = text[text.index(f" {name}("):]
         body = body[:body.index("\n}\n")]
         assert body.index("griddepcontrol.wait;") < body.index("step_done(pos_dev);")
+
+
+def test_tiles_asked_for_with_a_stale_position_are_waited_for():
+    """The decode attention asks for its first tiles with a position that may be a step old, and asks again where it was.  The
+    first copies are waited for by a wait that reports when it gives up; after that the warp takes no tile.  A poll that
+    says nothing would leave the barrier a phase behind, and the next wait would pass before its tile is there."""
+    text = open(os.path.join(CSRC, "attn_decode.cuh")).read()
+    item = text[text.index("void attn_dec_item("):]
+    init = item.index("tc::mbar_init(bar_v, 1);")
+    assert init < item.index("__syncwarp();\n    if (tid == 0) *cta_abort = 0;") < item.index("request(c0, true);")   # of every warp, for any number of slices
+    stale = item[item.index("if (pos_now != pos) {"):item.index("angles();\n    }\n  }\n\n  // ---- 1.")]
+    wait, poll, again = (stale.index(x) for x in ("tc::mbar_wait(bar_k, phase,", "tc::mbar_drain(bar_k, phase,", "request(c0, true);"))
+    assert wait < stale.index("if (!ok) {") < poll < again and stale[:again].rstrip().endswith("if (ok) {")
+    gone = item.index("if (!ok) {  // without keys")
+    assert item.rindex("env.sync_cta();", 0, gone) < gone < item.index("for (; c0 < t1; c0 += 4 * KT)")
+    assert "c0 = t1;" in item[gone:gone + 120]
