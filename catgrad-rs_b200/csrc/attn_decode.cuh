@@ -519,6 +519,9 @@ __device__ __forceinline__ void attn_dec_item(const AttnDecArgs& a, float scale,
     insert(vw, vnew);
     if (live < KT) {  // probability zero times whatever lies behind the live rows must not be NaN
       for (int i = lane; i < (KT - live) * CH; i += 32) *chunk_of(vw, live + i / CH, i % CH) = make_uint4(0u, 0u, 0u, 0u);
+      // (behind kept first keys the tile is loaded again: TMA's writes come after these)
+      if constexpr (Env::kPush && Env::kRows)
+        if (c0 + 4 * KT < t1) asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     }
     __syncwarp();
     // O^T += V^T P^T: the scores' fragments are those of P^T

@@ -70,3 +70,11 @@ def test_tiles_asked_for_with_a_stale_position_are_waited_for():
     gone = item.index("if (!ok) {  // without keys")
     assert item.rindex("env.sync_cta();", 0, gone) < gone < item.index("for (; c0 < t1; c0 += 4 * KT)")
     assert "c0 = t1;" in item[gone:gone + 120]
+
+
+def test_cleared_rows_of_a_tile_come_before_its_next_load():
+    """Ordinary stores to a tile and TMA's next writes to it are different proxies: without a fence the stores may come last."""
+    text = open(os.path.join(CSRC, "attn_decode.cuh")).read()
+    clear = text.index("*chunk_of(vw, live + i / CH, i % CH) = make_uint4")
+    fence = text.index("if (c0 + 4 * KT < t1) asm volatile(\"fence.proxy.async.shared::cta;\"", clear)
+    assert clear < fence < text.index("__syncwarp();", fence) < text.index("request(c0 + 4 * KT, false);")

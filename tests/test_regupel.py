@@ -494,6 +494,33 @@ def test_first_tokens_and_window_edges(backends, window, kept, dim, how, prec):
 
 
 @gpu
+@pytest.mark.parametrize("window,kept,dim", [(200, 33, 64), (200, 50, 64), (180, 1, 128), (160, 95, 128), (150, 17, 256), (200, 9, 256)])
+def test_kept_tokens_before_more_tiles(backends, window, kept, dim):
+    """So many rows that a context is one slice: the warp with the partly filled tile of kept tokens loads that tile again.  The
+    key that stands out is the last one kept, or lies where that tile had been cleared."""
+    layer = par(heads=2, kv_heads=1, dim=dim, vdim=dim, window=window, kept=kept, scale=1.0, left=1.5, right=0.1)
+    cfg, W, asks, sought = seeking_model(layer, "left.", 2, dim)
+    n, rows, tile = kept + window + 20, 150, 16 if dim > 128 else 32
+    padded = (kept + tile - 1) // tile * tile                    # keys are numbered from the next tile on
+    again = padded - 1 + 4 * tile                                # the last key of the tile that the same warp loads next
+    dec = decoder(backends["bf16"], cfg, W, max_seq=n, max_batch=rows)
+    for at in (kept - 1, again - padded + n - window):
+        seq = np.random.default_rng(at).integers(0, 102, n)
+        seq[n - 1], seq[at] = asks, sought
+        want = oracle.forward(cfg, W, seq)[-1]
+        other = seq.copy()
+        other[at] = 0
+        assert err(oracle.forward(cfg, W, other)[-1], want) > 4 * TOL["bf16"]
+        slots = [dec.open_sequence() for _ in range(rows)]
+        dec.run([(s, seq[:n - 1]) for s in slots])
+        got = dec.B.to_numpy(dec.run([(s, seq[n - 1:]) for s in slots], [(r, 0) for r in range(rows)]))
+        assert all(close(got[r], want, "bf16") for r in range(rows)), at
+        for s in slots:
+            dec.close_sequence(s)
+    dec.close()
+
+
+@gpu
 @pytest.mark.parametrize("prec", ["f32", "bf16"])
 def test_window_passes_over_decoded_tokens(backends, prec):
     """The sought token itself is decoded, and leaves the window while others are decoded; the same at a
