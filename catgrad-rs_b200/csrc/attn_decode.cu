@@ -43,16 +43,25 @@ struct KernelEnv {
   float* land;
   const CUtensorMap *map_k, *map_v;
   __device__ __forceinline__ float* landing() const { return land; }
-  // the projected row, and the position when it lives on the device, belong to the stream order
-  const AttnDecArgs* args;
   static constexpr bool kRows = ROWS;
+  // The position is first + *step, or first alone.  (Held by value: no address of a kernel parameter is taken, whatever space
+  // the parameters lie in.)
+  const int64_t* step;
+  int64_t first;
+  __device__ __forceinline__ int64_t position() const { return first + (step ? *(const volatile int64_t*)step : 0); }
+  // the projected row, and the position when it lives on the device, belong to the stream order
   __device__ __forceinline__ int64_t settle(int64_t) const {
     asm volatile("griddepcontrol.wait;" ::: "memory");
-    if constexpr (ROWS) return args->rows.pos0[blockIdx.y] + *(const volatile int64_t*)args->rows.step;
-    return args->pos_dev ? *(const volatile int64_t*)args->pos_dev : args->pos0;
+    return position();
   }
 };
 
+// What is reached by the tables and the counter on the device, before and behind the wait, and why it is in range: slot and
+// pos0 have an entry per row, blockIdx.y < rows of them; a slot whose cache would end past cache_rows and a settled position outside
+// [0, Tmax) raise the error word, are replaced by ones in range and append nothing; the early position is clamped.  Angles
+// are [Tmax][rot_dims / 2] (rows) or [Tmax][D / 2], temperatures [Tmax], by position; biases [nh][ld_bias], read for live
+// keys only, whose distance is 0 to the position.  A tile begins at a key below the position or the new one, so inside the cache; what
+// of it lies past the cache's end reads as zeros, past the row's end is masked.  Landing areas: attn_dec_landing_bytes.
 template <int D, bool ROWS>
 __global__ void __launch_bounds__(128, 4)
 k_attn_dec(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v, AttnDecArgs a, float scale) {
@@ -61,7 +70,6 @@ k_attn_dec(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CU
   const uint32_t raw = (uint32_t)__cvta_generic_to_shared(smem_raw);
   uint8_t* smem = smem_raw + (((raw + 1023u) & ~1023u) - raw);
   KernelEnv<ROWS> env;
-  env.args = &a;
   env.map_k = &map_k;
   env.map_v = &map_v;
   env.land = (float*)(smem + attn_dec_smem_bytes<D>());
@@ -72,8 +80,14 @@ k_attn_dec(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CU
   // has completed, so whatever value is visible here, the rows below it are complete.  The value
   // may be a step old; it is re-read after the wait and a changed value repeats the request.
   // (Row tables are copied in plain stream order before any kernel that reads them.)
-  int64_t pos_early = a.pos_dev ? *(const volatile int64_t*)a.pos_dev : a.pos0;
-  if constexpr (ROWS) pos_early = a.rows.pos0[blockIdx.y] + *(const volatile int64_t*)a.rows.step;
+  if constexpr (ROWS) {
+    env.step = a.rows.step;
+    env.first = a.rows.pos0[blockIdx.y];
+  } else {
+    env.step = a.pos_dev;
+    env.first = a.pos_dev ? 0 : a.pos0;
+  }
+  int64_t pos_early = env.position();
   pos_early = pos_early < 0 ? 0 : (pos_early >= a.Tmax ? a.Tmax - 1 : pos_early);
   attn_dec_item<D>(a, scale, (int)blockIdx.x, (int64_t)blockIdx.y, (int)blockIdx.z, pos_early, smem, env);
 }
@@ -133,6 +147,7 @@ int k_launch_attn_dec(cg_ctx* c, const AttnDecArgs& a) {
   if (!a.rows.rows && !a.pos_dev && a.pos0 >= a.Tmax) return fail(c, CG_ERR_SHAPE, "attention: KV cache capacity exceeded");
   if (a.B == 0) return CG_OK;
   if (a.cache_rows <= 0 || a.cache_rows > 2147483647ll) return fail(c, CG_ERR_UNSUPPORTED, "attention: more cache rows than a tile coordinate holds");
+  if (!a.rows.rows && a.B * a.nkv * a.Tmax > a.cache_rows) return fail(c, CG_ERR_SHAPE, "attention: more rows than the KV cache holds");
   if (a.rows.rows) {
     switch (a.d) {
       case 64: return launch<64, true>(c, a);

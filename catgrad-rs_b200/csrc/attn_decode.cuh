@@ -140,7 +140,15 @@ __device__ __forceinline__ void attn_dec_item(const AttnDecArgs& a, float scale,
   }
   // pos: position of the new token = number of cached keys
   int64_t place = b;
-  if constexpr (Env::kRows) place = a.rows.slot[b];
+  bool in_range = true;
+  if constexpr (Env::kRows) {
+    place = a.rows.slot[b];
+    if (place < 0 || (place + 1) * a.nkv * a.Tmax > a.cache_rows) {
+      *a.err = DEV_INDEX;
+      place = 0;
+      in_range = false;
+    }
+  }
   __nv_bfloat16* kbase = a.k_cache + ((place * a.nkv + kvh) * a.Tmax) * (int64_t)D;
   __nv_bfloat16* vbase = a.v_cache + ((place * a.nkv + kvh) * a.Tmax) * (int64_t)D;
 
@@ -251,7 +259,13 @@ __device__ __forceinline__ void attn_dec_item(const AttnDecArgs& a, float scale,
   for (int i = tid; i < (8 - rep) * CH; i += 128) *(uint4*)(qt + (rep + i / CH) * LD + i % CH * 8) = make_uint4(0u, 0u, 0u, 0u);
   bool ok = true;
   {
-    const int64_t pos_now = env.settle(pos);
+    int64_t pos_now = env.settle(pos);
+    if constexpr (Env::kPush)
+      if ((uint64_t)pos_now >= (uint64_t)a.Tmax) {
+        *a.err = DEV_INDEX;
+        pos_now = pos;
+        in_range = false;
+      }
     if (pos_now != pos) {  // the early position was stale: let the copies land, then ask again
       if constexpr (Env::kPush) {
         if (c0 < t1) {
@@ -390,7 +404,7 @@ __device__ __forceinline__ void attn_dec_item(const AttnDecArgs& a, float scale,
         }
       };
       put(id < rep ? qt + id * LD : id == rep ? knew : vnew);
-      if (id >= rep && split == 0) put((id == rep ? kbase : vbase) + pos * D);  // append to the cache for the following steps
+      if (id >= rep && split == 0 && in_range) put((id == rep ? kbase : vbase) + pos * D);  // append to the cache for the following steps
     }
   }
   env.sync_cta();

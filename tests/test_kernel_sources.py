@@ -78,3 +78,18 @@ def test_cleared_rows_of_a_tile_come_before_its_next_load():
     clear = text.index("*chunk_of(vw, live + i / CH, i % CH) = make_uint4")
     fence = text.index("if (c0 + 4 * KT < t1) asm volatile(\"fence.proxy.async.shared::cta;\"", clear)
     assert clear < fence < text.index("__syncwarp();", fence) < text.index("request(c0 + 4 * KT, false);")
+
+
+def test_decode_attention_checks_what_it_takes_from_the_device():
+    """Slots and positions come from device memory: one out of range raises the error word and appends nothing.  The environment
+    holds what it needs by value, not the address of a kernel parameter."""
+    text = open(os.path.join(CSRC, "attn_decode.cu")).read()
+    env = text[text.index("struct KernelEnv {"):text.index("__global__")]
+    assert "AttnDecArgs" not in env and "= &a;" not in kernel("attn_decode.cu", "k_attn_dec")
+    item = open(os.path.join(CSRC, "attn_decode.cuh")).read()
+    slot, settled = item.index("place = a.rows.slot[b];"), item.index("int64_t pos_now = env.settle(pos);")
+    for at, before in ((slot, "kbase ="), (settled, "if (pos_now != pos)")):
+        check = item[at:item.index(before, at)]
+        assert "*a.err = DEV_INDEX;" in check and "in_range = false;" in check
+    assert "(place + 1) * a.nkv * a.Tmax > a.cache_rows" in item and "(uint64_t)pos_now >= (uint64_t)a.Tmax" in item
+    assert "if (id >= rep && split == 0 && in_range) put(" in item and item.count("split == 0") == 1
