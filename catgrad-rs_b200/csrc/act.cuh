@@ -13,6 +13,16 @@ __device__ __forceinline__ float gelu_f(float x) {
   return 0.5f * x * (1.f + tanh_f(c * (x + 0.044715f * x * x * x)));
 }
 
+// g / (1 + e) for e >= 0 where a division is a call: an approximate reciprocal and one step of Newton's iteration, which keep
+// 24 bits.  The reciprocal is that of (1 + e) / 16: approximations are flushed to zero below 2^-126, and 1 / (1 + e) may be
+// smaller than that.  0 where e is infinite, NaN where it is NaN, as the division has it.
+__device__ __forceinline__ float over_one_plus(float g, float e) {
+  const float d = fmaf(e, 0.0625f, 0.0625f);
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(d));
+  return g * 0.0625f * (d < 3e37f ? fmaf(r, fmaf(-d, r, 1.f), r) : r);
+}
+
 // Cheaper forms for epilogues whose result is rounded to bf16 anyway: approximate division.
 __device__ __forceinline__ float sigmoid_fast(float x) { return __fdividef(1.f, 1.f + __expf(-x)); }
 __device__ __forceinline__ float silu_fast(float x) { return x * sigmoid_fast(x); }

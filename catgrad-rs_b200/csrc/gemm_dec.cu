@@ -116,14 +116,9 @@ __device__ __forceinline__ void with_form(const DecArgs& p, F f) {
   else if (p.out_mode == 3) f(std::integral_constant<int, FORM_PUSH>{});
   else f(std::integral_constant<int, FORM_BF16>{});
 }
-// silu or tanh-gelu of g: 1 / (1 + e^-x) by an approximation and one step of Newton's iteration, which keeps its 24 bits
-// where a division is a call; 0 where e^-x is infinite, NaN where x is NaN, as the division has it
+// silu or tanh-gelu of g
 __device__ __forceinline__ float act_of(int act, float g) {
-  const float x = act == 0 ? g : 1.5957691216f * (g + 0.044715f * g * g * g);
-  const float d = 1.f + __expf(-x);
-  float r;
-  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(d));
-  return g * (d < 1e37f ? fmaf(r, fmaf(-d, r, 1.f), r) : r);
+  return over_one_plus(g, __expf(-(act == 0 ? g : 1.5957691216f * (g + 0.044715f * g * g * g))));
 }
 // Output (m, n), o = m * ldo + n; `res`: the residual there; `gain`: the next norm's at n.  Returns what the row's sum of
 // squares gets.
