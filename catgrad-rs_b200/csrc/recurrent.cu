@@ -194,8 +194,9 @@ __global__ void __launch_bounds__(128) k_recur_steps(RecurArgs a) {
 // What bounds it is the chain from the projection to the output, beside 5 us of state bytes at batch 8: so all that does not
 // depend on the projection (state, earlier inputs of the convolutions, weights, gains) is read before it is waited
 // for, its values come in one round of loads, and four barriers are left.  Four blocks per SM where a thread has
-// eight rows, which lets 512 blocks start at once.  Us that a launch keeps the stream, 8 rows, before / now: 64 heads of
-// 128 x 64: 17.4 / 11.6; 32 heads of 128 x 128 with the delta rule: 12.9 / 12.0.
+// eight rows, which lets 512 blocks start at once (64 registers and 40 bytes of spills; three, with 80 and none, are slower from 256
+// blocks on: 273 and 289 us for a step of eight layers of 64 heads, 8 rows; 217 and 209 us with one row).  Us that a launch keeps
+// the stream, 8 rows, before / now: 64 heads of 128 x 64: 17.4 / 11.6; 32 heads of 128 x 128 with the delta rule: 12.9 / 12.0.
 // KD: a decay per key channel; the second factors of the low-rank projections are applied here, a row of them
 // per thread, from shared memory where they fit (rows R + 8 apart: no bank conflicts).
 __device__ __forceinline__ float low_rank_staged(const float* x, const __nv_bfloat16* w, int R) {
@@ -211,8 +212,8 @@ __device__ __forceinline__ float low_rank_staged(const float* x, const __nv_bflo
   }
   return v[0] + v[1];
 }
-template <int RD_ROWS, bool KD>
-__global__ void __launch_bounds__(256, RD_ROWS <= 8 ? 4 : 2) k_recur_decode(RecurArgs a, GatedNorm n) {
+template <int RD_ROWS, bool KD, int PER_SM>
+__global__ void __launch_bounds__(256, PER_SM) k_recur_decode(RecurArgs a, GatedNorm n) {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   __shared__ __align__(16) float sq[128], sk[128], sv[128];
   __shared__ float sg[4];
@@ -306,6 +307,11 @@ __global__ void __launch_bounds__(256, RD_ROWS <= 8 ? 4 : 2) k_recur_decode(Recu
     if (a.delta) b_in = sp[h];
     if (!KD && !a.log_decay) g_in = sp[a.delta ? a.H + h : h];
   }
+  // KD: the low-rank projections' values, first and second part behind one another, 256 of them now
+  const int n_low = KD ? a.a_rank + (a.w_g2 ? a.g_rank : 0) : 0;
+  auto low_of = [&](int j) { return p[j < a.a_rank ? a.a1_off + j : a.g1_off + j - a.a_rank]; };
+  float low_now = 0.f;
+  if (KD && tid < n_low) low_now = low_of(tid);
   if (a.delta && !KD && tid < a.dv) sgate[tid] = ((const float*)n.gate)[m * n.ldg + (int64_t)h * a.dv + tid];
   if (pos != pos_early) {
     load_state(pos > 0);
@@ -326,9 +332,8 @@ __global__ void __launch_bounds__(256, RD_ROWS <= 8 ? 4 : 2) k_recur_decode(Recu
     (seg == 0 ? sq : seg == 1 ? sk : sv)[x - seg * a.dk] = v;
   }
   if (KD) {
-    for (int j = tid; j < a.a_rank; j += 256) low[j] = p[a.a1_off + j];
-    if (a.w_g2)
-      for (int j = tid; j < a.g_rank; j += 256) low[a.a_rank + j] = p[a.g1_off + j];
+    if (tid < n_low) low[tid] = low_now;
+    for (int j = tid + 256; j < n_low; j += 256) low[j] = low_of(j);
     cp_async_wait_all();
     __syncthreads();
 #pragma unroll 1
@@ -587,7 +592,6 @@ int k_launch_recur_decode(cg_ctx* c, const RecurArgs& a, const GatedNorm& n) {
   if (a.rows.rows == 0) return CG_OK;
   const int rpp = 256 / (a.dvs / 4);  // state rows per pass
   const bool few = (a.dk + rpp - 1) / rpp <= 8;
-  auto kernel = a.key_decay ? (few ? k_recur_decode<8, true> : k_recur_decode<16, true>) : few ? k_recur_decode<8, false> : k_recur_decode<16, false>;
   RecurArgs args = a;
   size_t smem = a.key_decay ? (size_t)(a.a_rank + a.g_rank) * 4 : 0;
   if (smem > 32 * 1024) return fail(c, CG_ERR_UNSUPPORTED, "recurrence: low-rank projections too wide");
@@ -595,8 +599,17 @@ int k_launch_recur_decode(cg_ctx* c, const RecurArgs& a, const GatedNorm& n) {
     const size_t rows = ((size_t)a.dk * (a.a_rank + 8) + (a.w_g2 ? (size_t)a.dv * (a.g_rank + 8) : 0)) * 2;
     args.w_staged = a.a_rank % 8 == 0 && a.g_rank % 8 == 0 && smem + rows <= LOW_RANK_SMEM;
     if (args.w_staged) smem += rows;
-    static PerDeviceFlag configured_on[2];
-    bool& configured = configured_on[few ? 1 : 0].at(c->core->device);
+  }
+  // A decay per key channel: the form for four blocks per SM spills 68 bytes, and is taken only where it saves a wave and its
+  // shared memory (9 KB of the kernel's own) lets four in.  Us of a step of eight layers of 32 heads with three / four per SM: gated
+  // linear attention, 64 x 128 states, one row 231 / 239, 8 rows 259 / 274, 16 rows 334 / 305; delta rule, 64 x 64, 16 rows 362 / 295.
+  auto waves = [&](int per_sm) { return ((int64_t)a.H * a.rows.rows + per_sm * 148 - 1) / (per_sm * 148); };
+  const bool four = waves(4) < waves(3) && 4 * (smem + 9 * 1024) <= 228 * 1024;
+  auto kernel = a.key_decay ? (!few ? k_recur_decode<16, true, 2> : four ? k_recur_decode<8, true, 4> : k_recur_decode<8, true, 3>)
+                            : few ? k_recur_decode<8, false, 4> : k_recur_decode<16, false, 2>;
+  if (args.w_staged) {
+    static PerDeviceFlag configured_on[3];
+    bool& configured = configured_on[few ? 1 + four : 0].at(c->core->device);
     if (!configured) {
       CG_CUDA(c, cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)LOW_RANK_SMEM));
       configured = true;

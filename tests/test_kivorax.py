@@ -345,6 +345,25 @@ def test_portions(backends, cut, prec):
     dec.close()
 
 
+# 4 heads: three blocks per SM fill up at 111 rows, four at 148; low-rank projections of one round of loads and of more
+@gpu
+@pytest.mark.parametrize("prec", ["f32", "bf16"])
+@pytest.mark.parametrize("layer,ranks,rows", [(cdelta(4, 4, 64, 64), (10, 14), n) for n in (111, 112, 148, 149)] +
+                         [(cdelta(4, 2, 64, 128), (128, 128), 112), (gla(4, 64, 128), (16, 1), 112), (cdelta(2, 1, 24, 40), (248, 16), 3),
+                          (cdelta(2, 1, 24, 40), (130, 140), 3), (gla(2, 24, 40), (600, 1), 3)])
+def test_steps_of_many_rows_and_wide_ranks(backends, layer, ranks, rows, prec):
+    cfg = model([layer])
+    W, seq = weights(cfg, 23, ranks), toks(8, rows)
+    want = oracle.forward(cfg, W, seq)
+    dec = decoder(backends[prec], cfg, W, max_seq=8, max_batch=rows)
+    slots = [dec.open_sequence() for _ in range(rows)]
+    dec.run([(s, seq[:6]) for s in slots])
+    for t in (6, 7):
+        got = dec.B.to_numpy(dec.run([(s, seq[t:t + 1]) for s in slots], [(r, 0) for r in range(rows)]))
+        assert close(got, [want[t]] * rows, prec), t
+    dec.close()
+
+
 @gpu
 @pytest.mark.parametrize("prec", ["f32", "bf16"])
 def test_unequal_batch(backends, prec):
