@@ -126,16 +126,22 @@ int launch(cg_ctx* c, const AttnDecArgs& args) {
 // supports).  A slice keeps at least 128 keys at full context, one chunk per warp, and all CTAs together
 // stay within two per SM: beyond that a CTA's fixed part (query preparation, merges) costs more than the
 // shorter loop gives, unless a slice would have more than 256 keys; then three to four per SM, as many as fit, will do.
+// But a cluster of 16 has to fit into one GPC, where head sizes above 64 leave two or three CTAs per SM: with more than some 20
+// rows and kv heads (24 at head size 64) such clusters wait for one another.  Us per step of four layers with 8 / 16 slices, 2048 keys of
+// 4200: 32 x 64 124 / 144; 24 x 128 201 / 223; 24 x 256 178 / 197; 20 x 128 142 / 146; 20 x 256 173 / 170; 24 x 64, 4096 keys 116 / 112.
 // Ms per pass with 1 / 2 / 4 / 8 / 16 slices (the rule's choice in brackets):
 //   8 rows x 8 kv heads, 640 keys, d 64 (128 steps of 16 layers)    106.2  102.0 [100.1] 101.9  119.0
 //   32 x 8, 558 keys, d 128 (48 steps of 4 layers)                   66.1 [64.3]   65.2   67.6   74.3
 //   1 x 8, 8200 keys, d 128 (8 steps of 4 layers)                    22.7   20.7   20.2   20.5  [20.1]
 //   4 x 4, 2113 keys, d 256 (64 steps of 4 layers)                   42.0   36.6   33.7   32.5  [32.4]
 //   8 x 4, 1073 keys, d 128, 8 heads each (48 steps of 4 layers)     38.6   37.9   37.5  [37.5]  38.4
-int attn_dec_splits(int64_t Tmax, int64_t pairs) {
+int attn_dec_splits(int64_t Tmax, int64_t pairs, int d) {
   constexpr int64_t SMS = 148;
   int s = 1;
-  while (s < 16 && (int64_t)s * 128 < Tmax && (pairs * s * 2 <= 2 * SMS || ((int64_t)s * 256 < Tmax && pairs * s * 2 <= 4 * SMS))) s *= 2;
+  const bool fits = pairs <= (d == 64 ? 24 : 20);  // in clusters of 16
+  while (s < 16 && (int64_t)s * 128 < Tmax &&
+         (pairs * s * 2 <= 2 * SMS || ((int64_t)s * 256 < Tmax && pairs * s * 2 <= 4 * SMS && (s < 8 || fits))))
+    s *= 2;
   return s;
 }
 

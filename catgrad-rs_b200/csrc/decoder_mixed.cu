@@ -924,7 +924,7 @@ int attention_layer(cg_decoder* D, const MixedLayer& L, MixedRun& run, const Row
     f.scale = (float)k.scale; f.sink = sink;
     f.wide_gate = k.gate == 2; f.q_temp = q_temp; f.bias = bias; f.ld_bias = ld_bias;
     const int64_t reach = k.window > 0 ? std::min<int64_t>((int64_t)k.window + k.keep_first, f.Tmax) : f.Tmax;
-    f.splits = attn_dec_splits(reach, f.B * f.nkv);
+    f.splits = attn_dec_splits(reach, f.B * f.nkv, f.d);
     return k_launch_attn_dec(c, f);
   }
   RowsAttnArgs a;
