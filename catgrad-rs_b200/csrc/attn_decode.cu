@@ -62,6 +62,7 @@ struct KernelEnv {
 // are [Tmax][rot_dims / 2] (rows) or [Tmax][D / 2], temperatures [Tmax], by position; biases [nh][ld_bias], read for live
 // keys only, whose distance is 0 to the position.  A tile begins at a key below the position or the new one, so inside the cache; what
 // of it lies past the cache's end reads as zeros, past the row's end is masked.  Landing areas: attn_dec_landing_bytes.
+// (Four CTAs per SM leave 128 registers a thread: all that head sizes 128 and 256 use; the row form at 256 spills 8 bytes.)
 template <int D, bool ROWS>
 __global__ void __launch_bounds__(128, 4)
 k_attn_dec(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v, AttnDecArgs a, float scale) {
