@@ -499,11 +499,13 @@ __global__ void k_gated_norm(GatedNorm a) {
   }
 }
 
-// Groups of whole 128-bit vectors, kept in registers: G threads per group (a warp, or a block of up to THREADS).
-// Gains that wait for the dependency in registers make 73 or 74 a thread, which 1024 threads do not have: there they are read
-// when they are used.
-template <class TG, class T, int V, int THREADS>
-__global__ void __launch_bounds__(THREADS) k_gated_norm_vec(GatedNorm a, int n, int units, int threads) {
+// Groups of whole 128-bit vectors, kept in registers: G threads per group (a warp, or a block).
+// EARLY: the gains, which are weights, are read before the dependency.  That makes 72 to 74 registers a thread, so it is for
+// blocks of up to 512 threads and for steps, whose few blocks have an SM each; among the blocks of a prompt it takes the place of
+// others (8192 groups of 2048: 46.6 us, 42.3 without; 8 groups of 4096: 4.8, 6.5 without).  The other form has 56 to 62, which 1024
+// threads may have.
+template <class TG, class T, int V, bool EARLY>
+__global__ void k_gated_norm_vec(GatedNorm a, int n, int units, int threads) {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   __shared__ float sh[32];
   const int per = blockDim.x / threads, sub = threadIdx.x / threads, t = threadIdx.x - sub * threads;
@@ -515,12 +517,11 @@ __global__ void __launch_bounds__(THREADS) k_gated_norm_vec(GatedNorm a, int n, 
   const TG* gate = (const TG*)a.gate + m * a.ldg + c0;
   T* out = (T*)a.att + m * a.ld_att + c0;
   float4 x[V], g[V];
-  constexpr bool EARLY = THREADS <= 512;
   float4 w[EARLY ? V : 1];
-  auto gains = [&](int i) { return __ldg((const float4*)(a.norm + (a.shared_gain ? 0 : c0) + i)); };
+  auto gains = [&](int i) { return *(const float4*)(a.norm + (a.shared_gain ? 0 : c0) + i); };
   if constexpr (EARLY) {
 #pragma unroll
-    for (int j = 0; j < V; ++j) {  // the gains are weights: asked for before the dependency
+    for (int j = 0; j < V; ++j) {
       const int i = 4 * (t + j * threads);
       w[j] = live && i < n ? gains(i) : make_float4(0.f, 0.f, 0.f, 0.f);
     }
@@ -565,14 +566,15 @@ int launch_gated_norm(cg_ctx* c, const GatedNorm& a) {
   const int units = a.groups;
   const int n = a.H * a.dv / units;
   const bool vec = a.dv == a.dvs && n % 4 == 0 && a.ldg % 4 == 0 && a.ld_att % 4 == 0 && (((uintptr_t)a.gate | (uintptr_t)a.norm) & 15) == 0 && n <= 16384;
-  if (vec && n <= 512) {
-    const int64_t blocks = (a.M * units + 7) / 8;
-    if (n <= 128) CG_CUDA(c, launch_kernel(c, k_gated_norm_vec<TG, T, 1, 256>, dim3((unsigned)blocks), dim3(256), 0, 1, a, n, units, 32));
-    else CG_CUDA(c, launch_kernel(c, k_gated_norm_vec<TG, T, 4, 512>, dim3((unsigned)blocks), dim3(256), 0, 1, a, n, units, 32));
-  } else if (vec) {
+  if (vec) {
+    // up to 512 values a warp each, eight to a block
+    const bool warps = n <= 512;
+    const int64_t blocks = warps ? (a.M * units + 7) / 8 : a.M * units;
     const int threads = n <= 4096 ? 256 : n <= 8192 ? 512 : 1024;
-    auto kernel = threads <= 512 ? k_gated_norm_vec<TG, T, 4, 512> : k_gated_norm_vec<TG, T, 4, 1024>;
-    CG_CUDA(c, launch_kernel(c, kernel, dim3((unsigned)(a.M * units)), dim3(threads), 0, 1, a, n, units, threads));
+    const bool early = blocks <= 2 * 148 && threads <= 512;
+    auto kernel = n <= 128 ? (early ? k_gated_norm_vec<TG, T, 1, true> : k_gated_norm_vec<TG, T, 1, false>)
+                           : early ? k_gated_norm_vec<TG, T, 4, true> : k_gated_norm_vec<TG, T, 4, false>;
+    CG_CUDA(c, launch_kernel(c, kernel, dim3((unsigned)blocks), dim3(threads), 0, 1, a, n, units, warps ? 32 : threads));
   } else {
     dim3 grid((unsigned)units, (unsigned)a.M);
     if (grid.y > 65535) return fail(c, CG_ERR_UNSUPPORTED, "recurrence: too many tokens in one portion");

@@ -376,15 +376,17 @@ def test_wide_rows(backends, width, prec):
 
 @gpu
 @pytest.mark.parametrize("prec", ["f32", "bf16"])
-@pytest.mark.parametrize("heads,vdim,norm_groups", [(32, 128, 1), (64, 128, 1), (205, 40, 1), (130, 128, 2), (128, 128, 1)])
-def test_wide_norm_groups(backends, heads, vdim, norm_groups, prec):
-    """Groups of the gated norm of 4096 to 16384 values: 256, 512 and 1024 threads, behind a prompt and behind steps."""
+@pytest.mark.parametrize("heads,vdim,norm_groups,n", [(32, 128, 1, 9), (64, 128, 1, 9), (205, 40, 1, 9), (130, 128, 2, 9), (128, 128, 1, 9),
+                                                      (32, 128, 1, 296), (32, 128, 1, 297), (24, 64, 3, 800)])
+def test_wide_norm_groups(backends, heads, vdim, norm_groups, n, prec):
+    """Groups of the gated norm of 4096 to 16384 values: 256, 512 and 1024 threads, behind a prompt and behind steps; as many
+    groups as blocks of the form for few, one more, and groups of a warp each."""
     cfg = model([ssd(heads=heads, groups=1, vdim=vdim, norm_groups=norm_groups)])
-    W, seq = weights(cfg, 22), toks(9, heads)
+    W, seq = weights(cfg, 22), toks(n, heads)
     want = oracle.forward(cfg, W, seq)
-    dec = decoder(backends[prec], cfg, W, max_seq=16, max_batch=1)
+    dec = decoder(backends[prec], cfg, W, max_seq=n, max_batch=1)
     assert close(everything(dec, seq), want, prec)
-    assert close(everything(dec, seq, [5, 1, 1, 1, 1]), want, prec)
+    assert close(everything(dec, seq, [n - 4, 1, 1, 1, 1]), want, prec)
     dec.close()
 
 
